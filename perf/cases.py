@@ -4,7 +4,7 @@ A case is a dict of plain values.  ``listed()`` names twelve of them, ``draw(rng
 ranges, ``prepare(case, seed)`` makes what a program holds before the call (inputs, packed weights, the
 module or model that owns them), ``run(state)`` is one pass through the public entry points, ``work(case)``
 the bytes and operations a pass cannot do without, ``tolerance(case)`` how far two correct implementations
-may lie apart.
+may lie apart, ``exact(case, seed)`` the outputs in 64 bits by plain torch.
 
 Kinds:
 
@@ -24,6 +24,7 @@ from __future__ import annotations
 import math
 
 import torch
+import torch.nn.functional as F
 
 from dimq_b200 import ops
 from dimq_b200.export import activation_qparams_from_minmax
@@ -206,6 +207,126 @@ def run(state):
     out = fake_quant_weight(w, books, group_rows=group_rows)
     out.backward(grad)
     return out.detach(), w.grad
+
+
+# ---------------------------------------------------------------------------------------------
+# the same in 64 bits
+# ---------------------------------------------------------------------------------------------
+
+def _unpack64(packed: torch.Tensor, numel: int, bits: int) -> torch.Tensor:
+    """Indices of a little-endian bit stream, with plain torch."""
+    stream = (packed.view(-1, 1) >> torch.arange(8, device=packed.device, dtype=torch.uint8)) & 1
+    fields = stream.view(-1)[:numel * bits].view(numel, bits).long()
+    return (fields << torch.arange(bits, device=packed.device)).sum(1)
+
+
+def _weight64(packed: torch.Tensor, books: torch.Tensor, n: int, k: int, bits: int, group_rows: int) -> torch.Tensor:
+    idx = _unpack64(packed, n * k, bits).view(n, k)
+    books = books.double().reshape(-1, books.shape[-1])
+    rows = books[torch.arange(n, device=idx.device) // (group_rows or n)]        # [n, entries]
+    return torch.gather(rows, 1, idx)
+
+
+def _layer64(layer: dict) -> tuple[torch.Tensor, torch.Tensor]:
+    """Weight (in its own shape) and bias of a checkpoint's layer."""
+    shape = layer["weight_shape"]
+    w = _weight64(layer["packed_weight"], layer["codebook"], shape[0], math.prod(shape[1:]), layer["bit_w"],
+                  layer.get("group_rows") or 0)
+    return w.view(*shape), layer["bias"].double()
+
+
+def _centred64(x: torch.Tensor, q: dict) -> torch.Tensor:
+    """4-bit activation codes without the zero point, times the scale (the quotient is an fp32 one by contract)."""
+    scale = torch.tensor(q["scale"], device=x.device, dtype=torch.float32)
+    z = q["zero_point"]
+    return ((torch.round(x / scale) + z).clamp_(0, 15) - z).double() * scale.double()
+
+
+def _resnet64(ckpt: dict, images: torch.Tensor) -> torch.Tensor:
+    layers = {name: _layer64(layer) for name, layer in ckpt["layers"].items()}
+
+    def conv(name, x):
+        layer = ckpt["layers"][name]
+        w, b = layers[name]
+        return F.conv2d(x, w, b, layer["stride"], layer["padding"])
+
+    logits = []
+    for part in images.double().split(16):
+        x = F.max_pool2d(conv("conv1", part).relu_(), 3, 2, 1)
+        for stage in range(1, 5):
+            for block in range(2):
+                pre = f"layer{stage}.{block}."
+                skip = conv(pre + "downsample", x) if pre + "downsample" in layers else x
+                x = (conv(pre + "conv2", conv(pre + "conv1", x).relu_()) + skip).relu_()
+        logits.append(F.linear(x.mean(dim=(2, 3)), *layers["fc"]))
+    return torch.cat(logits)
+
+
+def _vit64(ckpt: dict, images: torch.Tensor) -> torch.Tensor:
+    cfg = ckpt["config"]
+    hid, heads = cfg["hidden"], cfg["heads"]
+    layers = {name: _layer64(layer) for name, layer in ckpt["layers"].items()}
+    dense = {name: value.double() for name, value in ckpt["non_quantized_state_dict"].items()}
+
+    def norm(name, x):
+        return F.layer_norm(x, (hid,), dense[name + ".weight"], dense[name + ".bias"], 1e-6)
+
+    logits = []
+    for part in images.double().split(16):
+        patches = F.conv2d(part, dense["patch_embed.weight"], dense["patch_embed.bias"], stride=cfg["patch"])
+        b = part.shape[0]
+        x = torch.cat([dense["cls_token"].expand(b, 1, hid), patches.flatten(2).transpose(1, 2)], 1) + dense["pos_embed"]
+        for i in range(cfg["layers"]):
+            pre = f"blocks.{i}."
+            qkv = F.linear(norm(pre + "norm1", x), *layers[pre + "attn.qkv"])
+            q, k, v = qkv.view(b, -1, 3, heads, hid // heads).permute(2, 0, 3, 1, 4)
+            a = torch.softmax(q @ k.transpose(-1, -2) * (hid // heads) ** -0.5, -1) @ v
+            x = x + F.linear(a.transpose(1, 2).reshape(b, -1, hid), *layers[pre + "attn.proj"])
+            h = F.gelu(F.linear(norm(pre + "norm2", x), *layers[pre + "mlp.fc1"]))
+            x = x + F.linear(h, *layers[pre + "mlp.fc2"])
+        logits.append(F.linear(norm("norm", x[:, 0]), *layers["head"]))
+    return torch.cat(logits)
+
+
+def exact(case: dict, seed: int):
+    """What ``run`` returns for the inputs of ``prepare(case, seed)``, in 64 bits and with plain torch."""
+    kind = case["kind"]
+    if kind in ("resnet", "vit"):
+        gen = torch.Generator(device="cuda").manual_seed(seed)
+        images = torch.randn(case["batch"], 3, 224, 224, device="cuda", generator=gen)
+        if kind == "resnet":
+            return _resnet64(build_resnet18_checkpoint(seed=seed), images)
+        return _vit64(build_vit_b16_checkpoint(seed=seed), images)
+    if kind == "export":
+        return None                                # whole numbers and bytes
+    if kind == "qat":
+        w, books, _, grad = prepare(case, seed)
+        w = w.detach().double()
+        books = books.double().reshape(-1, books.shape[-1]).sort(dim=1).values
+        rows = case["group_rows"] or case["n"]
+        out = torch.empty_like(w)
+        for g, book in enumerate(books):
+            part = w[g * rows:(g + 1) * rows]
+            out[g * rows:(g + 1) * rows] = book[torch.bucketize(part, (book[1:] + book[:-1]) / 2)]
+        return out, grad.double()
+    layer, x = prepare(case, seed)
+    bits = case.get("bits", 4)
+    n = case["cout"] if "cout" in case else case["n"]
+    ks = case.get("ksize", 1)
+    k = case["cin"] * ks * ks if "cout" in case else case["k"]
+    w = _weight64(layer.packed_weight, layer.codebook, n, k, bits, case.get("group_rows", 0))
+    if kind == "linear_a4":
+        x = _centred64(x, activation_qparams_from_minmax(-3.7, 3.9))
+    elif kind == "conv_a4":
+        x = _centred64(x, activation_qparams_from_minmax(0.0, 4.2))
+    x, bias = x.double(), layer.bias.double()
+    if "cout" in case:
+        y = torch.cat([F.conv2d(part.contiguous(), w.view(n, case["cin"], ks, ks), bias, case["stride"], ks // 2)
+                       for part in x.split(16)])
+    else:
+        y = F.linear(x, w, bias)
+    epilogue = case.get("epilogue", "none")
+    return y.relu_() if epilogue == "relu" else F.gelu(y) if epilogue == "gelu" else y
 
 
 # ---------------------------------------------------------------------------------------------
