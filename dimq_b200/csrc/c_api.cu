@@ -46,6 +46,12 @@ int64_t stem_conv_workspace_bytes(int x_dtype, const dimq_wq_weight* w, const di
 int launch_stem_conv(const void* x, int x_dtype, const dimq_wq_weight* w, const void* bias, int bias_dtype,
                      const void* residual, void* y, int y_dtype, const dimq_conv_geom* g, int epilogue, void* workspace,
                      int64_t workspace_bytes, cudaStream_t st);
+bool linear_exact_supported(bool a4, const void* x, int x_dtype, const dimq_wq_weight* w, const void* y, int y_dtype,
+                            const void* residual, int64_t M, int64_t N, int64_t K);
+int64_t linear_exact_workspace_bytes(bool a4, const dimq_wq_weight* w, int64_t M, int64_t N, int64_t K);
+int launch_linear_exact(bool a4, const void* x, int x_dtype, float scale, int zp, const dimq_wq_weight* w, const void* bias,
+                        int bias_dtype, const void* residual, void* y, int y_dtype, int64_t M, int64_t N, int64_t K,
+                        int epilogue, void* workspace, int64_t workspace_bytes, cudaStream_t st);
 int read_device_status(uint32_t* status);
 int read_ms_status(uint32_t* status);
 bool mma_regs_supported(const void* x, int x_dtype, const dimq_wq_weight* w, int64_t M, int64_t N, int64_t K);
@@ -218,6 +224,12 @@ extern "C" int dimq_linear_wq_workspace_bytes(const void* x, int x_dtype, const 
     return DIMQ_OK;
   }
   if (mma_stream_supported(x, x_dtype, w, M, N, K) || stream_supported(w, M, N, K)) return DIMQ_OK;
+  // fp32 activations: split into fp16 terms for the tensor cores (an fp32 output is assumed here;
+  // dimq_linear_wq_ws checks the real one)
+  if (linear_exact_supported(false, x, x_dtype, w, nullptr, DIMQ_F32, nullptr, M, N, K)) {
+    *bytes = linear_exact_workspace_bytes(false, w, M, N, K);
+    return DIMQ_OK;
+  }
   // many activation rows: the expanded 16-bit weight (the output is taken to be as wide as it may get
   // - 16-bit - and aligned; dimq_linear_wq_ws checks the real one and falls back if it does not fit)
   if (dense_pays(M) && (N * 2) % 16 == 0 && dense_supported(x, x_dtype, w, x, x_dtype, nullptr, M, N, K)) {
@@ -238,11 +250,15 @@ extern "C" int dimq_linear_wq_ws(const void* x, int x_dtype, const dimq_wq_weigh
       (bias == nullptr || valid_dtype(bias_dtype)) && epilogue >= DIMQ_EPI_NONE && epilogue <= DIMQ_EPI_ADD_RELU &&
       x != nullptr && y != nullptr &&
       dimq_linear_wq_workspace_bytes(x, x_dtype, w, M, N, K, &need) == DIMQ_OK && need > 0) {
-    if (workspace_bytes < need) return DIMQ_ERR_SCRATCH_TOO_SMALL;
+    if (workspace_bytes < need && x_dtype != DIMQ_F32) return DIMQ_ERR_SCRATCH_TOO_SMALL;   // fp32: runs without scratch too
     if (mma_regs_supported(x, x_dtype, w, M, N, K) && mma_regs_pays(w, N, K))
       return launch_linear_wq_mma_regs(x, x_dtype, w, bias, bias_dtype, residual, y, y_dtype, M, N, K, epilogue, workspace,
                                        workspace_bytes, static_cast<cudaStream_t>(stream));
-    if (dense_pays(M)) {
+    if (x_dtype == DIMQ_F32) {
+      if (workspace_bytes >= need && linear_exact_supported(false, x, x_dtype, w, y, y_dtype, residual, M, N, K))
+        return launch_linear_exact(false, x, x_dtype, 1.0f, 0, w, bias, bias_dtype, residual, y, y_dtype, M, N, K, epilogue,
+                                   workspace, workspace_bytes, static_cast<cudaStream_t>(stream));
+    } else if (dense_pays(M)) {
       if (dense_supported(x, x_dtype, w, y, y_dtype, residual, M, N, K))
         return launch_linear_wq_dense(x, x_dtype, w, bias, bias_dtype, residual, y, y_dtype, M, N, K, epilogue,
                                       workspace, workspace_bytes, static_cast<cudaStream_t>(stream));

@@ -28,6 +28,7 @@
 // vectors into a swizzled staging tile and one TMA store per 32 x 32 chunk writes y.
 #include <cstring>
 
+#include "exact_prep.cuh"
 #include "tc_common.cuh"
 
 namespace dimq {
@@ -57,7 +58,9 @@ struct DenseParams {
   int y_dtype;
   int64_t M, N;             // output rows (GEMM) / pixels (conv), output features
   int k_blocks;             // 64-k blocks of one pass over the reduction
-  int passes;               // 2 when the scratch carries hi and lo terms of every codeword side by side
+  int passes;               // passes over the reduction (2 when the scratch carries hi and lo terms of every codeword)
+  int a_term[3], b_term[3]; // the operand terms pass i multiplies: columns [term * K, (term + 1) * K) of either matrix
+  int b_terms;              // terms side by side in the weight matrix
   int bn;                   // weight rows per tile: 64, 128 or 256
   int m_tiles, n_tiles;
   int stages;
@@ -72,6 +75,11 @@ struct DenseParams {
   int kps;                  // 64-k blocks per ring stage (1 or 2): narrow tiles amortise the per-stage wait / commit over 8 MMAs
   int b_res;                // convolution: the whole expanded weight (one tile wide) stays in shared memory
   int pair;                 // 1: CTA pairs (cta_group::2), GEMM only; m_tiles then counts 256-row pairs of blocks
+  // SEG form only: out = acc * row_scale[row] * col_scale[n] (null: out_scale, 1)
+  const float* row_scale;
+  const float* col_scale;
+  float out_scale;
+  void* y_nchw;             // convolution with an NCHW output: plain stores instead of the TMA store
 #ifdef DIMQ_B200_DIAG
   int diag;
   unsigned long long* prof;   // 32 cycle counters per CTA, or null
@@ -105,7 +113,7 @@ struct DenseMaps {
 
 struct DenseHeader {
   uint64_t full[kMaxStages], empty[kMaxStages];
-  uint64_t d_full[kAccStages], d_empty[kAccStages];
+  uint64_t d_full[4], d_empty[4];   // kAccStages, or kSegAccStages
   uint64_t b_res_full;              // convolution with a resident weight: all its tiles have landed
   uint32_t tmem_base;
   volatile uint32_t abort_flag;
@@ -289,9 +297,75 @@ __device__ __forceinline__ void mma_commit_pair(uint32_t bar) {   // one arrival
                ::"r"(bar), "h"(static_cast<uint16_t>(3)) : "memory");
 }
 
-// ES = bytes per output element (2: bf16 / fp16, 4: fp32); PAIR: CTA pairs (GEMM only, bn = 256)
-template <int ES, bool PAIR>
-__global__ void __launch_bounds__(kThreads, 1)
+// One 32 x 32 chunk of the output: bias / activation / residual on this lane's 32 features, then one TMA store of the
+// warp's 32 rows - or, for an NCHW convolution output, plain stores: for one channel the 32 lanes are 32 pixels of the
+// tile, runs of tw consecutive ones.
+template <int ES, bool NCHW>
+__device__ __forceinline__ void store_chunk(float (&v)[32], const float* my_bias, unsigned char* my_out, const DenseMaps& maps,
+                                            const DenseParams& p, int64_t n_first, int64_t row_off, int c1, int c2, int c3,
+                                            int lane) {
+  float res[32];
+  const int64_t left = p.N - n_first;
+  const int valid = left >= 32 ? 32 : static_cast<int>(left);
+  bool relu_cvt;
+  if (p.residual != nullptr) {
+    if (row_off >= 0)
+      load_residual<ES>(static_cast<const char*>(p.residual) + (row_off + n_first) * ES, p.y_dtype, valid, res);
+    else {
+#pragma unroll
+      for (int j = 0; j < 32; ++j) res[j] = 0.0f;
+    }
+    relu_cvt = finish_row_epi<ES, true>(v, my_bias, res, p.epilogue);
+  } else {
+    relu_cvt = finish_row_epi<ES, false>(v, my_bias, res, p.epilogue);
+  }
+  if (NCHW && p.y_nchw != nullptr) {
+    float* dst = static_cast<float*>(p.y_nchw) + row_off + n_first * p.OH * p.OW;
+    if (row_off >= 0) {
+#pragma unroll
+      for (int j = 0; j < 32; ++j)
+        if (j < valid) dst[static_cast<int64_t>(j) * p.OH * p.OW] = v[j];
+    }
+    return;
+  }
+  // the previous store of this warp must have finished reading the staging tile
+  if (elect_one()) tma_store_wait_read();
+  __syncwarp();
+  if (ES == 2) {
+    // [32 rows][64 bytes], 64-byte swizzle: 16-byte piece j of row r sits at piece j ^ ((r >> 1) & 3)
+    stage_row16_any(v, my_out + lane * 64, (lane >> 1) & 3, p.y_dtype, relu_cvt);
+  } else {
+    // [32 rows][128 bytes], 128-byte swizzle: piece j of row r sits at piece j ^ (r & 7)
+    unsigned char* row_ptr = my_out + lane * 128;
+    const int sw = lane & 7;
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+      *reinterpret_cast<float4*>(row_ptr + ((j ^ sw) << 4)) = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+  }
+  fence_proxy_async_smem();
+  __syncwarp();
+#ifdef DIMQ_B200_DIAG
+  if (!(p.diag & 16))
+#endif
+  if (elect_one()) {
+    if (p.conv) tma_store_4d(&maps.y, smem_u32(my_out), static_cast<int>(n_first), c1, c2, c3);
+    else tma_store_2d(&maps.y, smem_u32(my_out), static_cast<int>(n_first), c1);
+    tma_store_commit();
+  }
+}
+
+// ES = bytes per output element (2: bf16 / fp16, 4: fp32); PAIR: CTA pairs (GEMM only, bn = 256).
+// SEG: the fp32-grade form (bn <= 128).  The tensor cores add into their fp32 accumulators by truncation: measured
+// against 64 bits, the error of a sum grows with its number of steps (fp16 operands: 6.4e-7 at K = 512, 3.7e-6 at
+// K = 3072, nearly all of it toward zero; fp32 FMAs 3.9e-7 and 9.5e-7).  So a tile's reduction is cut into segments
+// of kSegBlocks 64-k blocks, each started from zero in the other accumulator buffer, and the epilogue warps add the
+// segments in registers, rounding to nearest, while the next segment is being multiplied.
+constexpr int kSegBlocks = 4;
+constexpr int kSegAccStages = 4, kSegAccCols = 128;   // four buffers of 128 columns: the MMA warp runs ahead of a tile's final stores
+// three producers (a narrow tile's copies need no more) leave the epilogue warps 168 registers for the sums
+constexpr int kSegThreads = (1 + 3 + kEpiWarps) * 32;
+template <int ES, bool PAIR, bool SEG = false>
+__global__ void __launch_bounds__(SEG ? kSegThreads : kThreads, 1)
 lut_dense_tc_kernel(const __grid_constant__ DenseMaps maps, const DenseParams p) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   // [stages: A 16 KB | B bn*128 B (all 1024-aligned)] [header] [bias slices] [staging tiles]
@@ -308,6 +382,9 @@ lut_dense_tc_kernel(const __grid_constant__ DenseMaps maps, const DenseParams p)
   float* bias_area = reinterpret_cast<float*>(reinterpret_cast<unsigned char*>(hdr) + kHeaderBytes);
   unsigned char* staging = reinterpret_cast<unsigned char*>(bias_area) + kBiasBytes;   // 1024-aligned
   constexpr uint32_t kStagingBytes = 32u * 32u * ES;
+  constexpr int kAccBufs = SEG ? kSegAccStages : kAccStages;
+  constexpr uint32_t kBufCols = SEG ? kSegAccCols : kAccCols;
+  constexpr uint32_t kTurns = SEG ? 3 : kProducers;
 
   const int tid = threadIdx.x;
   const int warp = tid >> 5, lane = tid & 31;
@@ -319,13 +396,13 @@ lut_dense_tc_kernel(const __grid_constant__ DenseMaps maps, const DenseParams p)
 
   if (tid == 0) {
     for (int s = 0; s < kMaxStages; ++s) { mbar_init(smem_u32(&hdr->full[s]), 1); mbar_init(smem_u32(&hdr->empty[s]), 1); }   // full: one arrival per producer warp
-    for (int s = 0; s < kAccStages; ++s) { mbar_init(smem_u32(&hdr->d_full[s]), 1); mbar_init(smem_u32(&hdr->d_empty[s]), PAIR ? 2 * kEpiWarps : kEpiWarps); }
+    for (int s = 0; s < kAccBufs; ++s) { mbar_init(smem_u32(&hdr->d_full[s]), 1); mbar_init(smem_u32(&hdr->d_empty[s]), PAIR ? 2 * kEpiWarps : kEpiWarps); }
     mbar_init(smem_u32(&hdr->b_res_full), 1);
     hdr->abort_flag = 0u;
     fence_barrier_init();
     prefetch_tensormap(&maps.a[0]);
     prefetch_tensormap(&maps.b);
-    prefetch_tensormap(&maps.y);
+    if (p.y_nchw == nullptr) prefetch_tensormap(&maps.y);   // an NCHW output has no map
   }
   if (warp == 1) {
     if constexpr (PAIR) {   // one warp of each CTA of the pair: the same columns in both tensor memories
@@ -354,7 +431,7 @@ lut_dense_tc_kernel(const __grid_constant__ DenseMaps maps, const DenseParams p)
     // No more producers than stages: a warp's successive blocks must be at most one ring revolution apart, or its
     // parity wait on a stage's `empty` barrier could be satisfied by the completion before the one it needs (five
     // producers over a four-stage ring overwrote live stages and ended in "unspecified launch failure").
-    uint32_t n_turns = n_st < static_cast<uint32_t>(kProducers) ? n_st : static_cast<uint32_t>(kProducers), turn = 0;
+    uint32_t n_turns = n_st < kTurns ? n_st : kTurns, turn = 0;
 #ifdef DIMQ_B200_DIAG
     if (p.diag & 32768) n_turns = 1;   // timing experiments: warp 0 issues every block's copies
 #endif
@@ -411,16 +488,17 @@ lut_dense_tc_kernel(const __grid_constant__ DenseMaps maps, const DenseParams p)
           if (mine) {
             STEM_CLK(t_is);
             const uint32_t dst_a = dst + static_cast<uint32_t>(sub) * sub_bytes;
-            const int kcol_b = g * kBK;
+            const int kcol_b = SEG ? (p.b_term[pass] * p.k_blocks + kb) * kBK : g * kBK;
+            const int kcol_a = SEG ? (p.a_term[pass] * p.k_blocks + kb) * kBK : kb * kBK;
             if (!p.conv) {
               if constexpr (PAIR) {
                 if (elect_one()) {
                   const uint32_t lead_full = map_to_cta(full, 0);
-                  tma_load_2d_pair(dst_a, &maps.a[0], lead_full, kb * kBK, m_blk * kBM);
+                  tma_load_2d_pair(dst_a, &maps.a[0], lead_full, kcol_a, m_blk * kBM);
                   tma_load_2d_pair(dst_a + kABytes, &maps.b, lead_full, kcol_b, n_blk * p.bn + static_cast<int>(rank) * (p.bn / 2));
                 }
               } else if (elect_one()) {
-                tma_load_2d(dst_a, &maps.a[0], full, kb * kBK, m_blk * kBM);
+                tma_load_2d(dst_a, &maps.a[0], full, kcol_a, m_blk * kBM);
                 tma_load_2d(dst_a + kABytes, &maps.b, full, kcol_b, n_blk * p.bn);
               }
             } else {
@@ -480,13 +558,17 @@ lut_dense_tc_kernel(const __grid_constant__ DenseMaps maps, const DenseParams p)
     if (p.b_res && ok && !__all_sync(0xFFFFFFFFu, mbar_wait(smem_u32(&hdr->b_res_full), 0u, abort_flag, 0x1A00u))) ok = false;
     STEM_ACC_DECL;
     STEM_CLK(t_all);
-    for (int t = tile0; t < num_tiles && ok; t += tile_step) {
+    const int seg_kb = SEG ? kSegBlocks : total_kb;   // a multiple of kps, or the whole tile: no stage holds two segments
+    int seg0 = 0;                                     // first k block of the current segment
+    for (int t = tile0; t < num_tiles && ok;) {
       STEM_CLK(t_w1);
       if (!__all_sync(0xFFFFFFFFu, mbar_wait(smem_u32(&hdr->d_empty[as]), aph ^ 1u, abort_flag, 0x1200u | as))) { ok = false; break; }
       STEM_ACC(1, t_w1);
       tc_fence_after();
-      const uint32_t d_tmem = tmem_base + as * kAccCols;
-      for (int g = 0; g < total_kb; g += p.kps) {
+      const uint32_t d_tmem = tmem_base + as * kBufCols;
+      const int seg_end = SEG && seg0 + seg_kb < total_kb ? seg0 + seg_kb : total_kb;
+      const int seg_first = SEG ? seg0 : 0;
+      for (int g = seg_first; g < seg_end; g += p.kps) {
         const int nblk = total_kb - g < p.kps ? total_kb - g : p.kps;   // 64-k blocks in this stage
         STEM_CLK(t_w2);
         if (!__all_sync(0xFFFFFFFFu, mbar_wait(smem_u32(&hdr->full[stage]), phase, abort_flag, 0x1300u | stage))) { ok = false; break; }
@@ -508,7 +590,7 @@ lut_dense_tc_kernel(const __grid_constant__ DenseMaps maps, const DenseParams p)
                 const uint64_t a_desc = (static_cast<uint64_t>(a_hi) << 32) | (al + 2u * j);
                 const uint64_t b_desc = (static_cast<uint64_t>(b_hi) << 32) | (bl + 2u * j);
                 if constexpr (PAIR) mma_f16_ss_pair(d_tmem, a_desc, b_desc, p.idesc, (g | i | j) ? 1u : 0u);
-                else mma_f16_ss(d_tmem, a_desc, b_desc, p.idesc, (g | i | j) ? 1u : 0u);
+                else mma_f16_ss(d_tmem, a_desc, b_desc, p.idesc, ((g - seg_first) | i | j) ? 1u : 0u);
               }
             }
           }
@@ -526,7 +608,9 @@ lut_dense_tc_kernel(const __grid_constant__ DenseMaps maps, const DenseParams p)
         else mma_commit(smem_u32(&hdr->d_full[as]));
       }
       __syncwarp();
-      if (++as == kAccStages) { as = 0; aph ^= 1u; }
+      if (++as == kAccBufs) { as = 0; aph ^= 1u; }
+      seg0 = seg_end;
+      if (!SEG || seg0 == total_kb) { seg0 = 0; t += tile_step; }
     }
     STEM_ACC(0, t_all);
     STEM_FLUSH(4, 4);
@@ -540,6 +624,7 @@ lut_dense_tc_kernel(const __grid_constant__ DenseMaps maps, const DenseParams p)
     const int n_chunks = p.bn / 32;
     uint32_t as = 0, aph = 0;
     bool ok = true;
+    if constexpr (SEG) asm volatile("griddepcontrol.wait;" ::: "memory");   // the scales come from the kernel before
     STEM_ACC_DECL;
     STEM_CLK(t_all);
     for (int t = tile0; t < num_tiles && ok; t += tile_step) {
@@ -558,7 +643,8 @@ lut_dense_tc_kernel(const __grid_constant__ DenseMaps maps, const DenseParams p)
         const int oh = ((m_blk / p.tiles_w) % p.tiles_h) * p.th + hh;
         const int ob = (m_blk / (p.tiles_w * p.tiles_h)) * p.tb + bb;
         if (ob < p.Bn && oh < p.OH && ow < p.OW)
-          row_off = ((static_cast<int64_t>(ob) * p.OH + oh) * p.OW + ow) * p.N;
+          row_off = SEG && p.y_nchw != nullptr ? static_cast<int64_t>(ob) * p.N * p.OH * p.OW + static_cast<int64_t>(oh) * p.OW + ow
+                                               : ((static_cast<int64_t>(ob) * p.OH + oh) * p.OW + ow) * p.N;
         const int p0 = quarter * 32;         // all tile dimensions are powers of two: 32 pixels form a box
         c1 = (m_blk % p.tiles_w) * p.tw + p0 % p.tw;
         c2 = ((m_blk / p.tiles_w) % p.tiles_h) * p.th + (p0 / p.tw) % p.th;
@@ -571,6 +657,65 @@ lut_dense_tc_kernel(const __grid_constant__ DenseMaps maps, const DenseParams p)
       for (int i = 0; i < 4; ++i) {
         const int64_t nb = static_cast<int64_t>(n_blk) * p.bn + (sub + 2 * i) * 32 + lane;
         bj[i] = (p.bias != nullptr && sub + 2 * i < n_chunks && nb < p.N) ? load_as_float(p.bias, p.bias_dtype, nb) : 0.0f;
+      }
+      if constexpr (SEG) {
+        // add the tile's segments in registers: this warp's chunks are sub and sub + 2 (bn <= 128)
+        float sum[2][32];
+        const float rs = p.row_scale == nullptr ? p.out_scale
+                         : row_off >= 0 ? p.row_scale[static_cast<int64_t>(m_blk) * kBM + quarter * 32 + lane] : 0.0f;
+        for (int seg0 = 0; seg0 < total_kb; seg0 += kSegBlocks) {
+          if (!__all_sync(0xFFFFFFFFu, mbar_wait(smem_u32(&hdr->d_full[as]), aph, abort_flag, 0x1500u | as))) { ok = false; break; }
+          tc_fence_after();
+          const uint32_t d_tmem = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + as * kBufCols;
+          uint32_t r0[32], r1[32];
+          tmem_ld32(d_tmem + sub * 32, r0);
+          if (sub + 2 < n_chunks) tmem_ld32(d_tmem + (sub + 2) * 32, r1);
+          tmem_ld_wait();
+          tc_fence_before();      // both chunks are in registers: the buffer goes back before the sums are touched
+          __syncwarp();
+          if (lane == 0) mbar_arrive(smem_u32(&hdr->d_empty[as]));
+          __syncwarp();
+          if (++as == kAccBufs) { as = 0; aph ^= 1u; }
+          if (seg0 == 0) {
+#pragma unroll
+            for (int j = 0; j < 32; ++j) { sum[0][j] = __uint_as_float(r0[j]); sum[1][j] = __uint_as_float(r1[j]); }
+          } else {
+#pragma unroll
+            for (int j = 0; j < 32; ++j) { sum[0][j] += __uint_as_float(r0[j]); sum[1][j] += __uint_as_float(r1[j]); }
+          }
+        }
+        if (!ok) break;
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          const int c = sub + 2 * i;
+          const int64_t n_first = static_cast<int64_t>(n_blk) * p.bn + c * 32;
+          if (c < n_chunks && n_first < p.N) {     // warp-uniform
+            float (&v)[32] = sum[i];
+            __syncwarp();
+            my_bias[lane] = bj[i];
+            __syncwarp();
+            if (p.col_scale == nullptr) {
+#pragma unroll
+              for (int j = 0; j < 32; ++j) v[j] *= rs;
+            } else {
+              const float cs = n_first + lane < p.N ? p.col_scale[n_first + lane] : 1.0f;
+              constexpr float kBig = 1.099511627776e12f;     // 2^40
+              const bool plain = rs * kBig >= 1.0f && rs <= kBig && cs * kBig >= 1.0f && cs <= kBig;
+              if (__all_sync(0xFFFFFFFFu, plain)) {
+#pragma unroll
+                for (int j = 0; j < 32; ++j) v[j] *= rs * __shfl_sync(0xFFFFFFFFu, cs, j);
+              } else {   // the smaller scale first: no overflow or underflow on the way to a representable result
+#pragma unroll
+                for (int j = 0; j < 32; ++j) {
+                  const float csj = __shfl_sync(0xFFFFFFFFu, cs, j);
+                  v[j] = (v[j] * fminf(rs, csj)) * fmaxf(rs, csj);
+                }
+              }
+            }
+            store_chunk<ES, ES == 4>(v, my_bias, my_out, maps, p, n_first, row_off, c1, c2, c3, lane);
+          }
+        }
+        continue;
       }
       // tcgen05.ld is warp-collective: the whole warp proceeds or the whole warp gives up
       STEM_CLK(t_w1);
@@ -610,45 +755,7 @@ lut_dense_tc_kernel(const __grid_constant__ DenseMaps maps, const DenseParams p)
         float v[32];
 #pragma unroll
         for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
-        float res[32];
-        const int64_t left = p.N - n_first;
-        const int valid = left >= 32 ? 32 : static_cast<int>(left);
-        bool relu_cvt;
-        if (p.residual != nullptr) {
-          if (row_off >= 0)
-            load_residual<ES>(static_cast<const char*>(p.residual) + (row_off + n_first) * ES, p.y_dtype, valid, res);
-          else {
-#pragma unroll
-            for (int j = 0; j < 32; ++j) res[j] = 0.0f;
-          }
-          relu_cvt = finish_row_epi<ES, true>(v, my_bias, res, p.epilogue);
-        } else {
-          relu_cvt = finish_row_epi<ES, false>(v, my_bias, res, p.epilogue);
-        }
-        // the previous store of this warp must have finished reading the staging tile
-        if (elect_one()) tma_store_wait_read();
-        __syncwarp();
-        if (ES == 2) {
-          // [32 rows][64 bytes], 64-byte swizzle: 16-byte piece j of row r sits at piece j ^ ((r >> 1) & 3)
-          stage_row16_any(v, my_out + lane * 64, (lane >> 1) & 3, p.y_dtype, relu_cvt);
-        } else {
-          // [32 rows][128 bytes], 128-byte swizzle: piece j of row r sits at piece j ^ (r & 7)
-          unsigned char* row_ptr = my_out + lane * 128;
-          const int sw = lane & 7;
-#pragma unroll
-          for (int j = 0; j < 8; ++j)
-            *reinterpret_cast<float4*>(row_ptr + ((j ^ sw) << 4)) = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
-        }
-        fence_proxy_async_smem();
-        __syncwarp();
-#ifdef DIMQ_B200_DIAG
-        if (!(p.diag & 16))
-#endif
-        if (elect_one()) {
-          if (p.conv) tma_store_4d(&maps.y, smem_u32(my_out), static_cast<int>(n_first), c1, c2, c3);
-          else tma_store_2d(&maps.y, smem_u32(my_out), static_cast<int>(n_first), c1);
-          tma_store_commit();
-        }
+        store_chunk<ES, false>(v, my_bias, my_out, maps, p, n_first, row_off, c1, c2, c3, lane);
       }
       if (++as == kAccStages) { as = 0; aph ^= 1u; }
     }
@@ -683,87 +790,8 @@ lut_expand_kernel(const uint8_t* __restrict__ packed, const void* __restrict__ c
   // the GEMM that follows in the stream is launched as a programmatic dependent: its prologue may start now,
   // and it waits (griddepcontrol.wait) before it reads what this kernel writes
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  const int64_t units_per_row = K / 32;
-  const int64_t total = rows * units_per_row;
-  const int64_t u = static_cast<int64_t>(blockIdx.x) * 256 + threadIdx.x;
-  // Up to 16-entry codebooks: the codewords of the groups this block's rows belong to are converted once
-  // into a shared-memory table (hi | lo << 16), so an index costs one shared-memory read instead of a global
-  // read and two conversions.  A block covers at most 256 * 32 / 64 = 128 rows, i.e. at most 129 groups.
-  constexpr bool kTable = BITS <= 4;
-  __shared__ uint32_t tbl[kTable ? 129 * 16 : 1];
-  int64_t g_first = 0;
-  if (kTable) {
-    const int64_t u_first = static_cast<int64_t>(blockIdx.x) * 256;
-    const int64_t u_last = u_first + 255 < total - 1 ? u_first + 255 : total - 1;
-    g_first = (u_first / units_per_row) / group_rows;
-    const int n_groups = static_cast<int>((u_last / units_per_row) / group_rows - g_first) + 1;
-    for (int i = threadIdx.x; i < n_groups * 16; i += 256) {
-      const int e = i & 15;
-      const float c = e < entries ? load_as_float(codebooks, cb_dtype, (g_first + (i >> 4)) * entries + e) : 0.0f;
-      uint32_t v;
-      if (fmt == 0) {
-        v = __half_as_ushort(__float2half_rn(c));
-      } else {
-        const __nv_bfloat16 h = __float2bfloat16_rn(c);
-        v = __bfloat16_as_ushort(h) | (static_cast<uint32_t>(__bfloat16_as_ushort(__float2bfloat16_rn(c - __bfloat162float(h)))) << 16);
-      }
-      tbl[i] = v;
-    }
-    __syncthreads();
-  }
-  if (u >= total) return;
-  const int64_t row = u / units_per_row;
-  const int64_t k0 = (u - row * units_per_row) * 32;
-  const uint32_t* src = reinterpret_cast<const uint32_t*>(packed + (row * K + k0) * BITS / 8);
-  uint32_t w[BITS];
-#pragma unroll
-  for (int i = 0; i < BITS; ++i) w[i] = __ldg(src + i);
-  const int64_t cb0 = (row / group_rows) * entries;
-  const uint32_t* my_tbl = tbl + (kTable ? static_cast<int>(row / group_rows - g_first) * 16 : 0);
-  uint16_t hi[32], lo[32];
-#pragma unroll
-  for (int i = 0; i < 32; ++i) {
-    const int bit = i * BITS, word = bit >> 5, sh = bit & 31;
-    uint32_t idx = w[word] >> sh;
-    if (sh + BITS > 32) idx |= w[word + 1 < BITS ? word + 1 : word] << (32 - sh);
-    idx &= (1u << BITS) - 1u;
-    if (kTable) {
-      const uint32_t v = my_tbl[idx];      // entries past the codebook's count hold zero
-      hi[i] = static_cast<uint16_t>(v);
-      lo[i] = static_cast<uint16_t>(v >> 16);
-    } else {
-      const float c = idx < static_cast<uint32_t>(entries) ? load_as_float(codebooks, cb_dtype, cb0 + idx) : 0.0f;
-      if (fmt == 0) {
-        hi[i] = __half_as_ushort(__float2half_rn(c));
-        lo[i] = 0;
-      } else {
-        const __nv_bfloat16 h = __float2bfloat16_rn(c);
-        hi[i] = __bfloat16_as_ushort(h);
-        lo[i] = __bfloat16_as_ushort(__float2bfloat16_rn(c - __bfloat162float(h)));
-      }
-    }
-  }
-  uint16_t* dst = out + row * (K * passes) + k0;
-#pragma unroll
-  for (int v = 0; v < 4; ++v) {
-    uint4 q;
-    q.x = hi[8 * v] | (static_cast<uint32_t>(hi[8 * v + 1]) << 16);
-    q.y = hi[8 * v + 2] | (static_cast<uint32_t>(hi[8 * v + 3]) << 16);
-    q.z = hi[8 * v + 4] | (static_cast<uint32_t>(hi[8 * v + 5]) << 16);
-    q.w = hi[8 * v + 6] | (static_cast<uint32_t>(hi[8 * v + 7]) << 16);
-    reinterpret_cast<uint4*>(dst)[v] = q;
-  }
-  if (passes == 2) {
-#pragma unroll
-    for (int v = 0; v < 4; ++v) {
-      uint4 q;
-      q.x = lo[8 * v] | (static_cast<uint32_t>(lo[8 * v + 1]) << 16);
-      q.y = lo[8 * v + 2] | (static_cast<uint32_t>(lo[8 * v + 3]) << 16);
-      q.z = lo[8 * v + 4] | (static_cast<uint32_t>(lo[8 * v + 5]) << 16);
-      q.w = lo[8 * v + 6] | (static_cast<uint32_t>(lo[8 * v + 7]) << 16);
-      reinterpret_cast<uint4*>(dst + K)[v] = q;
-    }
-  }
+  __shared__ uint32_t tbl[BITS <= 4 ? kExpandTable : 1];
+  expand_block<BITS>(tbl, blockIdx.x, packed, codebooks, cb_dtype, entries, group_rows, rows, K, fmt, passes, out, nullptr);
 }
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -791,12 +819,13 @@ CUtensorMapDataType map_dtype(int dtype) {
 // simple model - waves of tiles over the SMs times the measured cycles of a 64-k block (four MMAs and
 // a commit: ~590 at N = 256, ~450 at N = 128, ~430 at N = 64: below N = 256 the per-instruction floor
 // of about 106 cycles shows).
-int choose_bn(int64_t m_tiles, int64_t N) {
+int choose_bn(int64_t m_tiles, int64_t N, int max_bn = 256) {
   const int cand[3] = {256, 128, 64};
   const double cycles[3] = {590.0, 450.0, 430.0};
-  int best = 256;
+  int best = max_bn;
   double best_cost = -1.0;
   for (int i = 0; i < 3; ++i) {
+    if (cand[i] > max_bn) continue;
     const int64_t tiles = m_tiles * ((N + cand[i] - 1) / cand[i]);
     const double cost = static_cast<double>((tiles + kNumSMs - 1) / kNumSMs) * cycles[i];
     if (best_cost < 0.0 || cost < best_cost) { best_cost = cost; best = cand[i]; }
@@ -856,7 +885,7 @@ cudaError_t launch_dependent(Kern kern, int grid, int threads, size_t smem, cuda
 }
 
 int launch_dense(DenseMaps& maps, DenseParams& p, const void* scratch, int64_t K, int x_dtype, const void* bias,
-                 int bias_dtype, const void* residual, int y_dtype, int epilogue, cudaStream_t st) {
+                 int bias_dtype, const void* residual, int y_dtype, int epilogue, cudaStream_t st, bool seg = false) {
   EncodeTiledFn encode = encode_tiled();
   if (encode == nullptr) return DIMQ_ERR_DRIVER;
   p.bias = bias;
@@ -873,8 +902,9 @@ int launch_dense(DenseMaps& maps, DenseParams& p, const void* scratch, int64_t K
 #endif
   const int fmt = x_dtype == DIMQ_BF16 ? 1 : 0;
   p.idesc = tc::make_idesc_f16(fmt, fmt, pair ? 2 * kBM : kBM, p.bn);
-  const cuuint64_t bdims[2] = {static_cast<cuuint64_t>(K * p.passes), static_cast<cuuint64_t>(p.N)};
-  const cuuint64_t bstr[1] = {static_cast<cuuint64_t>(K * p.passes) * 2};
+  const int64_t b_len = K * (seg ? p.b_terms : p.passes);
+  const cuuint64_t bdims[2] = {static_cast<cuuint64_t>(b_len), static_cast<cuuint64_t>(p.N)};
+  const cuuint64_t bstr[1] = {static_cast<cuuint64_t>(b_len) * 2};
   const cuuint32_t bbox[2] = {kBK, static_cast<cuuint32_t>(pair ? p.bn / 2 : p.bn)};
   const cuuint32_t estr[2] = {1, 1};
   if (encode(&maps.b, fmt == 1 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2,
@@ -933,6 +963,11 @@ int launch_dense(DenseMaps& maps, DenseParams& p, const void* scratch, int64_t K
       if (e != cudaSuccess) return static_cast<int>(e);
       e = launch_dependent(lut_dense_tc_kernel<4, true>, 2 * clusters, kThreads, smem, st, maps, p, 2);
     }
+  } else if (seg) {
+    auto kern = es == 2 ? lut_dense_tc_kernel<2, false, true> : lut_dense_tc_kernel<4, false, true>;
+    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    if (e != cudaSuccess) return static_cast<int>(e);
+    e = launch_dependent(kern, grid, kSegThreads, smem, st, maps, p);
   } else if (es == 2) {
     e = cudaFuncSetAttribute(lut_dense_tc_kernel<2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     if (e != cudaSuccess) return static_cast<int>(e);
@@ -1634,14 +1669,12 @@ int64_t conv_dense_workspace_bytes(int x_dtype, const dimq_wq_weight* w, const d
   return static_cast<int64_t>(g->out_channels) * g->kernel_h * g->kernel_w * g->in_channels * 2 * passes_for(x_dtype, w);
 }
 
-int launch_conv2d_wq_dense(const void* x, int x_dtype, const dimq_wq_weight* w, const void* bias, int bias_dtype,
-                           const void* residual, void* y, int y_dtype, const dimq_conv_geom* g, int epilogue,
-                           void* workspace, int64_t workspace_bytes, cudaStream_t st) {
-  if (!conv_dense_supported(x, x_dtype, w, g, y, y_dtype, residual)) return DIMQ_ERR_UNSUPPORTED;
-  if (workspace == nullptr || workspace_bytes < conv_dense_workspace_bytes(x_dtype, w, g)) return DIMQ_ERR_SCRATCH_TOO_SMALL;
-  if (!aligned(workspace, 16)) return DIMQ_ERR_ALIGNMENT;
-  EncodeTiledFn encode = encode_tiled();
-  if (encode == nullptr) return DIMQ_ERR_DRIVER;
+namespace {
+
+// Tile shape, geometry and tensor maps of an implicit-GEMM convolution over NHWC 16-bit activations; y (may be null)
+// is an NHWC output.
+int conv_setup(EncodeTiledFn encode, const void* x, int x_dtype, const void* y, int y_dtype, const dimq_conv_geom* g,
+               DenseMaps& maps, DenseParams& p) {
   const int OW = g->out_w, OH = g->out_h, B = g->batch;
   // Tile = tw x th x tb output pixels with tw * th * tb = 128, so every factor is a power of two and
   // any 32 consecutive tile pixels form a box (the TMA store of the epilogue needs that).  Prefer the
@@ -1663,9 +1696,7 @@ int launch_conv2d_wq_dense(const void* x, int x_dtype, const dimq_wq_weight* w, 
     best_tb = kBM / (best_tw * best_th);
   }
 #endif
-  DenseParams p;
   memset(&p, 0, sizeof(p));
-  DenseMaps maps;
   memset(&maps, 0, sizeof(maps));
   p.conv = 1;
   p.tw = best_tw;
@@ -1688,14 +1719,9 @@ int launch_conv2d_wq_dense(const void* x, int x_dtype, const dimq_wq_weight* w, 
   p.c_blocks = g->in_channels / kBK;
   p.M = static_cast<int64_t>(B) * OH * OW;
   p.N = g->out_channels;
-  p.passes = passes_for(x_dtype, w);
-  p.bn = choose_bn(p.m_tiles, p.N);
-  p.n_tiles = static_cast<int>((p.N + p.bn - 1) / p.bn);
-  const int64_t K = static_cast<int64_t>(g->kernel_h) * g->kernel_w * g->in_channels;
-
   const int s = g->stride_h;
   const int64_t C = g->in_channels, W = g->in_w, H = g->in_h;
-  const CUtensorMapDataType dt = x_dtype == DIMQ_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
+  const CUtensorMapDataType dt = map_dtype(x_dtype);
   for (int py = 0; py < s; ++py) {
     for (int px = 0; px < s; ++px) {
       const int64_t Wp = (W - px + s - 1) / s, Hp = (H - py + s - 1) / s;
@@ -1719,10 +1745,253 @@ int launch_conv2d_wq_dense(const void* x, int x_dtype, const dimq_wq_weight* w, 
   const cuuint64_t odims[4] = {static_cast<cuuint64_t>(g->out_channels), static_cast<cuuint64_t>(OW),
                                static_cast<cuuint64_t>(OH), static_cast<cuuint64_t>(B)};
   const cuuint32_t obox[4] = {32, static_cast<cuuint32_t>(cbw), static_cast<cuuint32_t>(cbh), static_cast<cuuint32_t>(cbb)};
-  if (!out_map(encode, &maps.y, y, y_dtype, 4, odims, obox)) return DIMQ_ERR_DRIVER;
-  int rc = expand(w, w->packed_khwc, p.N, K, x_dtype == DIMQ_BF16 ? 1 : 0, p.passes, workspace, st);
+  if (y != nullptr && !out_map(encode, &maps.y, y, y_dtype, 4, odims, obox)) return DIMQ_ERR_DRIVER;
+  return DIMQ_OK;
+}
+
+}  // namespace
+
+int launch_conv2d_wq_dense(const void* x, int x_dtype, const dimq_wq_weight* w, const void* bias, int bias_dtype,
+                           const void* residual, void* y, int y_dtype, const dimq_conv_geom* g, int epilogue,
+                           void* workspace, int64_t workspace_bytes, cudaStream_t st) {
+  if (!conv_dense_supported(x, x_dtype, w, g, y, y_dtype, residual)) return DIMQ_ERR_UNSUPPORTED;
+  if (workspace == nullptr || workspace_bytes < conv_dense_workspace_bytes(x_dtype, w, g)) return DIMQ_ERR_SCRATCH_TOO_SMALL;
+  if (!aligned(workspace, 16)) return DIMQ_ERR_ALIGNMENT;
+  EncodeTiledFn encode = encode_tiled();
+  if (encode == nullptr) return DIMQ_ERR_DRIVER;
+  DenseParams p;
+  DenseMaps maps;
+  int rc = conv_setup(encode, x, x_dtype, y, y_dtype, g, maps, p);
+  if (rc != DIMQ_OK) return rc;
+  p.passes = passes_for(x_dtype, w);
+  p.bn = choose_bn(p.m_tiles, p.N);
+  p.n_tiles = static_cast<int>((p.N + p.bn - 1) / p.bn);
+  const int64_t K = static_cast<int64_t>(g->kernel_h) * g->kernel_w * g->in_channels;
+  rc = expand(w, w->packed_khwc, p.N, K, x_dtype == DIMQ_BF16 ? 1 : 0, p.passes, workspace, st);
   if (rc != DIMQ_OK) return rc;
   return launch_dense(maps, p, workspace, K, x_dtype, bias, bias_dtype, residual, y_dtype, epilogue, st);
+}
+
+// ---- fp32-grade GEMM / convolution: W4A4 codes, or fp32 activations --------------------------------------
+//
+// Two launches: exact_prep_kernel (activations -> fp16 codes or hi | lo terms, indices -> fp16 codewords) and the SEG
+// form of lut_dense_tc_kernel.  What it replaces is a SIMT kernel bound by one shared-memory lookup per product
+// (linear_lut_a4_kernel, conv2d_direct_kernel) or by fp32 FMAs fed element by element (linear_wq_generic_kernel):
+//   W4A4, fp16 codebook: 197 x 768 -> 3072 605 -> 12 us; 7 x 128 channels on 28^2, 3x3, NCHW 3 310 -> 15 us
+//   fp32 activations, fp32 codebook: 1576 x 768 -> 3072 773 -> 50 us (three products), fp16 codebook 35 us (two)
+// Now bound by shared-memory bandwidth in the product (a 128 x 128 x 64 block moves 64 KB: 512 cycles, measured ~700)
+// and, for small calls, by the two launches.
+namespace {
+
+inline int64_t pad256(int64_t v) { return (v + 255) / 256 * 256; }
+
+// fp16 terms of a codeword: fp16 and (scaled) bf16 values are exact in one, fp32 ones take two
+int exact_terms(const dimq_wq_weight* w) { return w->cb_dtype == DIMQ_F32 ? 2 : 1; }
+
+// scratch regions: activations (halves), row scales, column scales, expanded weight
+struct ExactScratch {
+  int64_t x, row, col, w, total;
+  ExactScratch(int64_t x_halves, int64_t rows, int64_t N, int64_t K, int terms) {
+    x = 0;
+    row = x + pad256(x_halves * 2);
+    col = row + pad256(rows * 4);
+    w = col + pad256(N * 4);
+    total = w + pad256(N * K * 2 * terms);
+  }
+};
+
+// launches the preparation and fills in what the product needs to know about the operands
+int exact_prepare(PrepParams& q, DenseParams& p, const dimq_wq_weight* w, const uint8_t* packed, int64_t N, int64_t K,
+                  bool a4, float scale, const ExactScratch& at, void* workspace, int64_t x_blocks, cudaStream_t st) {
+  unsigned char* base = static_cast<unsigned char*>(workspace);
+  const int terms = exact_terms(w);
+  q.xo = reinterpret_cast<__half*>(base + at.x);
+  q.row_scale = a4 ? nullptr : reinterpret_cast<float*>(base + at.row);
+  q.col_scale = w->cb_dtype == DIMQ_F16 ? nullptr : reinterpret_cast<float*>(base + at.col);
+  q.wo = reinterpret_cast<uint16_t*>(base + at.w);
+  q.packed = packed;
+  q.codebooks = w->codebooks;
+  q.cb_dtype = w->cb_dtype;
+  q.entries = w->entries;
+  q.group_rows = w->group_rows;
+  q.rows = N;
+  q.K = K;
+  q.fmt = w->cb_dtype == DIMQ_F16 ? 0 : 2;
+  q.terms = terms;
+  q.x_blocks = x_blocks;
+  const int64_t blocks = x_blocks + (N * (K / 32) + 255) / 256;
+  if (blocks > 0x7FFFFFFFll) return DIMQ_ERR_TOO_LARGE;
+  const unsigned grid = static_cast<unsigned>(blocks);
+  if (w->bits == 2) exact_prep_kernel<2><<<grid, kPrepThreads, 0, st>>>(q);
+  else if (w->bits == 3) exact_prep_kernel<3><<<grid, kPrepThreads, 0, st>>>(q);
+  else exact_prep_kernel<4><<<grid, kPrepThreads, 0, st>>>(q);
+  p.row_scale = q.row_scale;
+  p.col_scale = q.col_scale;
+  p.out_scale = a4 ? scale : 1.0f;
+  // products of terms, the small ones first
+  p.b_terms = terms;
+  p.passes = 0;
+  auto pass = [&p](int a, int b) { p.a_term[p.passes] = a; p.b_term[p.passes++] = b; };
+  if (a4) {       // in column order: a convolution may keep the weight resident, pass after pass
+    for (int b = 0; b < terms; ++b) pass(0, b);
+  } else {
+    pass(1, 0);
+    if (terms == 2) pass(0, 1);
+    pass(0, 0);
+  }
+  return launch_status();
+}
+
+}  // namespace
+
+bool linear_exact_supported(bool a4, const void* x, int x_dtype, const dimq_wq_weight* w, const void* y, int y_dtype,
+                            const void* residual, int64_t M, int64_t N, int64_t K) {
+  if (a4 ? (w->bits != 4 || w->entries != 16) : (x_dtype != DIMQ_F32 || y_dtype != DIMQ_F32)) return false;
+  if (w->bits != 2 && w->bits != 3 && w->bits != 4) return false;
+  if (M < 1 || N < 1 || K < kBK || K % kBK != 0 || M > 0x7FFFFFFF / 2 || N > 0x7FFFFFFF / 2) return false;
+  const int64_t es = y_dtype == DIMQ_F32 ? 4 : 2;
+  if (!a4 && !aligned(x, 16)) return false;
+  if (!aligned(w->packed, 4) || !aligned(y, 16) || (N * es) % 16 != 0) return false;
+  return residual == nullptr || aligned(residual, 16);
+}
+
+int64_t linear_exact_workspace_bytes(bool a4, const dimq_wq_weight* w, int64_t M, int64_t N, int64_t K) {
+  return ExactScratch(a4 ? M * K : 2 * M * K, a4 ? 0 : M, N, K, exact_terms(w)).total;
+}
+
+int launch_linear_exact(bool a4, const void* x, int x_dtype, float scale, int zp, const dimq_wq_weight* w, const void* bias,
+                        int bias_dtype, const void* residual, void* y, int y_dtype, int64_t M, int64_t N, int64_t K,
+                        int epilogue, void* workspace, int64_t workspace_bytes, cudaStream_t st) {
+  if (!linear_exact_supported(a4, x, x_dtype, w, y, y_dtype, residual, M, N, K)) return DIMQ_ERR_UNSUPPORTED;
+  if (workspace == nullptr || workspace_bytes < linear_exact_workspace_bytes(a4, w, M, N, K)) return DIMQ_ERR_SCRATCH_TOO_SMALL;
+  if (!aligned(workspace, 16)) return DIMQ_ERR_ALIGNMENT;
+  EncodeTiledFn encode = encode_tiled();
+  if (encode == nullptr) return DIMQ_ERR_DRIVER;
+  const ExactScratch at(a4 ? M * K : 2 * M * K, a4 ? 0 : M, N, K, exact_terms(w));
+  DenseParams p;
+  memset(&p, 0, sizeof(p));
+  DenseMaps maps;
+  memset(&maps, 0, sizeof(maps));
+  p.M = M;
+  p.N = N;
+  p.m_tiles = static_cast<int>((M + kBM - 1) / kBM);
+  p.bn = choose_bn(p.m_tiles, N, 128);
+  p.n_tiles = static_cast<int>((N + p.bn - 1) / p.bn);
+  const int64_t row_len = a4 ? K : 2 * K;
+  const cuuint64_t adims[2] = {static_cast<cuuint64_t>(row_len), static_cast<cuuint64_t>(M)};
+  const cuuint64_t astr[1] = {static_cast<cuuint64_t>(row_len) * 2};
+  const cuuint32_t abox[2] = {kBK, kBM};
+  const cuuint32_t estr[2] = {1, 1};
+  if (encode(&maps.a[0], CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, static_cast<unsigned char*>(workspace) + at.x, adims, astr, abox,
+             estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+    return DIMQ_ERR_DRIVER;
+  const cuuint64_t odims[2] = {static_cast<cuuint64_t>(N), static_cast<cuuint64_t>(M)};
+  const cuuint32_t obox[2] = {32, 32};
+  if (!out_map(encode, &maps.y, y, y_dtype, 2, odims, obox)) return DIMQ_ERR_DRIVER;
+  PrepParams q;
+  memset(&q, 0, sizeof(q));
+  q.x = x;
+  q.x_dtype = x_dtype;
+  q.vec_ok = aligned(x, 16);
+  q.scale = scale;
+  q.zp = zp;
+  int64_t x_blocks;
+  if (a4) {
+    q.mode = kPrepCodes;
+    q.n = M * K;
+    x_blocks = ((q.n + 7) / 8 + kPrepThreads - 1) / kPrepThreads;
+  } else {
+    q.mode = kPrepSplitRows;
+    q.n = M;
+    q.C = K;
+    x_blocks = (M + 1) / 2;
+  }
+  int rc = exact_prepare(q, p, w, w->packed, N, K, a4, scale, at, workspace, x_blocks, st);
+  if (rc != DIMQ_OK) return rc;
+  return launch_dense(maps, p, static_cast<unsigned char*>(workspace) + at.w, K, DIMQ_F16, bias, bias_dtype, residual, y_dtype,
+                      epilogue, st, true);
+}
+
+namespace {
+
+// contiguous storage in the order of `stride`'s dimensions; an extent of one may carry any stride
+bool packed_strides(const int64_t stride[4], int64_t B, int64_t C, int64_t H, int64_t W, bool nhwc) {
+  const int64_t want[4] = {C * H * W, nhwc ? 1 : H * W, nhwc ? W * C : W, nhwc ? C : 1};
+  const int64_t size[4] = {B, C, H, W};
+  for (int i = 0; i < 4; ++i)
+    if (size[i] > 1 && stride[i] != want[i]) return false;
+  return true;
+}
+
+}  // namespace
+
+// x and y both NHWC, or both NCHW (fp32 output, no residual)
+bool conv_a4_exact_supported(const dimq_wq_weight* w, const dimq_conv_geom* g, const void* y, int y_dtype,
+                             const void* residual) {
+  if (w->packed_khwc == nullptr || w->bits != 4 || w->entries != 16 || !aligned(w->packed_khwc, 4)) return false;
+  if (g->groups != 1 || g->in_channels % kBK != 0 || g->batch < 1 || g->out_w < 1 || g->out_h < 1) return false;
+  if (g->stride_h != g->stride_w || (g->stride_h != 1 && g->stride_h != 2)) return false;
+  if (g->stride_h == 2 && (g->in_w < 2 || g->in_h < 2)) return false;   // a parity plane would be empty
+  const int64_t B = g->batch, OC = g->out_channels;
+  if (packed_strides(g->x_stride, B, g->in_channels, g->in_h, g->in_w, true) &&
+      packed_strides(g->y_stride, B, OC, g->out_h, g->out_w, true))
+    return aligned(y, 16) && (OC * (y_dtype == DIMQ_F32 ? 4 : 2)) % 16 == 0 && (residual == nullptr || aligned(residual, 16));
+  return y_dtype == DIMQ_F32 && residual == nullptr &&
+         packed_strides(g->x_stride, B, g->in_channels, g->in_h, g->in_w, false) &&
+         packed_strides(g->y_stride, B, OC, g->out_h, g->out_w, false);
+}
+
+int64_t conv_a4_exact_workspace_bytes(const dimq_wq_weight* w, const dimq_conv_geom* g) {
+  const int64_t x_numel = static_cast<int64_t>(g->batch) * g->in_channels * g->in_h * g->in_w;
+  return ExactScratch(x_numel, 0, g->out_channels, static_cast<int64_t>(g->kernel_h) * g->kernel_w * g->in_channels,
+                      exact_terms(w)).total;
+}
+
+int launch_conv_a4_exact(const void* x, int x_dtype, float scale, int zp, const dimq_wq_weight* w, const void* bias,
+                         int bias_dtype, const void* residual, void* y, int y_dtype, const dimq_conv_geom* g, int epilogue,
+                         void* workspace, int64_t workspace_bytes, cudaStream_t st) {
+  if (!conv_a4_exact_supported(w, g, y, y_dtype, residual)) return DIMQ_ERR_UNSUPPORTED;
+  if (workspace == nullptr || workspace_bytes < conv_a4_exact_workspace_bytes(w, g)) return DIMQ_ERR_SCRATCH_TOO_SMALL;
+  if (!aligned(workspace, 16)) return DIMQ_ERR_ALIGNMENT;
+  EncodeTiledFn encode = encode_tiled();
+  if (encode == nullptr) return DIMQ_ERR_DRIVER;
+  const int64_t B = g->batch, C = g->in_channels, HW = static_cast<int64_t>(g->in_h) * g->in_w;
+  const int64_t K = static_cast<int64_t>(g->kernel_h) * g->kernel_w * C, N = g->out_channels;
+  const bool nhwc = packed_strides(g->x_stride, B, C, g->in_h, g->in_w, true) &&
+                    packed_strides(g->y_stride, B, N, g->out_h, g->out_w, true) && aligned(y, 16) &&
+                    (N * (y_dtype == DIMQ_F32 ? 4 : 2)) % 16 == 0;
+  const ExactScratch at(B * C * HW, 0, N, K, exact_terms(w));
+  DenseParams p;
+  DenseMaps maps;
+  int rc = conv_setup(encode, static_cast<unsigned char*>(workspace) + at.x, DIMQ_F16, nhwc ? y : nullptr, y_dtype, g, maps, p);
+  if (rc != DIMQ_OK) return rc;
+  if (!nhwc) p.y_nchw = y;
+  p.bn = choose_bn(p.m_tiles, N, 128);
+  p.n_tiles = static_cast<int>((N + p.bn - 1) / p.bn);
+  PrepParams q;
+  memset(&q, 0, sizeof(q));
+  q.x = x;
+  q.x_dtype = x_dtype;
+  q.vec_ok = aligned(x, 16);
+  q.scale = scale;
+  q.zp = zp;
+  q.C = C;
+  q.HW = HW;
+  int64_t x_blocks;
+  if (nhwc) {
+    q.mode = kPrepCodes;
+    q.n = B * C * HW;
+    x_blocks = ((q.n + 7) / 8 + kPrepThreads - 1) / kPrepThreads;
+  } else {
+    q.mode = kPrepCodesNchw;
+    q.px_tiles = (HW + 31) / 32;
+    x_blocks = B * (C / 64) * q.px_tiles;
+  }
+  rc = exact_prepare(q, p, w, w->packed_khwc, N, K, true, scale, at, workspace, x_blocks, st);
+  if (rc != DIMQ_OK) return rc;
+  return launch_dense(maps, p, static_cast<unsigned char*>(workspace) + at.w, K, DIMQ_F16, bias, bias_dtype, residual, y_dtype,
+                      epilogue, st, true);
 }
 
 }  // namespace dimq

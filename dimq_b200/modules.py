@@ -107,8 +107,17 @@ class DIMQLinear(_PackedBase):
                                       packed_tiled=tiled)
         rows = x.numel() // self.in_features
         if rows >= ops.A4_TC_MIN_ROWS and self.in_features % 64 == 0:
-            # many rows: centred activation codes (exact in bf16) times the scaled codebook through the
-            # weight-only tensor-core path; per-layer state is cached, nothing is re-derived per call
+            # The fp32-grade form, except for an fp32 codebook on many rows: there it multiplies two fp16 terms in
+            # tiles of 128 x 128, the bf16 pair below in tiles of 256 (768 -> 3072: 20.5 against 21.1 us at 512 rows,
+            # 36 / 30 at 1576; with an fp16 codebook, one term, 13.6 / 20.9 and 22 / 30, 120 / 124 for 4096 x 3072 -> 3072).
+            if self.codebook.dtype != torch.float32 or rows < 1024:
+                y = ops.dimq_linear_a4(x, self.packed_weight, self.codebook, self.act_scale, self.act_zero_point,
+                                       self.bias, self.out_features, self.in_features, out_dtype=self.out_dtype,
+                                       epilogue=self.epilogue, residual=residual)
+                if y is not None:
+                    return y
+            # centred activation codes (exact in bf16) times the scaled codebook through the weight-only
+            # tensor-core path; per-layer state is cached, nothing is re-derived per call
             codes = ops.centre_quantize_u4(x, self.act_scale, self.act_zero_point)
             return ops.dimq_linear_wq(codes, self.packed_weight, self._scaled_codebook(), self.bias,
                                       self.out_features, self.in_features, bits=4, out_dtype=self.out_dtype,
@@ -173,9 +182,17 @@ class DIMQConv2d(_PackedBase):
             oh = (x.shape[2] + 2 * self.padding[0] - self.dilation[0] * (self.weight_shape[2] - 1) - 1) // self.stride[0] + 1
             ow = (x.shape[3] + 2 * self.padding[1] - self.dilation[1] * (self.weight_shape[3] - 1) - 1) // self.stride[1] + 1
             if x.shape[0] * oh * ow >= ops.A4_TC_MIN_ROWS:
-                # many output pixels: centred activation codes times the scaled codebook through the
-                # weight-only implicit-GEMM path, with the re-ordered indices and the scaled codebook
-                # cached on the module (no per-call index re-order)
+                # fp16 / bf16 codebooks are one exact term: the fp32-grade form (64 x 64 channels on 56^2, batch 64:
+                # 66 us, the bf16 pair 82; 512 on 7^2: 35 / 52); an fp32 codebook takes two there (94 / 82, 60 / 52)
+                if self.codebook.dtype != torch.float32:
+                    y = ops.dimq_conv2d_a4(x, self.packed_weight, self.codebook, self.act_scale, self.act_zero_point,
+                                           self.bias, self.weight_shape, self.stride, self.padding, self.dilation,
+                                           self.groups, out_dtype=self.out_dtype, epilogue=self.epilogue,
+                                           residual=residual, packed_khwc=khwc)
+                    if y is not None:
+                        return y
+                # centred activation codes times the scaled codebook through the weight-only implicit-GEMM path,
+                # with the re-ordered indices and the scaled codebook cached on the module
                 codes = ops.centre_quantize_u4(x, self.act_scale, self.act_zero_point)
                 return ops.dimq_conv2d_wq(codes, self.packed_weight, self._scaled_codebook(), self.bias,
                                           self.weight_shape, self.stride, self.padding, self.dilation, self.groups,
@@ -184,6 +201,13 @@ class DIMQConv2d(_PackedBase):
         if residual is not None or self.epilogue is not None:
             raise RuntimeError("a fused epilogue or residual needs the weight-only mode, or channels_last input "
                                f"with at least {ops.A4_TC_MIN_ROWS} output pixels")
+        if khwc is not None and x.dim() == 4:
+            # NCHW activations, or few pixels: the re-ordered indices are kept here, not re-derived per call
+            y = ops.dimq_conv2d_a4(x, self.packed_weight, self.codebook, self.act_scale, self.act_zero_point, self.bias,
+                                   self.weight_shape, self.stride, self.padding, self.dilation, self.groups,
+                                   packed_khwc=khwc)
+            if y is not None:
+                return y
         return ops.dimq_conv2d_lut(x, self.packed_weight, self.codebook, self.act_scale, self.act_zero_point,
                                    self.bias, self.weight_shape, self.stride, self.padding, self.dilation,
                                    self.groups)

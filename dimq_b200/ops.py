@@ -133,10 +133,65 @@ def _bias_arg(bias: torch.Tensor | None, n: int, device: torch.device, what: str
     return b, _lib.dtype_code(b, "bias")
 
 
-# W4A4 problems with at least this many activation rows (output pixels for the convolution) take the
-# tensor-core path (operands rounded to a hi + lo bf16 pair); smaller ones the exact table-lookup kernel.
+# W4A4 layers run on the tensor cores at fp32 grade (_linear_a4 / _conv2d_a4) wherever the reduction is a multiple of
+# 64 and the output rows of 16 bytes.  Of what is left, problems with at least this many activation rows (output
+# pixels for the convolution) take the kernels with codewords rounded to a hi + lo bf16 pair, the rest the exact
+# table-lookup kernel; a fused epilogue or residual needs this many rows in either case.
 A4_TC_MIN_ROWS = 512
 _UNSUPPORTED = -7
+
+
+def _a4_weight(pw: torch.Tensor, cb: torch.Tensor, rows: int, khwc: torch.Tensor | None = None) -> _lib.WqWeight:
+    return _lib.WqWeight(pw.data_ptr(), 4, cb.data_ptr(), _lib.dtype_code(cb, "codebook"), 16, 1, rows,
+                         0 if khwc is None else khwc.data_ptr())
+
+
+def _linear_a4(xc, pw, cb, act_scale, act_zp, b, b_dt, res, y, m, n, k, epilogue) -> bool:
+    """The fp32-grade tensor-core form into ``y`` (checked, contiguous tensors); False where it does not apply."""
+    w = _a4_weight(pw, cb, n)
+    need = C.c_int64(0)
+    _lib.lib().dimq_linear_a4_workspace_bytes(C.byref(w), _lib.dtype_code(y, "y"), C.c_int64(m), C.c_int64(n),
+                                              C.c_int64(k), C.byref(need))
+    if need.value == 0:
+        return False
+    ws = torch.empty(need.value, dtype=torch.uint8, device=xc.device)
+    with torch.cuda.device(xc.device):
+        st = _lib.lib().dimq_linear_a4(_lib.ptr(xc), _lib.dtype_code(xc, "x"), C.byref(w), C.c_float(act_scale),
+                                       C.c_int(act_zp), _lib.ptr(b), b_dt, _lib.ptr(res), _lib.ptr(y),
+                                       _lib.dtype_code(y, "y"), C.c_int64(m), C.c_int64(n), C.c_int64(k),
+                                       _EPILOGUES[epilogue], _lib.ptr(ws), C.c_int64(need.value),
+                                       _lib.stream_ptr(xc.device))
+    if st == _UNSUPPORTED:
+        return False
+    _lib.check(st, "linear_a4")
+    _lib.LAUNCH_COUNT[0] += 1  # the operand preparation and the GEMM
+    return True
+
+
+def _conv2d_a4(xc, pw, cb, act_scale, act_zp, b, b_dt, res, y, g, epilogue, khwc=None) -> bool:
+    """The same for the convolution; ``khwc`` holds the re-ordered indices where the caller keeps them."""
+    if g.groups != 1 or g.in_channels % 64 != 0:
+        return False
+    own = khwc if khwc is not None else pw          # a stand-in for the size query
+    w = _a4_weight(pw, cb, g.out_channels, own)
+    need = C.c_int64(0)
+    _lib.lib().dimq_conv2d_a4_workspace_bytes(C.byref(w), _lib.dtype_code(y, "y"), C.byref(g), C.byref(need))
+    if need.value == 0:
+        return False
+    if khwc is None:
+        khwc = conv_prepack(pw, (g.out_channels, g.in_channels, g.kernel_h, g.kernel_w), 4)
+        w = _a4_weight(pw, cb, g.out_channels, khwc)
+    ws = torch.empty(need.value, dtype=torch.uint8, device=xc.device)
+    with torch.cuda.device(xc.device):
+        st = _lib.lib().dimq_conv2d_a4(_lib.ptr(xc), _lib.dtype_code(xc, "x"), C.byref(w), C.c_float(act_scale),
+                                       C.c_int(act_zp), _lib.ptr(b), b_dt, _lib.ptr(res), _lib.ptr(y),
+                                       _lib.dtype_code(y, "y"), C.byref(g), _EPILOGUES[epilogue], _lib.ptr(ws),
+                                       C.c_int64(need.value), _lib.stream_ptr(xc.device))
+    if st == _UNSUPPORTED:
+        return False
+    _lib.check(st, "conv2d_a4")
+    _lib.LAUNCH_COUNT[0] += 1  # the operand preparation and the convolution
+    return True
 
 
 def _a4_workspace(x_numel: int, conv_weight_numel: int, device: torch.device) -> torch.Tensor:
@@ -193,6 +248,8 @@ def _linear_lut_impl(x, packed_w, codebook, act_scale, act_zp, bias, out_feature
     b, b_dt = _bias_arg(bias, out_features, xc.device, "out_features")
     m = xc.numel() // in_features
     y = torch.empty((m, out_features), dtype=torch.float32, device=xc.device)
+    if _linear_a4(xc, pw, cb, act_scale, act_zp, b, b_dt, None, y, m, out_features, in_features, None):
+        return y.view(*x.shape[:-1], out_features)
     if m >= A4_TC_MIN_ROWS and in_features % 64 == 0 and pw.data_ptr() % 16 == 0:
         ws = _a4_workspace(xc.numel(), 0, xc.device)
         with torch.cuda.device(xc.device):
@@ -282,6 +339,8 @@ def _conv2d_lut_impl(x, packed_w, codebook, act_scale, act_zp, bias, out_channel
         return y
     pw = packed_w.contiguous().view(-1)
     cb = codebook.contiguous().view(-1)
+    if _conv2d_a4(xc, pw, cb, act_scale, act_zp, b, b_dt, None, y, g, None):
+        return y
     channels_last = g.x_stride[1] == 1 and g.y_stride[1] == 1
     if (channels_last and groups == 1 and g.in_channels % 64 == 0
             and g.batch * g.out_h * g.out_w >= A4_TC_MIN_ROWS):
@@ -701,6 +760,62 @@ def dimq_conv2d_wq(x: torch.Tensor, packed_weight: torch.Tensor, codebooks: torc
                                        _EPILOGUES[epilogue], _ALGOS[algo], _lib.stream_ptr(x.device))
     _lib.check(st, "conv2d_wq")
     del keep
+    return y
+
+
+def dimq_linear_a4(x: torch.Tensor, packed_weight: torch.Tensor, codebook: torch.Tensor, act_scale: float,
+                   act_zero_point: int, bias: torch.Tensor | None, out_features: int, in_features: int, *,
+                   out_dtype: torch.dtype | None = None, epilogue: str | None = None,
+                   residual: torch.Tensor | None = None) -> torch.Tensor | None:
+    """W4A4 linear with an output type, epilogue and residual as in :func:`dimq_linear_wq`, on the tensor cores at
+    fp32 grade; ``None`` where that form does not apply (K not a multiple of 64, output rows not of 16 bytes)."""
+    require_extension()
+    _require_cuda(x, "linear_a4")
+    if not x.is_floating_point():
+        raise RuntimeError("linear_a4 expects floating input")
+    _check_qparams(act_scale, act_zero_point)
+    if x.dim() == 0 or x.size(-1) != in_features:
+        raise RuntimeError("input last dimension must equal in_features")
+    _, (pw, cb, _) = _wq_weight(packed_weight, codebook, 4, out_features, out_features * in_features, None)
+    xc = x.contiguous()
+    b, b_dt = _bias_arg(bias, out_features, xc.device, "out_features")
+    m = xc.numel() // in_features
+    y = torch.empty((m, out_features), dtype=out_dtype or torch.float32, device=xc.device)
+    res = None
+    if residual is not None:
+        if residual.dtype != y.dtype or residual.numel() != y.numel():
+            raise RuntimeError("residual must match the output shape and dtype")
+        res = residual.contiguous()
+    if not _linear_a4(xc, pw, cb, act_scale, act_zero_point, b, b_dt, res, y, m, out_features, in_features, epilogue):
+        return None
+    return y.view(*x.shape[:-1], out_features)
+
+
+def dimq_conv2d_a4(x: torch.Tensor, packed_weight: torch.Tensor, codebook: torch.Tensor, act_scale: float,
+                   act_zero_point: int, bias: torch.Tensor | None, weight_shape: Sequence[int], stride=(1, 1),
+                   padding=(0, 0), dilation=(1, 1), groups: int = 1, *, out_dtype: torch.dtype | None = None,
+                   epilogue: str | None = None, residual: torch.Tensor | None = None,
+                   packed_khwc: torch.Tensor | None = None) -> torch.Tensor | None:
+    """The same for the convolution (channels_last or NCHW storage, the output in the input's format; NCHW takes an
+    fp32 output and no residual).  ``packed_khwc``: the indices re-ordered by :func:`conv_prepack`, if kept."""
+    require_extension()
+    _require_cuda(x, "conv2d_a4")
+    if x.dim() != 4:
+        raise RuntimeError("conv2d_a4 expects NCHW input")
+    if not x.is_floating_point():
+        raise RuntimeError("conv2d_a4 expects floating input")
+    _check_qparams(act_scale, act_zero_point)
+    g = _conv_geom(x, weight_shape, _pair(stride), _pair(padding), _pair(dilation), groups)
+    numel = g.out_channels * g.in_channels_per_group * g.kernel_h * g.kernel_w
+    _, (pw, cb, khwc) = _wq_weight(packed_weight, codebook, 4, g.out_channels, numel, None, packed_khwc)
+    b, b_dt = _bias_arg(bias, g.out_channels, x.device, "out_channels")
+    xc, y = _conv_io(x, g, out_dtype or torch.float32)
+    if y.numel() == 0:
+        return y
+    if residual is not None and (residual.dtype != y.dtype or residual.shape != y.shape or residual.stride() != y.stride()):
+        raise RuntimeError("residual must match the output shape, dtype and memory format")
+    if not _conv2d_a4(xc, pw, cb, act_scale, act_zero_point, b, b_dt, residual, y, g, epilogue, khwc):
+        return None
     return y
 
 

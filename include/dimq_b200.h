@@ -209,7 +209,7 @@ DIMQ_API int dimq_conv2d_wq_static(const void* x, int x_dtype, const dimq_wq_wei
                                    int bias_dtype, const void* residual, void* y, int y_dtype,
                                    const dimq_conv_geom* geom, int epilogue, void* stream);
 
-/* dimq_linear_wq with caller-owned scratch memory, which three regimes use:
+/* dimq_linear_wq with caller-owned scratch memory, which four regimes use:
  *  - a few activation rows (M <= 16, 16-bit x) against 2 MB of 2- to 4-bit indices or more, N a multiple
  *    of 16 and K of 128, K >= 2048: the register-resident small-M kernel cuts K into slices of 2048 worked on by
  *    different CTAs, each writes its partial sums to the workspace (slices * M * N * 4 bytes, at most 8
@@ -224,6 +224,9 @@ DIMQ_API int dimq_conv2d_wq_static(const void* x, int x_dtype, const dimq_wq_wei
  *    in-pipeline tcgen05 kernel cuts K into slices (split-K), adds the partial sums into the workspace
  *    (M*N*4 bytes, float atomics: the last bits can differ from run to run) and a second small kernel
  *    applies bias / epilogue / residual.
+ *  - fp32 activations and output, more than 8 rows, 2- to 4-bit indices, K a multiple of 64: activations and
+ *    codewords are split into fp16 terms (2*M*K + up to 2*N*K halves) and multiplied on the tensor cores at fp32
+ *    grade; with too small a workspace the fp32 SIMT kernel runs instead.
  * dimq_linear_wq_workspace_bytes reports the bytes of the regime that applies and 0 otherwise (then
  * dimq_linear_wq_ws is dimq_linear_wq with DIMQ_ALGO_AUTO and the workspace is not touched).  The
  * workspace must be 16-byte aligned; its contents after the call are unspecified.  The reference has no
@@ -307,6 +310,26 @@ DIMQ_API int dimq_conv2d_lut_tc(const void* x, int x_dtype, const uint8_t* packe
                                 int cb_dtype, float act_scale, int act_zp, const void* bias, int bias_dtype,
                                 float* y, const dimq_conv_geom* geom, void* workspace, int64_t workspace_bytes,
                                 void* stream);
+
+/* The W4A4 ops at fp32 grade on the tensor cores, at any number of rows / pixels: activation codes minus the zero
+ * point (integers in [-15, 15]) and codewords as fp16 operands - one term per codeword for an fp16 codebook, one
+ * scaled term for bf16, hi + lo for fp32 - the sums taken out of the tensor-core accumulators every 256 k and added
+ * in fp32, then y = epilogue(act_scale * sum + bias) [+ residual] as in dimq_linear_wq.  w: 4-bit, 16 entries; y any of the three types.
+ * Linear: K a multiple of 64, y rows of a multiple of 16 bytes.  Convolution: w->packed_khwc from
+ * dimq_conv_prepack, groups 1, in_channels a multiple of 64, stride 1 or 2; x and y both packed NHWC, or both packed
+ * NCHW (then y is fp32 and residual null).  The workspace (16-byte aligned) holds the codes and the expanded weight;
+ * *_workspace_bytes reports 0 where the form does not apply (the calls then return DIMQ_ERR_UNSUPPORTED). */
+DIMQ_API int dimq_linear_a4_workspace_bytes(const dimq_wq_weight* w, int y_dtype, int64_t M, int64_t N, int64_t K,
+                                            int64_t* bytes);
+DIMQ_API int dimq_linear_a4(const void* x, int x_dtype, const dimq_wq_weight* w, float act_scale, int act_zp,
+                            const void* bias, int bias_dtype, const void* residual, void* y, int y_dtype, int64_t M,
+                            int64_t N, int64_t K, int epilogue, void* workspace, int64_t workspace_bytes, void* stream);
+DIMQ_API int dimq_conv2d_a4_workspace_bytes(const dimq_wq_weight* w, int y_dtype, const dimq_conv_geom* geom,
+                                            int64_t* bytes);
+DIMQ_API int dimq_conv2d_a4(const void* x, int x_dtype, const dimq_wq_weight* w, float act_scale, int act_zp,
+                            const void* bias, int bias_dtype, const void* residual, void* y, int y_dtype,
+                            const dimq_conv_geom* geom, int epilogue, void* workspace, int64_t workspace_bytes,
+                            void* stream);
 
 /* ---- dense helper of the whole-model harness --------------------------- */
 

@@ -1,0 +1,148 @@
+"""GPU parity of the fp32-grade tensor-core forms (W4A4 codes, fp32 activations) against 64-bit references.
+
+Tolerance: both forms carry the operands to 2^-23 of each product and add fp32 partial sums of 256 k; the bound
+used, 6e-7 of the result's norm, is four roundings of 2^-23 and a third over the 4.6e-7 that sequential fp32 FMAs
+show at K = 768.
+"""
+
+from __future__ import annotations
+
+import pytest
+import torch
+import torch.nn.functional as F
+
+pytestmark = pytest.mark.gpu
+
+REL = 6e-7
+
+
+@pytest.fixture(scope="module")
+def ops(cuda_device):
+    from dimq_b200 import ops as _ops
+
+    _ops.require_extension()
+    return _ops
+
+
+def _rel(y, want):
+    return float((y.double() - want).norm() / want.norm())
+
+
+def _weight(ops, n, k, bits, dtype, group_rows=None, seed=0):
+    gen = torch.Generator(device="cuda").manual_seed(seed)
+    groups = 1 if group_rows is None else (n + group_rows - 1) // group_rows
+    # codebooks of very different sizes, so that the scale of every group counts
+    books = torch.randn(groups, 1 << bits, device="cuda", generator=gen) * 0.02
+    books = (books * 4.0 ** torch.arange(groups, device="cuda").view(-1, 1)).to(dtype)
+    idx = torch.randint(0, 1 << bits, (n, k), device="cuda", generator=gen, dtype=torch.uint8)
+    rows = torch.arange(n, device="cuda") // (group_rows or n)
+    return ops.pack_bits(idx, bits), books, torch.gather(books.double()[rows], 1, idx.long())
+
+
+def _codes(x, scale, zp):
+    q = torch.round(x.float() / torch.tensor(scale, device=x.device)) + zp
+    return (q.clamp(0, 15) - zp).double() * torch.tensor(scale, dtype=torch.float32).double().item()
+
+
+@pytest.mark.parametrize("m,k,n", [(1, 64, 4), (127, 192, 68), (129, 320, 132), (300, 1024, 1000), (1576, 768, 260)])
+@pytest.mark.parametrize("book", [torch.float16, torch.bfloat16, torch.float32])
+def test_linear_a4(ops, m, k, n, book):
+    packed, books, w = _weight(ops, n, k, 4, book, seed=m)
+    x = torch.randn(m, k, device="cuda").to(torch.float16 if m == 127 else torch.float32)
+    bias = torch.randn(n, device="cuda")
+    y = ops.dimq_linear_lut(x, packed, books.reshape(-1), 0.23, 7, bias, n, k)
+    assert y.dtype == torch.float32 and ops.last_device_status() == 0
+    assert _rel(y, _codes(x, 0.23, 7) @ w.t() + bias.double()) < REL
+
+
+def test_linear_a4_long_sums(ops):
+    # one-signed codes and codewords at K = 8192: sums far beyond 24 bits
+    packed, books, w = _weight(ops, 128, 8192, 4, torch.float16, seed=3)
+    books, w = books.abs(), w.abs()
+    x = torch.rand(200, 8192, device="cuda") * 3
+    y = ops.dimq_linear_lut(x, packed, books.reshape(-1), 0.2, 0, None, 128, 8192)
+    assert _rel(y, _codes(x, 0.2, 0) @ w.t()) < REL
+
+
+@pytest.mark.parametrize("epilogue,out", [("gelu", torch.float32), ("add_relu", torch.bfloat16), ("relu", torch.float16)])
+def test_linear_a4_epilogues(ops, epilogue, out):
+    m, k, n = 515, 256, 200
+    packed, books, w = _weight(ops, n, k, 4, torch.float32, seed=9)
+    x, res = torch.randn(m, k, device="cuda"), torch.randn(m, n, device="cuda").to(out)
+    y = ops.dimq_linear_a4(x, packed, books.reshape(-1), 0.25, 8, None, n, k, out_dtype=out, epilogue=epilogue, residual=res)
+    z = _codes(x, 0.25, 8) @ w.t()
+    r = res.double()
+    want = {"gelu": F.gelu(z) + r, "relu": z.relu() + r, "add_relu": (z + r).relu()}[epilogue]
+    assert y.dtype == out and _rel(y, want) < {torch.float32: REL, torch.bfloat16: 2.0 ** -9, torch.float16: 2.0 ** -12}[out]
+
+
+@pytest.mark.parametrize("batch,cin,cout,h,w_,ks,stride,pad", [
+    (1, 64, 64, 1, 1, 1, 1, 0), (2, 64, 60, 7, 9, 3, 1, 1), (7, 128, 128, 28, 28, 3, 1, 1), (3, 64, 129, 15, 13, 3, 2, 1),
+    (5, 192, 256, 14, 14, 1, 2, 0), (2, 512, 64, 7, 7, 3, 1, 1)])
+@pytest.mark.parametrize("nhwc", [False, True])
+@pytest.mark.parametrize("book", [torch.float16, torch.float32])
+def test_conv2d_a4(ops, batch, cin, cout, h, w_, ks, stride, pad, nhwc, book):
+    packed, books, w = _weight(ops, cout, cin * ks * ks, 4, book, seed=cin + ks)
+    x = torch.randn(batch, cin, h, w_, device="cuda").relu_()
+    if nhwc:
+        x = x.contiguous(memory_format=torch.channels_last)
+    bias = torch.randn(cout, device="cuda")
+    y = ops.dimq_conv2d_lut(x, packed, books.reshape(-1), 0.28, 0, bias, (cout, cin, ks, ks), (stride, stride), (pad, pad),
+                            (1, 1), 1)
+    assert ops.last_device_status() == 0 and y.is_contiguous(memory_format=torch.channels_last if nhwc else torch.contiguous_format)
+    want = F.conv2d(_codes(x.contiguous(), 0.28, 0), w.view(cout, cin, ks, ks), bias.double(), stride, pad)
+    assert _rel(y, want) < REL
+
+
+@pytest.mark.parametrize("m,k,n", [(9, 64, 4), (128, 128, 128), (197, 768, 1000), (130, 3072, 68)])
+@pytest.mark.parametrize("bits,group_rows,book", [(4, None, torch.float32), (3, 16, torch.float32), (2, 128, torch.float16),
+                                                  (4, 1, torch.bfloat16)])
+def test_linear_f32(ops, m, k, n, bits, group_rows, book):
+    if book == torch.float16 and n > 4 * 128:
+        group_rows = 512                        # keeps the last group's codewords inside fp16
+    if group_rows is not None and n // group_rows > 24:
+        group_rows = (n + 23) // 24
+    packed, books, w = _weight(ops, n, k, bits, book, group_rows, seed=m + bits)
+    x = torch.randn(m, k, device="cuda") * 10.0 ** torch.linspace(-12, 12, m, device="cuda").view(-1, 1)
+    bias = torch.randn(n, device="cuda")
+    y = ops.dimq_linear_wq(x, packed, books, None, n, k, bits=bits, group_rows=group_rows)
+    assert ops.last_device_status() == 0
+    want = x.double() @ w.t()
+    # row by row and group by group: neither a large row nor a large group may hide a small one
+    err = (y.double() - want).view(m, n)
+    gr = group_rows or n
+    for g0 in range(0, n, gr):
+        # the norm of |x| |w| / sqrt(k), not of the result: a row's few columns of one group may cancel, and rounding
+        # errors follow the products.  The worst of 197 rows lies within 4 standard deviations.
+        e = err[:, g0:g0 + gr].norm(dim=1)
+        r = x.double().norm(dim=1) * w[g0:g0 + gr].norm() / k ** 0.5
+        assert float((e / r).max()) < 4 * REL
+    y2 = ops.dimq_linear_wq(x[:, :], packed, books, bias, n, k, bits=bits, group_rows=group_rows, epilogue="relu")
+    # one row dominates this norm, and its few columns may cancel: rounding errors follow the products here too
+    scale = float((x.double().norm() * w.norm() / k ** 0.5).clamp_min(1.0))
+    assert float((y2.double() - (want + bias.double()).relu()).norm()) < REL * scale
+
+
+def test_linear_f32_non_finite(ops):
+    m, k, n = 40, 128, 64
+    packed, books, w = _weight(ops, n, k, 4, torch.float32, seed=1)
+    x = torch.randn(m, k, device="cuda")
+    x[3, 5], x[7, 9], x[11, 2] = float("inf"), float("-inf"), float("nan")
+    x[20] = 0.0
+    x[21] *= 1e30
+    y = ops.dimq_linear_wq(x, packed, books, None, n, k, bits=4)
+    want = x @ w.float().t()
+    assert torch.equal(y.isnan(), want.isnan()) and torch.equal(y.isinf(), want.isinf())
+    ok = want.isfinite()
+    assert torch.equal(y[~ok & ~want.isnan()].sign(), want[~ok & ~want.isnan()].sign())
+    rows = ok.all(1)                                     # the rows without a non-finite element
+    bound = 1e-5 * x[rows].double().norm(dim=1, keepdim=True) * w.norm(dim=1)
+    assert bool(((y[rows] - want[rows]).abs() <= bound).all())
+    # an infinite codeword
+    bad = books.clone()
+    bad[0, 3] = float("inf")
+    hit = torch.isinf(bad.double()[torch.zeros(n, device="cuda", dtype=torch.long)].gather(
+        1, torch.stack([(packed.view(n, -1) & 15), (packed.view(n, -1) >> 4)], 2).view(n, k).long())).any(1)
+    x = torch.rand(m, k, device="cuda") + 0.5
+    y = ops.dimq_linear_wq(x, packed, bad, None, n, k, bits=4)
+    assert torch.equal(y.isinf().all(0), hit) and bool(y[:, ~hit].isfinite().all())
