@@ -7,6 +7,7 @@ missing or an entry point reports an error, a ``RuntimeError`` is raised.
 from __future__ import annotations
 
 import ctypes as C
+import importlib.util
 from functools import lru_cache
 from pathlib import Path
 
@@ -64,10 +65,24 @@ def lib() -> C.CDLL:
     return handle
 
 
+@lru_cache(maxsize=1)
+def host():
+    """The native host path (``csrc/host.cpp``); raises like :func:`lib` if it was not built."""
+    lib()
+    path = PKG / "_host.so"
+    if not path.exists():
+        raise RuntimeError(f"{path} is missing: build it with `python -m dimq_b200.build`.  dimq_b200 has no fallback.")
+    spec = importlib.util.spec_from_file_location("dimq_b200._host", path)
+    module = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(module)
+    module.set_launch_count(LAUNCH_COUNT)
+    return module
+
+
 def is_available() -> bool:
     try:
-        lib()
-    except (RuntimeError, OSError):
+        host()
+    except (RuntimeError, OSError, ImportError):
         return False
     return True
 

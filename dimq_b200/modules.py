@@ -20,7 +20,14 @@ from typing import Any, Mapping
 import torch
 import torch.nn as nn
 
-from . import ops
+from . import _lib, ops
+
+
+def _eager(x: torch.Tensor) -> bool:
+    """Plain eager execution: no tracer, dispatch mode, tensor subclass or function transform that has to see the
+    registered operator."""
+    return (type(x) is torch.Tensor and torch._C._len_torch_dispatch_stack() == 0 and not torch._C._is_tracing()
+            and torch._C._functorch.peek_interpreter_stack() is None)
 
 
 def _pair(value) -> tuple[int, int]:
@@ -62,9 +69,8 @@ class _PackedBase(nn.Module):
     def _check_input(self, x: torch.Tensor) -> None:
         if not self.use_cuda_kernel:
             raise RuntimeError("dimq_b200 has no Python fallback path (use_cuda_kernel=False is not supported)")
-        if not (x.is_cuda and self.packed_weight.is_cuda):
+        if not (x.is_cuda and self._buffers["packed_weight"].is_cuda):
             raise RuntimeError("dimq_b200 layers run on CUDA tensors only; move the module and its input to a B200")
-        ops.require_extension()
 
 
 class DIMQLinear(_PackedBase):
@@ -100,11 +106,11 @@ class DIMQLinear(_PackedBase):
     def forward(self, x: torch.Tensor, residual: torch.Tensor | None = None) -> torch.Tensor:
         self._check_input(x)
         if self.act_scale is None:
+            buf = self._buffers
             tiled = self._prepacked(x.numel() // self.in_features, x)
-            return ops.dimq_linear_wq(x, self.packed_weight, self.codebook, self.bias, self.out_features,
-                                      self.in_features, bits=self.bits, group_rows=self.group_rows,
-                                      out_dtype=self.out_dtype, epilogue=self.epilogue, residual=residual,
-                                      packed_tiled=tiled)
+            return _lib.host().linear_wq(x, buf["packed_weight"], buf["codebook"], buf["bias"], self.out_features,
+                                         self.in_features, self.bits, self.group_rows, self.out_dtype,
+                                         ops._EPILOGUES[self.epilogue], residual, tiled)
         rows = x.numel() // self.in_features
         if rows >= ops.A4_TC_MIN_ROWS and self.in_features % 64 == 0:
             # The fp32-grade form, except for an fp32 codebook on many rows: there it multiplies two fp16 terms in
@@ -162,7 +168,7 @@ class DIMQConv2d(_PackedBase):
     def _prepacked(self) -> torch.Tensor | None:
         if self.groups != 1 or self.weight_shape[1] % 64 != 0:
             return None
-        pw = self.packed_weight
+        pw = self._buffers["packed_weight"]
         key = (pw.data_ptr(), pw._version, pw.device)
         if self._khwc is None or self._khwc_key != key:
             self._khwc = ops.conv_prepack(pw, self.weight_shape, self.bits)
@@ -172,10 +178,11 @@ class DIMQConv2d(_PackedBase):
     def forward(self, x: torch.Tensor, residual: torch.Tensor | None = None) -> torch.Tensor:
         self._check_input(x)
         if self.act_scale is None:
-            return ops.dimq_conv2d_wq(x, self.packed_weight, self.codebook, self.bias, self.weight_shape,
-                                      self.stride, self.padding, self.dilation, self.groups, bits=self.bits,
-                                      group_rows=self.group_rows, out_dtype=self.out_dtype, epilogue=self.epilogue,
-                                      residual=residual, packed_khwc=self._prepacked())
+            buf = self._buffers
+            return _lib.host().conv2d_wq(x, buf["packed_weight"], buf["codebook"], buf["bias"], self.weight_shape,
+                                         self.stride, self.padding, self.dilation, self.groups, self.bits,
+                                         self.group_rows, self.out_dtype, ops._EPILOGUES[self.epilogue], residual,
+                                         self._prepacked())
         khwc = self._prepacked()
         channels_last = x.dim() == 4 and x.is_contiguous(memory_format=torch.channels_last) and not x.is_contiguous()
         if khwc is not None and channels_last and self.stride[0] == self.stride[1] and self.stride[0] in (1, 2):
@@ -201,7 +208,7 @@ class DIMQConv2d(_PackedBase):
         if residual is not None or self.epilogue is not None:
             raise RuntimeError("a fused epilogue or residual needs the weight-only mode, or channels_last input "
                                f"with at least {ops.A4_TC_MIN_ROWS} output pixels")
-        if khwc is not None and x.dim() == 4:
+        if khwc is not None and x.dim() == 4 and _eager(x):
             # NCHW activations, or few pixels: the re-ordered indices are kept here, not re-derived per call
             y = ops.dimq_conv2d_a4(x, self.packed_weight, self.codebook, self.act_scale, self.act_zero_point, self.bias,
                                    self.weight_shape, self.stride, self.padding, self.dilation, self.groups,

@@ -52,42 +52,11 @@ def _pair(value) -> tuple[int, int]:
 # ---------------------------------------------------------------------------
 
 def _pack_bits_impl(indices: torch.Tensor, bits: int) -> torch.Tensor:
-    _require_cuda(indices, "pack")
-    if indices.dtype != torch.uint8:
-        raise RuntimeError("pack expects uint8 indices")
-    flat = indices.contiguous().view(-1)
-    n = flat.numel()
-    packed = torch.empty(((n * bits + 7) // 8,), dtype=torch.uint8, device=flat.device)
-    with torch.cuda.device(flat.device):
-        st = _lib.lib().dimq_pack_bits(_lib.ptr(flat), C.c_int64(n), C.c_int(bits), _lib.ptr(packed),
-                                       _lib.stream_ptr(flat.device))
-    _lib.check(st, "pack_bits")
-    return packed
+    return _lib.host().pack_bits(indices, bits)
 
 
 def _unpack_bits_impl(packed: torch.Tensor, numel: int, bits: int) -> torch.Tensor:
-    _require_cuda(packed, "unpack")
-    if packed.dtype != torch.uint8:
-        raise RuntimeError("unpack expects uint8 packed data")
-    if numel < 0:
-        raise RuntimeError("numel must be non-negative")
-    if packed.numel() < (numel * bits + 7) // 8:
-        raise RuntimeError("packed tensor is too small for requested numel")
-    flat = packed.contiguous().view(-1)
-    out = torch.empty((numel,), dtype=torch.uint8, device=flat.device)
-    with torch.cuda.device(flat.device):
-        st = _lib.lib().dimq_unpack_bits(_lib.ptr(flat), C.c_int64(numel), C.c_int(bits), _lib.ptr(out),
-                                         _lib.stream_ptr(flat.device))
-    _lib.check(st, "unpack_bits")
-    return out
-
-
-def _pack_u4_impl(indices: torch.Tensor) -> torch.Tensor:
-    return _pack_bits_impl(indices, 4)
-
-
-def _unpack_u4_impl(packed: torch.Tensor, numel: int) -> torch.Tensor:
-    return _unpack_bits_impl(packed, int(numel), 4)
+    return _lib.host().unpack_bits(packed, numel, bits)
 
 
 def _check_qparams(act_scale: float, act_zp: int) -> None:
@@ -133,73 +102,11 @@ def _bias_arg(bias: torch.Tensor | None, n: int, device: torch.device, what: str
     return b, _lib.dtype_code(b, "bias")
 
 
-# W4A4 layers run on the tensor cores at fp32 grade (_linear_a4 / _conv2d_a4) wherever the reduction is a multiple of
-# 64 and the output rows of 16 bytes.  Of what is left, problems with at least this many activation rows (output
-# pixels for the convolution) take the kernels with codewords rounded to a hi + lo bf16 pair, the rest the exact
+# W4A4 layers run on the tensor cores at fp32 grade (dimq_linear_a4 / dimq_conv2d_a4) wherever the reduction is a
+# multiple of 64 and the output rows of 16 bytes.  Of what is left, problems with at least this many activation rows
+# (output pixels for the convolution) take the kernels with codewords rounded to a hi + lo bf16 pair, the rest the exact
 # table-lookup kernel; a fused epilogue or residual needs this many rows in either case.
 A4_TC_MIN_ROWS = 512
-_UNSUPPORTED = -7
-
-
-def _a4_weight(pw: torch.Tensor, cb: torch.Tensor, rows: int, khwc: torch.Tensor | None = None) -> _lib.WqWeight:
-    return _lib.WqWeight(pw.data_ptr(), 4, cb.data_ptr(), _lib.dtype_code(cb, "codebook"), 16, 1, rows,
-                         0 if khwc is None else khwc.data_ptr())
-
-
-def _linear_a4(xc, pw, cb, act_scale, act_zp, b, b_dt, res, y, m, n, k, epilogue) -> bool:
-    """The fp32-grade tensor-core form into ``y`` (checked, contiguous tensors); False where it does not apply."""
-    w = _a4_weight(pw, cb, n)
-    need = C.c_int64(0)
-    _lib.lib().dimq_linear_a4_workspace_bytes(C.byref(w), _lib.dtype_code(y, "y"), C.c_int64(m), C.c_int64(n),
-                                              C.c_int64(k), C.byref(need))
-    if need.value == 0:
-        return False
-    ws = torch.empty(need.value, dtype=torch.uint8, device=xc.device)
-    with torch.cuda.device(xc.device):
-        st = _lib.lib().dimq_linear_a4(_lib.ptr(xc), _lib.dtype_code(xc, "x"), C.byref(w), C.c_float(act_scale),
-                                       C.c_int(act_zp), _lib.ptr(b), b_dt, _lib.ptr(res), _lib.ptr(y),
-                                       _lib.dtype_code(y, "y"), C.c_int64(m), C.c_int64(n), C.c_int64(k),
-                                       _EPILOGUES[epilogue], _lib.ptr(ws), C.c_int64(need.value),
-                                       _lib.stream_ptr(xc.device))
-    if st == _UNSUPPORTED:
-        return False
-    _lib.check(st, "linear_a4")
-    _lib.LAUNCH_COUNT[0] += 1  # the operand preparation and the GEMM
-    return True
-
-
-def _conv2d_a4(xc, pw, cb, act_scale, act_zp, b, b_dt, res, y, g, epilogue, khwc=None) -> bool:
-    """The same for the convolution; ``khwc`` holds the re-ordered indices where the caller keeps them."""
-    if g.groups != 1 or g.in_channels % 64 != 0:
-        return False
-    own = khwc if khwc is not None else pw          # a stand-in for the size query
-    w = _a4_weight(pw, cb, g.out_channels, own)
-    need = C.c_int64(0)
-    _lib.lib().dimq_conv2d_a4_workspace_bytes(C.byref(w), _lib.dtype_code(y, "y"), C.byref(g), C.byref(need))
-    if need.value == 0:
-        return False
-    if khwc is None:
-        khwc = conv_prepack(pw, (g.out_channels, g.in_channels, g.kernel_h, g.kernel_w), 4)
-        w = _a4_weight(pw, cb, g.out_channels, khwc)
-    ws = torch.empty(need.value, dtype=torch.uint8, device=xc.device)
-    with torch.cuda.device(xc.device):
-        st = _lib.lib().dimq_conv2d_a4(_lib.ptr(xc), _lib.dtype_code(xc, "x"), C.byref(w), C.c_float(act_scale),
-                                       C.c_int(act_zp), _lib.ptr(b), b_dt, _lib.ptr(res), _lib.ptr(y),
-                                       _lib.dtype_code(y, "y"), C.byref(g), _EPILOGUES[epilogue], _lib.ptr(ws),
-                                       C.c_int64(need.value), _lib.stream_ptr(xc.device))
-    if st == _UNSUPPORTED:
-        return False
-    _lib.check(st, "conv2d_a4")
-    _lib.LAUNCH_COUNT[0] += 1  # the operand preparation and the convolution
-    return True
-
-
-def _a4_workspace(x_numel: int, conv_weight_numel: int, device: torch.device) -> torch.Tensor:
-    need = C.c_int64(0)
-    st = _lib.lib().dimq_a4_workspace_bytes(C.c_int64(x_numel), C.c_int64(conv_weight_numel), C.byref(need))
-    if st != 0:
-        raise RuntimeError(f"dimq_b200.a4_workspace_bytes failed (status {st})")
-    return torch.empty(need.value, dtype=torch.uint8, device=device)
 
 
 def centre_quantize_u4(x: torch.Tensor, act_scale: float, act_zero_point: int) -> torch.Tensor:
@@ -219,56 +126,6 @@ def centre_quantize_u4(x: torch.Tensor, act_scale: float, act_zero_point: int) -
                                                 _lib.stream_ptr(xc.device))
     _lib.check(st, "centre_quantize_u4")
     return out
-
-
-def _linear_lut_impl(x, packed_w, codebook, act_scale, act_zp, bias, out_features, in_features):
-    _require_cuda(x, "linear_lut")
-    _require_cuda(packed_w, "linear_lut")
-    _require_cuda(codebook, "linear_lut")
-    if not x.is_floating_point():
-        raise RuntimeError("linear_lut expects floating input")
-    if packed_w.dtype != torch.uint8:
-        raise RuntimeError("packed_weight must be uint8")
-    if not codebook.is_floating_point():
-        raise RuntimeError("codebook must be floating point")
-    if codebook.numel() != 16:
-        raise RuntimeError("codebook must have 16 entries for W4")
-    _check_qparams(act_scale, act_zp)
-    if out_features <= 0 or in_features <= 0:
-        raise RuntimeError("linear dimensions must be positive")
-    if x.numel() % in_features != 0:
-        raise RuntimeError("input numel must be divisible by in_features")
-    if packed_w.numel() < (out_features * in_features + 1) // 2:
-        raise RuntimeError("packed_weight is too small for out_features * in_features")
-    if x.dim() == 0 or x.size(-1) != in_features:
-        raise RuntimeError("input last dimension must equal in_features")
-    xc = x.contiguous()
-    pw = packed_w.contiguous().view(-1)
-    cb = codebook.contiguous().view(-1)
-    b, b_dt = _bias_arg(bias, out_features, xc.device, "out_features")
-    m = xc.numel() // in_features
-    y = torch.empty((m, out_features), dtype=torch.float32, device=xc.device)
-    if _linear_a4(xc, pw, cb, act_scale, act_zp, b, b_dt, None, y, m, out_features, in_features, None):
-        return y.view(*x.shape[:-1], out_features)
-    if m >= A4_TC_MIN_ROWS and in_features % 64 == 0 and pw.data_ptr() % 16 == 0:
-        ws = _a4_workspace(xc.numel(), 0, xc.device)
-        with torch.cuda.device(xc.device):
-            st = _lib.lib().dimq_linear_lut_tc(_lib.ptr(xc), _lib.dtype_code(xc, "x"), _lib.ptr(pw), _lib.ptr(cb),
-                                               _lib.dtype_code(cb, "codebook"), C.c_float(act_scale), C.c_int(act_zp),
-                                               _lib.ptr(b), b_dt, _lib.ptr(y), C.c_int64(m), C.c_int64(out_features),
-                                               C.c_int64(in_features), _lib.ptr(ws), C.c_int64(ws.numel()),
-                                               _lib.stream_ptr(xc.device))
-        if st != _UNSUPPORTED:
-            _lib.check(st, "linear_lut_tc")
-            _lib.LAUNCH_COUNT[0] += 1  # the activation quantiser and the GEMM
-            return y.view(*x.shape[:-1], out_features)
-    with torch.cuda.device(xc.device):
-        st = _lib.lib().dimq_linear_lut(_lib.ptr(xc), _lib.dtype_code(xc, "x"), _lib.ptr(pw), _lib.ptr(cb),
-                                        _lib.dtype_code(cb, "codebook"), C.c_float(act_scale), C.c_int(act_zp),
-                                        _lib.ptr(b), b_dt, _lib.ptr(y), C.c_int64(m), C.c_int64(out_features),
-                                        C.c_int64(in_features), _lib.stream_ptr(xc.device))
-    _lib.check(st, "linear_lut")
-    return y.view(*x.shape[:-1], out_features)
 
 
 def _conv_geom(x: torch.Tensor, weight_shape, stride, padding, dilation, groups) -> _lib.ConvGeom:
@@ -312,83 +169,42 @@ def _conv_io(x: torch.Tensor, g: _lib.ConvGeom, out_dtype: torch.dtype):
     return xc, y
 
 
-def _conv2d_lut_impl(x, packed_w, codebook, act_scale, act_zp, bias, out_channels, in_channels_per_group,
-                     kernel_h, kernel_w, stride_h, stride_w, pad_h, pad_w, dilation_h, dilation_w, groups):
-    _require_cuda(x, "conv2d_lut")
-    if x.dim() != 4:
-        raise RuntimeError("conv2d_lut expects NCHW input")
-    _require_cuda(packed_w, "conv2d_lut")
-    _require_cuda(codebook, "conv2d_lut")
-    if not x.is_floating_point():
-        raise RuntimeError("conv2d_lut expects floating input")
-    if packed_w.dtype != torch.uint8:
-        raise RuntimeError("packed_weight must be uint8")
-    if not codebook.is_floating_point():
-        raise RuntimeError("codebook must be floating point")
-    if codebook.numel() != 16:
-        raise RuntimeError("codebook must have 16 entries for W4")
-    _check_qparams(act_scale, act_zp)
-    g = _conv_geom(x, (out_channels, in_channels_per_group, kernel_h, kernel_w), (stride_h, stride_w),
-                   (pad_h, pad_w), (dilation_h, dilation_w), groups)
-    numel = out_channels * in_channels_per_group * kernel_h * kernel_w
-    if packed_w.numel() < (numel + 1) // 2:
-        raise RuntimeError("packed_weight is too small for requested conv weight shape")
-    b, b_dt = _bias_arg(bias, out_channels, x.device, "out_channels")
-    xc, y = _conv_io(x, g, torch.float32)
-    if y.numel() == 0:
-        return y
-    pw = packed_w.contiguous().view(-1)
-    cb = codebook.contiguous().view(-1)
-    if _conv2d_a4(xc, pw, cb, act_scale, act_zp, b, b_dt, None, y, g, None):
-        return y
-    channels_last = g.x_stride[1] == 1 and g.y_stride[1] == 1
-    if (channels_last and groups == 1 and g.in_channels % 64 == 0
-            and g.batch * g.out_h * g.out_w >= A4_TC_MIN_ROWS):
-        ws = _a4_workspace(xc.numel(), numel, x.device)
-        with torch.cuda.device(x.device):
-            st = _lib.lib().dimq_conv2d_lut_tc(_lib.ptr(xc), _lib.dtype_code(xc, "x"), _lib.ptr(pw), _lib.ptr(cb),
-                                               _lib.dtype_code(cb, "codebook"), C.c_float(act_scale), C.c_int(act_zp),
-                                               _lib.ptr(b), b_dt, _lib.ptr(y), C.byref(g), _lib.ptr(ws),
-                                               C.c_int64(ws.numel()), _lib.stream_ptr(x.device))
-        if st != _UNSUPPORTED:
-            _lib.check(st, "conv2d_lut_tc")
-            _lib.LAUNCH_COUNT[0] += 2  # index re-order, activation quantiser, convolution
-            return y
-    with torch.cuda.device(x.device):
-        st = _lib.lib().dimq_conv2d_lut(_lib.ptr(xc), _lib.dtype_code(xc, "x"), _lib.ptr(pw), _lib.ptr(cb),
-                                        _lib.dtype_code(cb, "codebook"), C.c_float(act_scale), C.c_int(act_zp),
-                                        _lib.ptr(b), b_dt, _lib.ptr(y), C.byref(g), _lib.stream_ptr(x.device))
-    _lib.check(st, "conv2d_lut")
-    return y
-
-
 # ---------------------------------------------------------------------------
 # torch.ops.dimq registration: the reference's six schemas, CUDA key only
 # ---------------------------------------------------------------------------
 
 _SCHEMAS = (
-    ("pack_u4(Tensor indices) -> Tensor", _pack_u4_impl),
-    ("unpack_u4(Tensor packed, int numel) -> Tensor", _unpack_u4_impl),
-    ("quantize_activation_u4(Tensor x, float act_scale, int act_zp) -> Tensor", _quantize_activation_u4_impl),
-    ("build_product_table(Tensor codebook, float act_scale, int act_zp) -> Tensor", _build_product_table_impl),
-    ("linear_lut(Tensor x, Tensor packed_w, Tensor codebook, float act_scale, int act_zp, Tensor? bias, "
-     "int out_features, int in_features) -> Tensor", _linear_lut_impl),
-    ("conv2d_lut(Tensor x, Tensor packed_w, Tensor codebook, float act_scale, int act_zp, Tensor? bias, "
-     "int out_channels, int in_channels_per_group, int kernel_h, int kernel_w, int stride_h, int stride_w, "
-     "int pad_h, int pad_w, int dilation_h, int dilation_w, int groups) -> Tensor", _conv2d_lut_impl),
+    "pack_u4(Tensor indices) -> Tensor",
+    "unpack_u4(Tensor packed, int numel) -> Tensor",
+    "quantize_activation_u4(Tensor x, float act_scale, int act_zp) -> Tensor",
+    "build_product_table(Tensor codebook, float act_scale, int act_zp) -> Tensor",
+    "linear_lut(Tensor x, Tensor packed_w, Tensor codebook, float act_scale, int act_zp, Tensor? bias, "
+    "int out_features, int in_features) -> Tensor",
+    "conv2d_lut(Tensor x, Tensor packed_w, Tensor codebook, float act_scale, int act_zp, Tensor? bias, "
+    "int out_channels, int in_channels_per_group, int kernel_h, int kernel_w, int stride_h, int stride_w, "
+    "int pad_h, int pad_w, int dilation_h, int dilation_w, int groups) -> Tensor",
 )
 
 _TORCH_LIBRARY = None
 
 
+def _missing(*args):
+    _lib.host()     # raises: what is missing and how to build it
+
+
 def _register() -> None:
+    """The six schemas; four of their kernels are registered by the native host path when it is loaded."""
     global _TORCH_LIBRARY
     if _TORCH_LIBRARY is not None:
         return
     library = torch.library.Library("dimq", "DEF")
-    for schema, fn in _SCHEMAS:
+    for schema in _SCHEMAS:
         library.define(schema)
-        library.impl(schema.split("(", 1)[0], fn, "CUDA")
+    library.impl("quantize_activation_u4", _quantize_activation_u4_impl, "CUDA")
+    library.impl("build_product_table", _build_product_table_impl, "CUDA")
+    if not _lib.is_available():
+        for name in ("pack_u4", "unpack_u4", "linear_lut", "conv2d_lut"):
+            library.impl(name, _missing, "CUDA")
     _TORCH_LIBRARY = library
 
 
@@ -482,44 +298,7 @@ def hard_quantize(w: torch.Tensor, codebooks: torch.Tensor, *, group_rows: int |
     ``group_rows`` leading-dimension rows of ``w`` per codebook.  Returns
     ``(indices uint8 shaped like w | None, packed uint8 | None)``.
     """
-    require_extension()
-    _require_cuda(w, "hard_quantize")
-    if not w.is_floating_point():
-        raise RuntimeError("hard_quantize expects floating weights")
-    wc = w.contiguous()
-    cb = codebooks.to(device=wc.device, dtype=torch.float32).contiguous()
-    if cb.dim() == 1:
-        cb = cb.view(1, -1)
-    entries = cb.shape[1]
-    if entries == 0:
-        raise RuntimeError("centers must be non-empty")
-    if entries > 256:
-        raise RuntimeError("hard_quantize supports at most 256 centres")
-    if cb.shape[0] == 1:
-        rows, cols, grp = 1, wc.numel(), 1
-    else:
-        if group_rows is None or wc.dim() < 1:
-            raise RuntimeError("grouped codebooks need group_rows")
-        rows = wc.shape[0]
-        cols = wc.numel() // max(rows, 1)
-        grp = int(group_rows)
-        if cb.shape[0] * grp < rows:
-            raise RuntimeError("not enough codebooks for the rows of w")
-    if bits is not None and (bits not in (1, 2, 3, 4, 8) or entries > (1 << bits)):
-        raise RuntimeError(f"cannot pack {entries}-entry indices into {bits} bits")
-    idx = torch.empty(wc.shape, dtype=torch.uint8, device=wc.device) if return_indices else None
-    packed = None
-    if bits is not None:
-        packed = torch.empty(((wc.numel() * bits + 7) // 8,), dtype=torch.uint8, device=wc.device)
-    if idx is None and packed is None:
-        raise RuntimeError("nothing to compute: ask for indices, packed bytes or both")
-    with torch.cuda.device(wc.device):
-        st = _lib.lib().dimq_hard_quantize(_lib.ptr(wc), _lib.dtype_code(wc, "w"), C.c_int64(rows), C.c_int64(cols),
-                                           _lib.ptr(cb), C.c_int(entries), C.c_int64(grp), _lib.ptr(idx),
-                                           _lib.ptr(packed), C.c_int(bits if bits is not None else 8),
-                                           _lib.stream_ptr(wc.device))
-    _lib.check(st, "hard_quantize")
-    return idx, packed
+    return _lib.host().hard_quantize(w, codebooks, group_rows, bits, return_indices)
 
 
 def fake_quantize_ste(w: torch.Tensor, codebooks: torch.Tensor, *, group_rows: int | None = None,
@@ -527,37 +306,7 @@ def fake_quantize_ste(w: torch.Tensor, codebooks: torch.Tensor, *, group_rows: i
     """``w + (codebook[idx].to(w.dtype) - w)`` with ``idx`` the nearest codeword (ties to the lowest
     index), in one kernel: the value of the straight-through fake quantisation of
     quant/dimq_wrapper.py:72-75.  Returns ``out`` or ``(out, idx uint8)``."""
-    require_extension()
-    _require_cuda(w, "fake_quantize_ste")
-    if not w.is_floating_point() or w.dtype == torch.float64:
-        raise RuntimeError("fake_quantize_ste expects float32, float16 or bfloat16 weights")
-    wc = w.contiguous()
-    cb = codebooks.detach().to(device=wc.device, dtype=torch.float32).contiguous()
-    if cb.dim() == 1:
-        cb = cb.view(1, -1)
-    entries = cb.shape[1]
-    if entries == 0:
-        raise RuntimeError("centers must be non-empty")
-    if entries > 256:
-        raise RuntimeError("fake_quantize_ste supports at most 256 centres")
-    if cb.shape[0] == 1:
-        rows, cols, grp = 1, wc.numel(), 1
-    else:
-        if group_rows is None or wc.dim() < 1:
-            raise RuntimeError("grouped codebooks need group_rows")
-        rows = wc.shape[0]
-        cols = wc.numel() // max(rows, 1)
-        grp = int(group_rows)
-        if cb.shape[0] * grp < rows:
-            raise RuntimeError("not enough codebooks for the rows of w")
-    out = torch.empty_like(wc)
-    idx = torch.empty(wc.shape, dtype=torch.uint8, device=wc.device) if return_indices else None
-    with torch.cuda.device(wc.device):
-        st = _lib.lib().dimq_fake_quantize_ste(_lib.ptr(wc), _lib.dtype_code(wc, "w"), C.c_int64(rows), C.c_int64(cols),
-                                               _lib.ptr(cb), C.c_int(entries), C.c_int64(grp), _lib.ptr(out),
-                                               _lib.ptr(idx), _lib.stream_ptr(wc.device))
-    _lib.check(st, "fake_quantize_ste")
-    return (out, idx) if return_indices else out
+    return _lib.host().fake_quantize_ste(w, codebooks, group_rows, return_indices)
 
 
 def _wq_weight(packed_weight: torch.Tensor, codebooks: torch.Tensor, bits: int, out_rows: int, numel: int,
@@ -609,6 +358,9 @@ def dimq_linear_wq(x: torch.Tensor, packed_weight: torch.Tensor, codebooks: torc
     re-ordered by :func:`linear_prepack`) speeds up the small-M kernel for large weights; the result is the
     same bits with and without it.
     """
+    if algo is None:
+        return _lib.host().linear_wq(x, packed_weight, codebooks, bias, out_features, in_features, bits, group_rows,
+                                     out_dtype, _EPILOGUES[epilogue], residual, packed_tiled)
     require_extension()
     _require_cuda(x, "linear_wq")
     if not x.is_floating_point():
@@ -666,26 +418,6 @@ def dimq_linear_wq(x: torch.Tensor, packed_weight: torch.Tensor, codebooks: torc
             _lib.LAUNCH_COUNT[0] += 1  # the kernel that adds the k slices
         del keep
         return y.view(*x.shape[:-1], out_features)
-    if algo is None:
-        # Three shapes get scratch memory: a few activation rows against a large weight (the k slices of
-        # the small-M kernel meet there), many activation rows (the indices are expanded once to a
-        # 16-bit weight and a dense tensor-core GEMM follows) and a few hundred rows against a long K
-        # (the kernel splits K and sums partial tiles there).
-        need = C.c_int64(0)
-        _lib.lib().dimq_linear_wq_workspace_bytes(_lib.ptr(xc), _lib.dtype_code(xc, "x"), C.byref(w), C.c_int64(m),
-                                                  C.c_int64(out_features), C.c_int64(in_features), C.byref(need))
-        if need.value > 0:
-            ws = torch.empty(need.value, dtype=torch.uint8, device=xc.device)
-            with torch.cuda.device(xc.device):
-                st = _lib.lib().dimq_linear_wq_ws(_lib.ptr(xc), _lib.dtype_code(xc, "x"), C.byref(w), _lib.ptr(b), b_dt,
-                                                  _lib.ptr(res), _lib.ptr(y), _lib.dtype_code(y, "y"), C.c_int64(m),
-                                                  C.c_int64(out_features), C.c_int64(in_features),
-                                                  _EPILOGUES[epilogue], _lib.ptr(ws), C.c_int64(need.value),
-                                                  _lib.stream_ptr(xc.device))
-            _lib.check(st, "linear_wq_ws")
-            _lib.LAUNCH_COUNT[0] += 1  # two kernels: expansion + GEMM, or GEMM + the kernel that finishes the sums
-            del keep
-            return y.view(*x.shape[:-1], out_features)
     with torch.cuda.device(xc.device):
         st = _lib.lib().dimq_linear_wq(_lib.ptr(xc), _lib.dtype_code(xc, "x"), C.byref(w), _lib.ptr(b), b_dt,
                                        _lib.ptr(res), _lib.ptr(y), _lib.dtype_code(y, "y"), C.c_int64(m),
@@ -708,6 +440,9 @@ def dimq_conv2d_wq(x: torch.Tensor, packed_weight: torch.Tensor, codebooks: torc
     activations, ``groups == 1``, a multiple of 64 input channels and stride 1 or 2, the convolution
     runs as an implicit GEMM on the tensor cores; otherwise as a direct convolution.
     """
+    if algo is None:
+        return _lib.host().conv2d_wq(x, packed_weight, codebooks, bias, weight_shape, stride, padding, dilation, groups,
+                                     bits, group_rows, out_dtype, _EPILOGUES[epilogue], residual, packed_khwc)
     require_extension()
     _require_cuda(x, "conv2d_wq")
     if x.dim() != 4:
@@ -729,31 +464,24 @@ def dimq_conv2d_wq(x: torch.Tensor, packed_weight: torch.Tensor, codebooks: torc
         if residual.dtype != out_dtype or residual.shape != y.shape or residual.stride() != y.stride():
             raise RuntimeError("residual must match the output shape, dtype and memory format")
         res = residual
-    if algo in (None, "expand"):
-        # Many output pixels: expand the indices once to a 16-bit weight in scratch and run a dense
-        # tensor-core kernel - the implicit GEMM over the re-ordered indices (packed_khwc), or the stem
-        # kernel for a 3-channel stride-2 convolution.  "expand" forces that form at any size.
+    if algo == "expand":
+        # always the expanded form: the implicit GEMM over the re-ordered indices (packed_khwc), or the stem kernel;
+        # scratch for the larger of the two layouts, [OC][KH*KW*IC] and the stem's [OC][192]
+        numel_k = max(numel // g.out_channels, 192)
         need = C.c_int64(0)
-        if algo == "expand":
-            # the larger of the two layouts: [OC][KH*KW*IC] and the stem's [OC][192]
-            numel_k = max(numel // g.out_channels, 192)
-            _lib.check(_lib.lib().dimq_expand_workspace_bytes(_lib.dtype_code(xc, "x"), C.byref(w),
-                                                              C.c_int64(g.out_channels), C.c_int64(numel_k),
-                                                              C.byref(need)), "expand_workspace_bytes")
-        else:
-            _lib.lib().dimq_conv2d_wq_workspace_bytes(_lib.ptr(xc), _lib.dtype_code(xc, "x"), C.byref(w), C.byref(g),
-                                                      C.byref(need))
-        if need.value > 0:
-            ws = torch.empty(need.value, dtype=torch.uint8, device=x.device)
-            fn = _lib.lib().dimq_conv2d_wq_expand if algo == "expand" else _lib.lib().dimq_conv2d_wq_ws
-            with torch.cuda.device(x.device):
-                st = fn(_lib.ptr(xc), _lib.dtype_code(xc, "x"), C.byref(w), _lib.ptr(b), b_dt, _lib.ptr(res), _lib.ptr(y),
-                        _lib.dtype_code(y, "y"), C.byref(g), _EPILOGUES[epilogue], _lib.ptr(ws), C.c_int64(need.value),
-                        _lib.stream_ptr(x.device))
-            _lib.check(st, "conv2d_wq_ws")
-            _lib.LAUNCH_COUNT[0] += 1  # the expansion and the convolution
-            del keep
-            return y
+        _lib.check(_lib.lib().dimq_expand_workspace_bytes(_lib.dtype_code(xc, "x"), C.byref(w),
+                                                          C.c_int64(g.out_channels), C.c_int64(numel_k),
+                                                          C.byref(need)), "expand_workspace_bytes")
+        ws = torch.empty(max(need.value, 16), dtype=torch.uint8, device=x.device)
+        with torch.cuda.device(x.device):
+            st = _lib.lib().dimq_conv2d_wq_expand(_lib.ptr(xc), _lib.dtype_code(xc, "x"), C.byref(w), _lib.ptr(b), b_dt,
+                                                  _lib.ptr(res), _lib.ptr(y), _lib.dtype_code(y, "y"), C.byref(g),
+                                                  _EPILOGUES[epilogue], _lib.ptr(ws), C.c_int64(ws.numel()),
+                                                  _lib.stream_ptr(x.device))
+        _lib.check(st, "conv2d_wq_expand")
+        _lib.LAUNCH_COUNT[0] += 1  # the expansion and the convolution
+        del keep
+        return y
     with torch.cuda.device(x.device):
         st = _lib.lib().dimq_conv2d_wq(_lib.ptr(xc), _lib.dtype_code(xc, "x"), C.byref(w), _lib.ptr(b), b_dt,
                                        _lib.ptr(res), _lib.ptr(y), _lib.dtype_code(y, "y"), C.byref(g),
@@ -769,26 +497,8 @@ def dimq_linear_a4(x: torch.Tensor, packed_weight: torch.Tensor, codebook: torch
                    residual: torch.Tensor | None = None) -> torch.Tensor | None:
     """W4A4 linear with an output type, epilogue and residual as in :func:`dimq_linear_wq`, on the tensor cores at
     fp32 grade; ``None`` where that form does not apply (K not a multiple of 64, output rows not of 16 bytes)."""
-    require_extension()
-    _require_cuda(x, "linear_a4")
-    if not x.is_floating_point():
-        raise RuntimeError("linear_a4 expects floating input")
-    _check_qparams(act_scale, act_zero_point)
-    if x.dim() == 0 or x.size(-1) != in_features:
-        raise RuntimeError("input last dimension must equal in_features")
-    _, (pw, cb, _) = _wq_weight(packed_weight, codebook, 4, out_features, out_features * in_features, None)
-    xc = x.contiguous()
-    b, b_dt = _bias_arg(bias, out_features, xc.device, "out_features")
-    m = xc.numel() // in_features
-    y = torch.empty((m, out_features), dtype=out_dtype or torch.float32, device=xc.device)
-    res = None
-    if residual is not None:
-        if residual.dtype != y.dtype or residual.numel() != y.numel():
-            raise RuntimeError("residual must match the output shape and dtype")
-        res = residual.contiguous()
-    if not _linear_a4(xc, pw, cb, act_scale, act_zero_point, b, b_dt, res, y, m, out_features, in_features, epilogue):
-        return None
-    return y.view(*x.shape[:-1], out_features)
+    return _lib.host().linear_a4(x, packed_weight, codebook, act_scale, act_zero_point, bias, out_features, in_features,
+                                 out_dtype, _EPILOGUES[epilogue], residual)
 
 
 def dimq_conv2d_a4(x: torch.Tensor, packed_weight: torch.Tensor, codebook: torch.Tensor, act_scale: float,
@@ -798,25 +508,8 @@ def dimq_conv2d_a4(x: torch.Tensor, packed_weight: torch.Tensor, codebook: torch
                    packed_khwc: torch.Tensor | None = None) -> torch.Tensor | None:
     """The same for the convolution (channels_last or NCHW storage, the output in the input's format; NCHW takes an
     fp32 output and no residual).  ``packed_khwc``: the indices re-ordered by :func:`conv_prepack`, if kept."""
-    require_extension()
-    _require_cuda(x, "conv2d_a4")
-    if x.dim() != 4:
-        raise RuntimeError("conv2d_a4 expects NCHW input")
-    if not x.is_floating_point():
-        raise RuntimeError("conv2d_a4 expects floating input")
-    _check_qparams(act_scale, act_zero_point)
-    g = _conv_geom(x, weight_shape, _pair(stride), _pair(padding), _pair(dilation), groups)
-    numel = g.out_channels * g.in_channels_per_group * g.kernel_h * g.kernel_w
-    _, (pw, cb, khwc) = _wq_weight(packed_weight, codebook, 4, g.out_channels, numel, None, packed_khwc)
-    b, b_dt = _bias_arg(bias, g.out_channels, x.device, "out_channels")
-    xc, y = _conv_io(x, g, out_dtype or torch.float32)
-    if y.numel() == 0:
-        return y
-    if residual is not None and (residual.dtype != y.dtype or residual.shape != y.shape or residual.stride() != y.stride()):
-        raise RuntimeError("residual must match the output shape, dtype and memory format")
-    if not _conv2d_a4(xc, pw, cb, act_scale, act_zero_point, b, b_dt, residual, y, g, epilogue, khwc):
-        return None
-    return y
+    return _lib.host().conv2d_a4(x, packed_weight, codebook, act_scale, act_zero_point, bias, weight_shape, stride,
+                                 padding, dilation, groups, out_dtype, _EPILOGUES[epilogue], residual, packed_khwc)
 
 
 def linear_prepack(packed_weight: torch.Tensor, out_features: int, in_features: int, bits: int = 4) -> torch.Tensor:
@@ -872,39 +565,13 @@ def im2col(x: torch.Tensor, weight_shape: Sequence[int], stride, padding, dilati
 
 def max_pool_nhwc(x: torch.Tensor, kernel: int, stride: int, padding: int) -> torch.Tensor:
     """Max-pool of a channels_last 16-bit tensor (logical NCHW in, logical NCHW / channels_last out)."""
-    require_extension()
-    _require_cuda(x, "max_pool_nhwc")
-    if x.dim() != 4 or not x.is_contiguous(memory_format=torch.channels_last):
-        raise RuntimeError("max_pool_nhwc expects a channels_last 4-D tensor")
-    b, c, h, w = x.shape
-    oh = (h + 2 * padding - kernel) // stride + 1
-    ow = (w + 2 * padding - kernel) // stride + 1
-    y = torch.empty((b, c, oh, ow), dtype=x.dtype, device=x.device, memory_format=torch.channels_last)
-    with torch.cuda.device(x.device):
-        st = _lib.lib().dimq_max_pool_nhwc(_lib.ptr(x), _lib.ptr(y), _lib.dtype_code(x, "x"), C.c_int64(b), C.c_int64(h),
-                                           C.c_int64(w), C.c_int64(c), C.c_int(kernel), C.c_int(stride),
-                                           C.c_int(padding), _lib.stream_ptr(x.device))
-    _lib.check(st, "max_pool_nhwc")
-    return y
+    return _lib.host().max_pool_nhwc(x, kernel, stride, padding)
 
 
 def images_to_nhwc(images: torch.Tensor, dtype: torch.dtype = torch.bfloat16) -> torch.Tensor:
     """``images.to(dtype).contiguous(memory_format=torch.channels_last)`` for a contiguous NCHW batch of
     3-channel images (fp32 / fp16 / bf16) in one pass of 16-byte loads and stores."""
-    require_extension()
-    _require_cuda(images, "images_to_nhwc")
-    if images.dim() != 4 or images.shape[1] != 3 or not images.is_contiguous() or (images.shape[2] * images.shape[3]) % 8:
-        raise RuntimeError("images_to_nhwc expects a contiguous [B, 3, H, W] tensor with H * W a multiple of 8")
-    if dtype not in (torch.bfloat16, torch.float16):
-        raise RuntimeError("images_to_nhwc writes bf16 or fp16")
-    b, _, h, w = images.shape
-    y = torch.empty((b, 3, h, w), dtype=dtype, device=images.device, memory_format=torch.channels_last)
-    with torch.cuda.device(images.device):
-        st = _lib.lib().dimq_images_to_nhwc(_lib.ptr(images), _lib.dtype_code(images, "images"), _lib.ptr(y),
-                                            _lib.dtype_code(y, "y"), C.c_int64(b), C.c_int64(h), C.c_int64(w),
-                                            _lib.stream_ptr(images.device))
-    _lib.check(st, "images_to_nhwc")
-    return y
+    return _lib.host().images_to_nhwc(images, dtype)
 
 
 def add_layer_norm(x: torch.Tensor, delta: torch.Tensor | None, weight: torch.Tensor, bias: torch.Tensor,
@@ -913,26 +580,7 @@ def add_layer_norm(x: torch.Tensor, delta: torch.Tensor | None, weight: torch.Te
 
     bf16 / fp16 CUDA tensors with a last dimension that is a multiple of 8 and at most 1024.
     """
-    require_extension()
-    _require_cuda(x, "add_layer_norm")
-    cols = x.shape[-1]
-    xc = x.contiguous()
-    dc = None if delta is None else delta.contiguous()
-    if dc is not None and (dc.shape != xc.shape or dc.dtype != xc.dtype):
-        raise RuntimeError("delta must match x in shape and dtype")
-    w = weight.to(xc.dtype).contiguous()
-    b = bias.to(xc.dtype).contiguous()
-    if w.numel() != cols or b.numel() != cols:
-        raise RuntimeError("weight / bias must have one element per column")
-    x_out = torch.empty_like(xc) if dc is not None else xc
-    h = torch.empty_like(xc)
-    with torch.cuda.device(xc.device):
-        st = _lib.lib().dimq_add_layer_norm(_lib.ptr(xc), _lib.ptr(dc), _lib.ptr(w), _lib.ptr(b),
-                                            _lib.ptr(x_out) if dc is not None else C.c_void_p(0), _lib.ptr(h),
-                                            C.c_int64(xc.numel() // cols), C.c_int64(cols), C.c_float(eps),
-                                            _lib.dtype_code(xc, "x"), _lib.stream_ptr(xc.device))
-    _lib.check(st, "add_layer_norm")
-    return x_out, h
+    return _lib.host().add_layer_norm(x, delta, weight, bias, eps)
 
 
 def last_device_status() -> int:

@@ -135,10 +135,10 @@ class DIMQViT(nn.Module):
             self.q[name.replace(".", "__")] = DIMQLinear.from_export_layer(layer, out_dtype=out_dtype, epilogue=epi)
 
     def _t(self, key: str) -> torch.Tensor:
-        return getattr(self, key.replace(".", "__"))
+        return self._buffers[key.replace(".", "__")]
 
     def _lin(self, name: str) -> DIMQLinear:
-        return self.q[name.replace(".", "__")]
+        return self.q._modules[name.replace(".", "__")]
 
     def forward(self, images: torch.Tensor) -> torch.Tensor:
         cfg = self.cfg
