@@ -31,6 +31,7 @@ bool dense_pays(int64_t rows);
 bool dense_supported(const void* x, int x_dtype, const dimq_wq_weight* w, const void* y, int y_dtype,
                      const void* residual, int64_t M, int64_t N, int64_t K);
 int64_t dense_workspace_bytes(int x_dtype, const dimq_wq_weight* w, int64_t N, int64_t K);
+int64_t linear_dense_workspace_bytes(const void* x, int x_dtype, const dimq_wq_weight* w, int64_t M, int64_t N, int64_t K);
 int launch_linear_wq_dense(const void* x, int x_dtype, const dimq_wq_weight* w, const void* bias, int bias_dtype,
                            const void* residual, void* y, int y_dtype, int64_t M, int64_t N, int64_t K, int epilogue,
                            void* workspace, int64_t workspace_bytes, cudaStream_t st);
@@ -233,7 +234,7 @@ extern "C" int dimq_linear_wq_workspace_bytes(const void* x, int x_dtype, const 
   // many activation rows: the expanded 16-bit weight (the output is taken to be as wide as it may get
   // - 16-bit - and aligned; dimq_linear_wq_ws checks the real one and falls back if it does not fit)
   if (dense_pays(M) && (N * 2) % 16 == 0 && dense_supported(x, x_dtype, w, x, x_dtype, nullptr, M, N, K)) {
-    *bytes = dense_workspace_bytes(x_dtype, w, N, K);
+    *bytes = linear_dense_workspace_bytes(x, x_dtype, w, M, N, K);
     return DIMQ_OK;
   }
   // else only where the automatic choice would take the tcgen05 kernel and splitting K pays
@@ -250,7 +251,10 @@ extern "C" int dimq_linear_wq_ws(const void* x, int x_dtype, const dimq_wq_weigh
       (bias == nullptr || valid_dtype(bias_dtype)) && epilogue >= DIMQ_EPI_NONE && epilogue <= DIMQ_EPI_ADD_RELU &&
       x != nullptr && y != nullptr &&
       dimq_linear_wq_workspace_bytes(x, x_dtype, w, M, N, K, &need) == DIMQ_OK && need > 0) {
-    if (workspace_bytes < need && x_dtype != DIMQ_F32) return DIMQ_ERR_SCRATCH_TOO_SMALL;   // fp32: runs without scratch too
+    // fp32 activations run without scratch too, many 16-bit rows with the expanded weight's alone
+    if (workspace_bytes < need && x_dtype != DIMQ_F32 &&
+        !(dense_pays(M) && workspace_bytes >= dense_workspace_bytes(x_dtype, w, N, K)))
+      return DIMQ_ERR_SCRATCH_TOO_SMALL;
     if (mma_regs_supported(x, x_dtype, w, M, N, K) && mma_regs_pays(w, N, K))
       return launch_linear_wq_mma_regs(x, x_dtype, w, bias, bias_dtype, residual, y, y_dtype, M, N, K, epilogue, workspace,
                                        workspace_bytes, static_cast<cudaStream_t>(stream));

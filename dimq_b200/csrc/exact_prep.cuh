@@ -146,7 +146,7 @@ __device__ __forceinline__ void expand_block(uint32_t* tbl, int64_t block, const
 }
 
 // Activation side of the preparation.
-enum PrepMode { kPrepSplitRows = 0, kPrepCodes = 1, kPrepCodesNchw = 2 };
+enum PrepMode { kPrepSplitRows = 0, kPrepCodes = 1, kPrepCodesNchw = 2, kPrepScaleRows = 3 };
 
 struct PrepParams {
   // activations
@@ -154,12 +154,12 @@ struct PrepParams {
   const void* x;
   int x_dtype;
   int vec_ok;                // x is 16-byte aligned
-  int64_t n;                 // kPrepCodes: elements; kPrepSplitRows: rows
-  int64_t C, HW;             // kPrepSplitRows: C = row length; kPrepCodesNchw: channels, pixels per image
+  int64_t n;                 // kPrepCodes: elements; kPrepSplitRows, kPrepScaleRows: rows
+  int64_t C, HW;             // kPrepSplitRows, kPrepScaleRows: C = row length; kPrepCodesNchw: channels, pixels per image
   float scale;
   int zp;
   __half* xo;                // codes, or [rows][hi C | lo C]
-  float* row_scale;          // kPrepSplitRows: 2^-e per row
+  float* row_scale;          // kPrepSplitRows, kPrepScaleRows: 2^-e per row
   int64_t x_blocks;          // blocks [0, x_blocks) prepare activations, the rest the weight
   int64_t px_tiles;          // kPrepCodesNchw: ceil(HW / 32)
   // weight
@@ -242,6 +242,38 @@ exact_prep_kernel(const PrepParams p) {
     if (px0 + my_px < p.HW) {
       const uint32_t* src = smem + my_px * 33 + cg * 4;
       *reinterpret_cast<uint4*>(p.xo + (b * p.HW + px0 + my_px) * p.C + c0 + cg * 8) = make_uint4(src[0], src[1], src[2], src[3]);
+    }
+  } else if (p.mode == kPrepScaleRows) {
+    // bf16 rows -> fp16(x * 2^e), two rows per block, four warps each (infinities and NaN stay what they are)
+    const int half_id = tid >> 7, t = tid & 127;
+    const int64_t row = blk * 2 + half_id;
+    const bool live = row < p.n;
+    const uint16_t* xr = static_cast<const uint16_t*>(p.x) + (live ? row : 0) * p.C;
+    float mx = 0.0f;
+    if (live)
+      for (int64_t k = t * 8; k < p.C; k += 1024) {     // C % 64 == 0
+        float f[8];
+        load8(xr, DIMQ_BF16, k, f);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) mx = fmaxf(mx, finite_f32(f[i]) ? fabsf(f[i]) : 0.0f);
+      }
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xFFFFFFFFu, mx, d));
+    if ((tid & 31) == 0) smem[tid >> 5] = __float_as_uint(mx);
+    __syncthreads();
+    if (!live) return;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) mx = fmaxf(mx, __uint_as_float(smem[half_id * 4 + i]));
+    const int ex = fp16_scale_exponent(mx);
+    if (t == 0) p.row_scale[row] = scalbnf(1.0f, -ex);
+    const float up = scalbnf(1.0f, ex);      // -113 <= ex <= 63: a normal number
+    for (int64_t k = t * 8; k < p.C; k += 1024) {
+      float f[8];
+      load8(xr, DIMQ_BF16, k, f);
+      __align__(16) __half o[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) o[i] = __float2half_rn(f[i] * up);
+      *reinterpret_cast<uint4*>(p.xo + row * p.C + k) = *reinterpret_cast<const uint4*>(o);
     }
   } else {
     // two rows per block, four warps each: the row's largest finite magnitude, then hi and lo (the second read of

@@ -75,7 +75,10 @@ struct DenseParams {
   int kps;                  // 64-k blocks per ring stage (1 or 2): narrow tiles amortise the per-stage wait / commit over 8 MMAs
   int b_res;                // convolution: the whole expanded weight (one tile wide) stays in shared memory
   int pair;                 // 1: CTA pairs (cta_group::2), GEMM only; m_tiles then counts 256-row pairs of blocks
-  // SEG form only: out = acc * row_scale[row] * col_scale[n] (null: out_scale, 1)
+  // Two-term weights on a narrow tile: the tile's B operand holds the bn rows of the first term and under them the bn rows
+  // of the second, one MMA of N = 2 bn multiplies both, and the epilogue adds the two halves of the accumulator
+  int stack;
+  // acc * row_scale[row] (null: no scale); SEG form: * row_scale[row] * col_scale[n] (null: out_scale, 1)
   const float* row_scale;
   const float* col_scale;
   float out_scale;
@@ -445,8 +448,11 @@ lut_dense_tc_kernel(const __grid_constant__ DenseMaps maps, const DenseParams p)
       if (elect_one()) {
         const uint32_t bar = smem_u32(&hdr->b_res_full);
         mbar_arrive_expect_tx(bar, static_cast<uint32_t>(total_kb) * p.b_bytes);
-        for (int kb = 0; kb < total_kb; ++kb)
-          tma_load_2d(smem_u32(b_resident + static_cast<uint32_t>(kb) * p.b_bytes), &maps.b, bar, kb * kBK, 0);
+        for (int kb = 0; kb < total_kb; ++kb) {
+          const uint32_t dst = smem_u32(b_resident + static_cast<uint32_t>(kb) * p.b_bytes);
+          tma_load_2d(dst, &maps.b, bar, kb * kBK, 0);
+          if (!SEG && p.stack) tma_load_2d(dst + p.b_bytes / 2, &maps.b, bar, (p.k_blocks + kb) * kBK, 0);
+        }
       }
       __syncwarp();
     }
@@ -500,6 +506,7 @@ lut_dense_tc_kernel(const __grid_constant__ DenseMaps maps, const DenseParams p)
               } else if (elect_one()) {
                 tma_load_2d(dst_a, &maps.a[0], full, kcol_a, m_blk * kBM);
                 tma_load_2d(dst_a + kABytes, &maps.b, full, kcol_b, n_blk * p.bn);
+                if (!SEG && p.stack) tma_load_2d(dst_a + kABytes + p.b_bytes / 2, &maps.b, full, (p.k_blocks + kb) * kBK, n_blk * p.bn);
               }
             } else {
               // input pixel = stride * out + tap offset.  With stride 2 the input is addressed through one
@@ -515,7 +522,10 @@ lut_dense_tc_kernel(const __grid_constant__ DenseMaps maps, const DenseParams p)
               }
               if (elect_one()) {
                 tma_load_4d(dst_a, &maps.a[map], full, cb * kBK, wx, hy, b0);
-                if (!p.b_res) tma_load_2d(dst_a + kABytes, &maps.b, full, kcol_b, n_blk * p.bn);
+                if (!p.b_res) {
+                  tma_load_2d(dst_a + kABytes, &maps.b, full, kcol_b, n_blk * p.bn);
+                  if (!SEG && p.stack) tma_load_2d(dst_a + kABytes + p.b_bytes / 2, &maps.b, full, (p.k_blocks + kb) * kBK, n_blk * p.bn);
+                }
               }
             }
             __syncwarp();
@@ -624,7 +634,7 @@ lut_dense_tc_kernel(const __grid_constant__ DenseMaps maps, const DenseParams p)
     const int n_chunks = p.bn / 32;
     uint32_t as = 0, aph = 0;
     bool ok = true;
-    if constexpr (SEG) asm volatile("griddepcontrol.wait;" ::: "memory");   // the scales come from the kernel before
+    if (SEG || p.row_scale != nullptr) asm volatile("griddepcontrol.wait;" ::: "memory");   // the scales come from the kernel before
     STEM_ACC_DECL;
     STEM_CLK(t_all);
     for (int t = tile0; t < num_tiles && ok; t += tile_step) {
@@ -717,6 +727,8 @@ lut_dense_tc_kernel(const __grid_constant__ DenseMaps maps, const DenseParams p)
         }
         continue;
       }
+      const float row_scale = p.row_scale != nullptr && row_off >= 0
+                                  ? p.row_scale[static_cast<int64_t>(m_blk) * kBM + quarter * 32 + lane] : 1.0f;
       // tcgen05.ld is warp-collective: the whole warp proceeds or the whole warp gives up
       STEM_CLK(t_w1);
       if (!__all_sync(0xFFFFFFFFu, mbar_wait(smem_u32(&hdr->d_full[as]), aph, abort_flag, 0x1500u | as))) { ok = false; break; }
@@ -741,6 +753,13 @@ lut_dense_tc_kernel(const __grid_constant__ DenseMaps maps, const DenseParams p)
           my_bias[lane] = i == 0 ? bj[0] : i == 1 ? bj[1] : i == 2 ? bj[2] : bj[3];
         }
         tmem_ld_wait();
+        if (!PAIR && p.stack) {      // the second term's columns
+          uint32_t r2[32];
+          tmem_ld32(d_tmem + p.bn + c * 32, r2);
+          tmem_ld_wait();
+#pragma unroll
+          for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) + __uint_as_float(r2[j]));
+        }
         if (c + 2 >= n_chunks) {
           // every column this warp reads of the buffer is in registers: hand it back to the MMA warp
           tc_fence_before();
@@ -755,6 +774,10 @@ lut_dense_tc_kernel(const __grid_constant__ DenseMaps maps, const DenseParams p)
         float v[32];
 #pragma unroll
         for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
+        if (p.row_scale != nullptr) {
+#pragma unroll
+          for (int j = 0; j < 32; ++j) v[j] *= row_scale;
+        }
         store_chunk<ES, false>(v, my_bias, my_out, maps, p, n_first, row_off, c1, c2, c3, lane);
       }
       if (++as == kAccStages) { as = 0; aph ^= 1u; }
@@ -819,9 +842,10 @@ CUtensorMapDataType map_dtype(int dtype) {
 // simple model - waves of tiles over the SMs times the measured cycles of a 64-k block (four MMAs and
 // a commit: ~590 at N = 256, ~450 at N = 128, ~430 at N = 64: below N = 256 the per-instruction floor
 // of about 106 cycles shows).
-int choose_bn(int64_t m_tiles, int64_t N, int max_bn = 256) {
+// Two-term weights: 256 wide they take two passes; narrower tiles multiply both terms at once (stacked).
+int choose_bn(int64_t m_tiles, int64_t N, int max_bn = 256, bool stacked = false) {
   const int cand[3] = {256, 128, 64};
-  const double cycles[3] = {590.0, 450.0, 430.0};
+  const double cycles[3] = {stacked ? 1180.0 : 590.0, stacked ? 590.0 : 450.0, stacked ? 450.0 : 430.0};
   int best = max_bn;
   double best_cost = -1.0;
   for (int i = 0; i < 3; ++i) {
@@ -902,7 +926,13 @@ int launch_dense(DenseMaps& maps, DenseParams& p, const void* scratch, int64_t K
 #endif
   const int fmt = x_dtype == DIMQ_BF16 ? 1 : 0;
   p.idesc = tc::make_idesc_f16(fmt, fmt, pair ? 2 * kBM : kBM, p.bn);
-  const int64_t b_len = K * (seg ? p.b_terms : p.passes);
+  const int64_t b_len = K * (seg ? p.b_terms : p.passes);   // row length of the weight matrix
+  p.stack = !seg && !pair && p.passes == 2 && p.bn <= 128;
+  if (p.stack) {
+    p.passes = 1;
+    p.b_bytes *= 2;
+    p.idesc = tc::make_idesc_f16(fmt, fmt, kBM, 2 * p.bn);
+  }
   const cuuint64_t bdims[2] = {static_cast<cuuint64_t>(b_len), static_cast<cuuint64_t>(p.N)};
   const cuuint64_t bstr[1] = {static_cast<cuuint64_t>(b_len) * 2};
   const cuuint32_t bbox[2] = {kBK, static_cast<cuuint32_t>(pair ? p.bn / 2 : p.bn)};
@@ -918,7 +948,7 @@ int launch_dense(DenseMaps& maps, DenseParams& p, const void* scratch, int64_t K
   // stage costs ~240 cycles beside 48-64 per MMA, so eight MMAs per stage nearly halve its time per block.
   // A convolution whose expanded weight is one tile wide and fits beside the activation stages keeps it in
   // shared memory: no per-stage weight copies.
-  p.kps = (!pair && p.bn <= 128) ? 2 : 1;
+  p.kps = (!pair && p.bn * (p.stack + 1) <= 128) ? 2 : 1;
 #ifdef DIMQ_B200_DIAG
   if (g_dense_diag & 65536) p.kps = 1;   // timing experiments: one block per stage
 #endif
@@ -1028,6 +1058,62 @@ int64_t dense_workspace_bytes(int x_dtype, const dimq_wq_weight* w, int64_t N, i
   return N * K * 2 * passes_for(x_dtype, w);
 }
 
+namespace {
+
+inline int64_t pad256(int64_t v) { return (v + 255) / 256 * 256; }
+
+// scratch regions: activations (halves), row scales, column scales, expanded weight
+struct ExactScratch {
+  int64_t x, row, col, w, total;
+  ExactScratch(int64_t x_halves, int64_t rows, int64_t N, int64_t K, int terms) {
+    x = 0;
+    row = x + pad256(x_halves * 2);
+    col = row + pad256(rows * 4);
+    w = col + pad256(N * 4);
+    total = w + pad256(N * K * 2 * terms);
+  }
+};
+
+// bf16 activations against an fp16 codebook, GEMM: rows of activations scaled by a power of two into fp16 (bf16's 8 bits
+// are exact there down to 2^-29 of the row's largest element) meet the codewords as they are stored - one product where
+// the bf16 hi + lo pair takes two, and no rounding of the codeword.
+bool rows16_applies(const void* x, int x_dtype, const dimq_wq_weight* w) {
+  return x_dtype == DIMQ_BF16 && w->cb_dtype == DIMQ_F16 && w->bits <= 4 && aligned(x, 16);
+}
+
+// q's activation side is filled in; adds the weight side (fmt, terms: see expand_block) and launches
+int launch_prep(PrepParams& q, const dimq_wq_weight* w, const uint8_t* packed, int64_t N, int64_t K, int fmt, int terms, void* wo,
+                int64_t x_blocks, cudaStream_t st) {
+  q.packed = packed;
+  q.codebooks = w->codebooks;
+  q.cb_dtype = w->cb_dtype;
+  q.entries = w->entries;
+  q.group_rows = w->group_rows;
+  q.rows = N;
+  q.K = K;
+  q.fmt = fmt;
+  q.terms = terms;
+  q.wo = static_cast<uint16_t*>(wo);
+  q.x_blocks = x_blocks;
+  const int64_t blocks = x_blocks + (N * (K / 32) + 255) / 256;
+  if (blocks > 0x7FFFFFFFll) return DIMQ_ERR_TOO_LARGE;
+  const unsigned grid = static_cast<unsigned>(blocks);
+  if (w->bits == 2) exact_prep_kernel<2><<<grid, kPrepThreads, 0, st>>>(q);
+  else if (w->bits == 3) exact_prep_kernel<3><<<grid, kPrepThreads, 0, st>>>(q);
+  else exact_prep_kernel<4><<<grid, kPrepThreads, 0, st>>>(q);
+  return launch_status();
+}
+
+}  // namespace
+
+// what launch_linear_wq_dense uses at its fastest; dense_workspace_bytes is enough for it to run
+int64_t linear_dense_workspace_bytes(const void* x, int x_dtype, const dimq_wq_weight* w, int64_t M, int64_t N, int64_t K) {
+  const int64_t least = dense_workspace_bytes(x_dtype, w, N, K);
+  if (!rows16_applies(x, x_dtype, w)) return least;
+  const int64_t need = ExactScratch(M * K, M, 0, 0, 1).total + pad256(N * K * 2);
+  return need > least ? need : least;
+}
+
 // CTA pairs pay when the single-CTA tiling is the 128 x 256 one and the pair tiling's waves (74 clusters) at its
 // per-block cost come out ahead of the single-CTA waves (148 CTAs) at theirs.
 bool pair_pays(int m_blocks, int64_t N, int64_t k_total, int bn) {
@@ -1057,9 +1143,10 @@ int launch_linear_wq_dense(const void* x, int x_dtype, const dimq_wq_weight* w, 
   memset(&maps, 0, sizeof(maps));
   p.M = M;
   p.N = N;
-  p.passes = passes_for(x_dtype, w);
+  const bool rows16 = rows16_applies(x, x_dtype, w) && workspace_bytes >= linear_dense_workspace_bytes(x, x_dtype, w, M, N, K);
+  p.passes = rows16 ? 1 : passes_for(x_dtype, w);
   p.m_tiles = static_cast<int>((M + kBM - 1) / kBM);
-  p.bn = choose_bn(p.m_tiles, N);
+  p.bn = choose_bn(p.m_tiles, N, 256, p.passes == 2);
   p.n_tiles = static_cast<int>((N + p.bn - 1) / p.bn);
   if (pair_pays(p.m_tiles, N, K * p.passes, p.bn)) {
     p.pair = 1;
@@ -1072,25 +1159,44 @@ int launch_linear_wq_dense(const void* x, int x_dtype, const dimq_wq_weight* w, 
   const cuuint64_t astr[1] = {static_cast<cuuint64_t>(K) * 2};
   const cuuint32_t abox[2] = {kBK, kBM};
   const cuuint32_t estr[2] = {1, 1};
-  if (encode(&maps.a[0], dt, 2, const_cast<void*>(x), adims, astr, abox, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-             CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+  const ExactScratch at(M * K, M, 0, 0, 1);       // rows16: fp16 activations, row scales, then the weight
+  unsigned char* base = static_cast<unsigned char*>(workspace);
+  void* w16 = rows16 ? base + at.total : base;
+  if (encode(&maps.a[0], rows16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : dt, 2, rows16 ? base + at.x : const_cast<void*>(x), adims, astr,
+             abox, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
     return DIMQ_ERR_DRIVER;
   const cuuint64_t odims[2] = {static_cast<cuuint64_t>(N), static_cast<cuuint64_t>(M)};
   const cuuint32_t obox[2] = {32, 32};
   if (!out_map(encode, &maps.y, y, y_dtype, 2, odims, obox)) return DIMQ_ERR_DRIVER;
-  int rc = expand(w, w->packed, N, K, x_dtype == DIMQ_BF16 ? 1 : 0, p.passes, workspace, st);
+  int rc;
+  if (rows16) {
+    PrepParams q;
+    memset(&q, 0, sizeof(q));
+    q.mode = kPrepScaleRows;
+    q.x = x;
+    q.x_dtype = x_dtype;
+    q.n = M;
+    q.C = K;
+    q.xo = reinterpret_cast<__half*>(base + at.x);
+    q.row_scale = reinterpret_cast<float*>(base + at.row);
+    p.row_scale = q.row_scale;
+    rc = launch_prep(q, w, w->packed, N, K, 0, 1, w16, (M + 1) / 2, st);
+  } else {
+    rc = expand(w, w->packed, N, K, x_dtype == DIMQ_BF16 ? 1 : 0, p.passes, workspace, st);
+  }
   if (rc != DIMQ_OK) return rc;
-  rc = launch_dense(maps, p, workspace, K, x_dtype, bias, bias_dtype, residual, y_dtype, epilogue, st);
+  rc = launch_dense(maps, p, w16, K, rows16 ? DIMQ_F16 : x_dtype, bias, bias_dtype, residual, y_dtype, epilogue, st);
   if (rc > 0 && p.pair) {
     // the cluster launch was refused (a positive status is the cudaError_t of the launch: e.g. a partition of the
     // GPU that cannot co-schedule CTA pairs): the same problem on single CTAs, over the weight already expanded
     (void)cudaGetLastError();
     p.pair = 0;
     p.m_tiles = static_cast<int>((M + kBM - 1) / kBM);
-    p.bn = choose_bn(p.m_tiles, N);
+    p.passes = rows16 ? 1 : passes_for(x_dtype, w);
+    p.bn = choose_bn(p.m_tiles, N, 256, p.passes == 2);
     p.n_tiles = static_cast<int>((N + p.bn - 1) / p.bn);
-    rc = launch_dense(maps, p, workspace, K, x_dtype, bias, bias_dtype, residual, y_dtype, epilogue, st);
+    rc = launch_dense(maps, p, w16, K, rows16 ? DIMQ_F16 : x_dtype, bias, bias_dtype, residual, y_dtype, epilogue, st);
   }
   return rc;
 }
@@ -1764,7 +1870,7 @@ int launch_conv2d_wq_dense(const void* x, int x_dtype, const dimq_wq_weight* w, 
   int rc = conv_setup(encode, x, x_dtype, y, y_dtype, g, maps, p);
   if (rc != DIMQ_OK) return rc;
   p.passes = passes_for(x_dtype, w);
-  p.bn = choose_bn(p.m_tiles, p.N);
+  p.bn = choose_bn(p.m_tiles, p.N, 256, p.passes == 2);
   p.n_tiles = static_cast<int>((p.N + p.bn - 1) / p.bn);
   const int64_t K = static_cast<int64_t>(g->kernel_h) * g->kernel_w * g->in_channels;
   rc = expand(w, w->packed_khwc, p.N, K, x_dtype == DIMQ_BF16 ? 1 : 0, p.passes, workspace, st);
@@ -1783,22 +1889,8 @@ int launch_conv2d_wq_dense(const void* x, int x_dtype, const dimq_wq_weight* w, 
 // and, for small calls, by the two launches.
 namespace {
 
-inline int64_t pad256(int64_t v) { return (v + 255) / 256 * 256; }
-
 // fp16 terms of a codeword: fp16 and (scaled) bf16 values are exact in one, fp32 ones take two
 int exact_terms(const dimq_wq_weight* w) { return w->cb_dtype == DIMQ_F32 ? 2 : 1; }
-
-// scratch regions: activations (halves), row scales, column scales, expanded weight
-struct ExactScratch {
-  int64_t x, row, col, w, total;
-  ExactScratch(int64_t x_halves, int64_t rows, int64_t N, int64_t K, int terms) {
-    x = 0;
-    row = x + pad256(x_halves * 2);
-    col = row + pad256(rows * 4);
-    w = col + pad256(N * 4);
-    total = w + pad256(N * K * 2 * terms);
-  }
-};
 
 // launches the preparation and fills in what the product needs to know about the operands
 int exact_prepare(PrepParams& q, DenseParams& p, const dimq_wq_weight* w, const uint8_t* packed, int64_t N, int64_t K,
@@ -1808,23 +1900,7 @@ int exact_prepare(PrepParams& q, DenseParams& p, const dimq_wq_weight* w, const 
   q.xo = reinterpret_cast<__half*>(base + at.x);
   q.row_scale = a4 ? nullptr : reinterpret_cast<float*>(base + at.row);
   q.col_scale = w->cb_dtype == DIMQ_F16 ? nullptr : reinterpret_cast<float*>(base + at.col);
-  q.wo = reinterpret_cast<uint16_t*>(base + at.w);
-  q.packed = packed;
-  q.codebooks = w->codebooks;
-  q.cb_dtype = w->cb_dtype;
-  q.entries = w->entries;
-  q.group_rows = w->group_rows;
-  q.rows = N;
-  q.K = K;
-  q.fmt = w->cb_dtype == DIMQ_F16 ? 0 : 2;
-  q.terms = terms;
-  q.x_blocks = x_blocks;
-  const int64_t blocks = x_blocks + (N * (K / 32) + 255) / 256;
-  if (blocks > 0x7FFFFFFFll) return DIMQ_ERR_TOO_LARGE;
-  const unsigned grid = static_cast<unsigned>(blocks);
-  if (w->bits == 2) exact_prep_kernel<2><<<grid, kPrepThreads, 0, st>>>(q);
-  else if (w->bits == 3) exact_prep_kernel<3><<<grid, kPrepThreads, 0, st>>>(q);
-  else exact_prep_kernel<4><<<grid, kPrepThreads, 0, st>>>(q);
+  const int rc = launch_prep(q, w, packed, N, K, w->cb_dtype == DIMQ_F16 ? 0 : 2, terms, base + at.w, x_blocks, st);
   p.row_scale = q.row_scale;
   p.col_scale = q.col_scale;
   p.out_scale = a4 ? scale : 1.0f;
@@ -1839,7 +1915,7 @@ int exact_prepare(PrepParams& q, DenseParams& p, const dimq_wq_weight* w, const 
     if (terms == 2) pass(0, 1);
     pass(0, 0);
   }
-  return launch_status();
+  return rc;
 }
 
 }  // namespace

@@ -146,3 +146,49 @@ def test_linear_f32_non_finite(ops):
     x = torch.rand(m, k, device="cuda") + 0.5
     y = ops.dimq_linear_wq(x, packed, bad, None, n, k, bits=4)
     assert torch.equal(y.isinf().all(0), hit) and bool(y[:, ~hit].isfinite().all())
+
+
+# ---- bf16 activations against an fp16 codebook: rows scaled into fp16 (GEMM), two terms in one MMA (convolution) --------
+# Bound: the products are exact or carry 2^-17, the accumulators truncate: 3.7e-6 at K = 3072, 5.5e-6 at 4608.
+
+@pytest.mark.parametrize("m,k,n", [(1024, 64, 8), (1025, 768, 328), (2000, 3072, 256), (9473, 256, 512)])
+@pytest.mark.parametrize("bits,group_rows", [(4, None), (3, 128), (2, 1)])
+def test_linear_bf16_rows_with_fp16_codebook(ops, m, k, n, bits, group_rows):
+    if group_rows is not None and n // group_rows > 3:
+        group_rows = n // 3                       # keeps the last group's codewords inside fp16
+    packed, books, w = _weight(ops, n, k, bits, torch.float16, group_rows, seed=m + bits)
+    x = (torch.randn(m, k, device="cuda") * 10.0 ** torch.linspace(-14, 14, m, device="cuda").view(-1, 1)).bfloat16()
+    bias, res = torch.randn(n, device="cuda"), torch.randn(m, n, device="cuda")
+    y = ops.dimq_linear_wq(x, packed, books, None, n, k, bits=bits, group_rows=group_rows)
+    want = x.double() @ w.t()
+    r = x.double().norm(dim=1) * w.norm() / k ** 0.5
+    assert ops.last_device_status() == 0 and float(((y.double() - want).norm(dim=1) / r).max()) < 1.2e-5
+    y = ops.dimq_linear_wq(x[:1024], packed, books, bias, n, k, bits=bits, group_rows=group_rows, epilogue="relu",
+                           residual=res[:1024])
+    z = (want[:1024] + bias.double()).relu() + res[:1024].double()
+    assert float((y.double() - z).norm() / z.norm()) < 1.2e-5
+
+
+def test_linear_bf16_rows_non_finite(ops):
+    m, k, n = 1100, 128, 64
+    packed, books, w = _weight(ops, n, k, 4, torch.float16, seed=5)
+    x = torch.randn(m, k, device="cuda").bfloat16()
+    x[3, 5], x[700, 9], x[1099, 2] = float("inf"), float("-inf"), float("nan")
+    x[20] = 0.0
+    y = ops.dimq_linear_wq(x, packed, books, None, n, k, bits=4)
+    want = x.float() @ w.float().t()
+    assert torch.equal(y.isnan(), want.isnan()) and torch.equal(y.isinf(), want.isinf())
+    assert bool((y[20] == 0).all())
+
+
+@pytest.mark.parametrize("cout", [8, 64, 72, 128, 136, 256])
+@pytest.mark.parametrize("cin,ks,stride,size", [(64, 3, 1, 28), (128, 1, 2, 28), (64, 1, 1, 33)])
+def test_conv2d_two_terms(ops, cout, cin, ks, stride, size):
+    packed, books, w = _weight(ops, cout, cin * ks * ks, 4, torch.float16, seed=cout + ks)
+    x = torch.randn(9, cin, size, size, device="cuda").bfloat16().contiguous(memory_format=torch.channels_last)
+    bias = torch.randn(cout, device="cuda")
+    wshape = (cout, cin, ks, ks)
+    y = ops.dimq_conv2d_wq(x, packed, books.reshape(-1), bias, wshape, stride, ks // 2, bits=4,
+                           packed_khwc=ops.conv_prepack(packed, wshape, 4))
+    want = F.conv2d(x.double().contiguous(), w.view(wshape), bias.double(), stride, ks // 2)
+    assert ops.last_device_status() == 0 and _rel(y, want) < 1.2e-5
