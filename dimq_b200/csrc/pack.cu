@@ -179,6 +179,169 @@ product_table_kernel(const void* __restrict__ codebook, int cb_dtype, int64_t to
 }
 
 // ---------------------------------------------------------------------------
+// hard quantise over a well-spaced sorted codebook: the path of trained and quantile codebooks
+// ---------------------------------------------------------------------------
+// One codebook per blockIdx.y; a block walks its group's weights, 8 consecutive ones per thread and step.
+//
+// The scan of hard_quantize_kernel takes the first minimum of d(k) = fl(fl(w - c[k])^2).  Let the codebook be strictly
+// increasing and finite with smallest gap g, span <= 2^20 g and g in [2^-50, 2^38], and let w lie within 2^20 g of
+// [c[0], c[last]].  Then every |w - c| <= 2^21 g, two codewords on one side of w lie at distances that differ by g, at
+// least 2^-21 of either, so neither the subtraction nor the square (2^-24 each, no underflow or overflow) can make them
+// equal or swap them: the minimum is at one of the two codewords around w, and the lower one on a tie.  They are found
+// by bisection in a shared-memory table and compared exactly as the scan would.  Everything else - a codebook that is
+// not so spaced, a weight farther out, a NaN - is scanned.
+//
+// Bound: HBM (4 bytes in, 1 + bits / 8 or 4 out per weight), with ~30 instructions per weight beside it.  The kernel
+// below it replaces here spent 64-bit divisions per element, a serial sortedness check per 2 048 weights and
+// byte-wise stores: 4096 x 1024 fp32, 16 codewords, indices + packed and their unpacking took 28.7 us per call there,
+// 16.4 here (both kernels and three allocations).
+__device__ __noinline__ uint32_t nearest_scan(float wv, const float* __restrict__ cb, int entries) {
+  float d = __fsub_rn(wv, cb[0]);
+  float best = __fmul_rn(d, d);
+  uint32_t bi = 0u;
+  for (int k = 1; k < entries; ++k) {
+    d = __fsub_rn(wv, cb[k]);
+    const float dd = __fmul_rn(d, d);
+    if (dd < best || (dd != dd && best == best)) { best = dd; bi = k; }   // a NaN beats any number, the first NaN stays
+  }
+  return bi;
+}
+
+template <typename T, int E>   // E: the number of codewords rounded up to a power of two
+__global__ void __launch_bounds__(kThreads)
+nearest_sorted_kernel(const T* __restrict__ w, int64_t n, int64_t group_elems, const float* __restrict__ codebooks,
+                      int entries, uint8_t* __restrict__ idx_out, uint8_t* __restrict__ packed, int bits,
+                      T* __restrict__ fake_out) {
+  __shared__ float tab[E + 2];          // -inf, the codewords, +inf up to E
+  __shared__ int gap_bits, bad;
+  const int tid = threadIdx.x;
+  const float kInf = __int_as_float(0x7F800000);
+  const float* cb = codebooks + static_cast<int64_t>(blockIdx.y) * entries;
+  if (tid == 0) { gap_bits = 0x7F800000; bad = 0; tab[0] = -kInf; tab[E + 1] = kInf; }
+  for (int k = tid; k < E; k += kThreads) tab[k + 1] = k < entries ? cb[k] : kInf;
+  __syncthreads();
+  for (int k = tid; k + 1 < entries; k += kThreads) {
+    const float gap = __fsub_rn(tab[k + 2], tab[k + 1]);
+    if (!(gap > 0.0f) || !isfinite(tab[k + 1]) || !isfinite(tab[k + 2])) bad = 1;
+    else atomicMin(&gap_bits, __float_as_int(gap));     // positive floats order like their bits
+  }
+  __syncthreads();
+  const float gap = __int_as_float(gap_bits);
+  const float first = tab[1], last = tab[entries];
+  const float reach = gap * 1048576.0f;
+  const bool spaced = bad == 0 && entries > 1 && gap >= 8.8817842e-16f && gap <= 2.7487791e11f && last - first <= reach;
+  // limits a little inside the proven range (the sums round)
+  const float lim_lo = spaced ? first - 0.5f * reach : kInf, lim_hi = spaced ? last + 0.5f * reach : -kInf;
+
+  const int64_t start = static_cast<int64_t>(blockIdx.y) * group_elems;      // a multiple of 8
+  const int64_t end = start + group_elems < n ? start + group_elems : n;
+  const int64_t total_bytes = (n * bits + 7) / 8;
+  for (int64_t base = start + (static_cast<int64_t>(blockIdx.x) * kThreads + tid) * 8; base < end;
+       base += static_cast<int64_t>(gridDim.x) * kThreads * 8) {
+    const bool full = base + 8 <= end;
+    float f[8];
+    if (full) {
+      if constexpr (sizeof(T) == 4) {
+        const float4 a = __ldg(reinterpret_cast<const float4*>(w + base));
+        const float4 b = __ldg(reinterpret_cast<const float4*>(w + base) + 1);
+        f[0] = a.x; f[1] = a.y; f[2] = a.z; f[3] = a.w; f[4] = b.x; f[5] = b.y; f[6] = b.z; f[7] = b.w;
+      } else {
+        const uint4 q = __ldg(reinterpret_cast<const uint4*>(w + base));
+        const T* h = reinterpret_cast<const T*>(&q);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) f[i] = to_float<T>(h[i]);
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) f[i] = base + i < end ? to_float<T>(w[base + i]) : first;
+    }
+    uint32_t r[8];
+    bool in = true;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) in = in && f[i] >= lim_lo && f[i] <= lim_hi;
+    if (in) {
+      int pos[8];        // number of codewords below the weight, at most E - 1
+#pragma unroll
+      for (int i = 0; i < 8; ++i) pos[i] = 0;
+#pragma unroll
+      for (int step = E / 2; step > 0; step >>= 1) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) pos[i] += tab[pos[i] + step] < f[i] ? step : 0;
+      }
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        float d = __fsub_rn(f[i], tab[pos[i]]);
+        const float dlo = __fmul_rn(d, d);
+        d = __fsub_rn(f[i], tab[pos[i] + 1]);
+        const float dhi = __fmul_rn(d, d);
+        r[i] = static_cast<uint32_t>(dhi < dlo ? pos[i] : pos[i] - 1);
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) r[i] = nearest_scan(f[i], tab + 1, entries);
+    }
+    if (idx_out != nullptr) {
+      if (full) {
+        const uint32_t w0 = r[0] | (r[1] << 8) | (r[2] << 16) | (r[3] << 24);
+        const uint32_t w1 = r[4] | (r[5] << 8) | (r[6] << 16) | (r[7] << 24);
+        *reinterpret_cast<uint2*>(idx_out + base) = make_uint2(w0, w1);
+      } else {
+        for (int i = 0; i < 8 && base + i < end; ++i) idx_out[base + i] = static_cast<uint8_t>(r[i]);
+      }
+    }
+    if (fake_out != nullptr) {
+      // w + (c[idx].to(w.dtype) - w), every operation rounded to the weight's type
+      __align__(16) T o[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const float c = to_float<T>(from_float<T>(tab[1 + r[i]]));
+        const float diff = to_float<T>(from_float<T>(__fsub_rn(c, f[i])));
+        o[i] = from_float<T>(__fadd_rn(f[i], diff));
+      }
+      if (full) {
+#pragma unroll
+        for (int i = 0; i < static_cast<int>(sizeof(T)) / 2; ++i)
+          reinterpret_cast<uint4*>(fake_out + base)[i] = reinterpret_cast<const uint4*>(o)[i];
+      } else {
+        for (int i = 0; i < 8 && base + i < end; ++i) fake_out[base + i] = o[i];
+      }
+    }
+    if (packed != nullptr) {
+      unsigned long long s = 0ull;
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        if (base + i < end) s |= static_cast<unsigned long long>(r[i]) << (i * bits);
+      uint8_t* dst = packed + base / 8 * bits;
+      if (full && bits == 4) *reinterpret_cast<uint32_t*>(dst) = static_cast<uint32_t>(s);
+      else if (full && bits == 2) *reinterpret_cast<uint16_t*>(dst) = static_cast<uint16_t>(s);
+      else if (full && bits == 8) *reinterpret_cast<unsigned long long*>(dst) = s;
+      else
+        for (int b = 0; b < bits; ++b)
+          if (base / 8 * bits + b < total_bytes) dst[b] = static_cast<uint8_t>(s >> (8 * b));
+    }
+  }
+}
+
+template <typename T>
+int launch_nearest_sorted(const void* w, int64_t n, int64_t groups, int64_t group_elems, const float* codebooks, int entries,
+                          uint8_t* idx, uint8_t* packed, int bits, void* fake_out, cudaStream_t st) {
+  // enough blocks for every SM to hold eight, each with as few steps as that leaves
+  const int64_t chunks = ((group_elems < n ? group_elems : n) + kThreads * 8 - 1) / (kThreads * 8);
+  const int64_t most = (8 * kNumSMs + groups - 1) / groups;
+  const dim3 grid(static_cast<unsigned>(chunks < most ? chunks : most), static_cast<unsigned>(groups));
+  const T* src = static_cast<const T*>(w);
+  T* fake = static_cast<T*>(fake_out);
+#define DIMQ_NEAREST(E) nearest_sorted_kernel<T, E><<<grid, kThreads, 0, st>>>(src, n, group_elems, codebooks, entries, idx, packed, bits, fake)
+  if (entries <= 4) DIMQ_NEAREST(4);
+  else if (entries <= 8) DIMQ_NEAREST(8);
+  else if (entries <= 16) DIMQ_NEAREST(16);
+  else if (entries <= 64) DIMQ_NEAREST(64);
+  else DIMQ_NEAREST(256);
+#undef DIMQ_NEAREST
+  return launch_status();
+}
+
+// ---------------------------------------------------------------------------
 // hard quantise (+ pack): 8 consecutive weights per thread
 // ---------------------------------------------------------------------------
 constexpr int kHqSmemEntries = 8192;  // codebook entries staged in shared memory (32 KB)
@@ -468,8 +631,21 @@ static int hard_quantize_launch(const void* w, int w_dtype, int64_t rows, int64_
   const size_t smem = use_smem ? sizeof(float) * static_cast<size_t>(groups * entries) + static_cast<size_t>(groups) : 0;
   const int vec_ok = aligned(w, 16) && (indices == nullptr || aligned(indices, 8));
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const unsigned blocks = (unsigned)blocks_for((n + 7) / 8);
   const int pbits = packed != nullptr ? bits : 8;
+  // Whole groups of at least 4 096 weights (two blocks' step: below, checking the codebook costs more than the scan) that
+  // start on the 8-weight boundaries of the vector accesses
+  const int64_t group_elems = group_rows * cols;
+  if ((groups == 1 || (group_elems % 8 == 0 && group_elems >= 4096)) && groups <= 65535 && aligned(w, 16) &&
+      (indices == nullptr || aligned(indices, 8)) && (packed == nullptr || aligned(packed, 8)) &&
+      (fake_out == nullptr || aligned(fake_out, 16))) {
+    const int64_t ge = groups == 1 ? n : group_elems;
+    if (w_dtype == DIMQ_F32)
+      return launch_nearest_sorted<float>(w, n, groups, ge, codebooks, entries, indices, packed, pbits, fake_out, st);
+    if (w_dtype == DIMQ_F16)
+      return launch_nearest_sorted<__half>(w, n, groups, ge, codebooks, entries, indices, packed, pbits, fake_out, st);
+    return launch_nearest_sorted<__nv_bfloat16>(w, n, groups, ge, codebooks, entries, indices, packed, pbits, fake_out, st);
+  }
+  const unsigned blocks = (unsigned)blocks_for((n + 7) / 8);
   if (w_dtype == DIMQ_F32)
     hard_quantize_kernel<float><<<blocks, kThreads, smem, st>>>(static_cast<const float*>(w), n, cols, codebooks,
                                                                 entries, groups, group_rows, indices, packed, pbits,

@@ -267,3 +267,27 @@ def test_fake_quant_weight_half_types_and_groups(ops, dtype):
     assert torch.equal(out, w + (hard - w))
     with pytest.raises(ValueError):
         fake_quant_weight(w, books[:, :0])
+
+
+@pytest.mark.parametrize("dtype", ["f32", "f16"])
+@pytest.mark.parametrize("rows,cols,group_rows,bits", [(1, 5, None, 4), (64, 147, None, 8), (257, 512, 128, 3), (40, 104, 40, 2),
+                                                       (300, 4608, 100, 8), (9, 520, 8, 4), (31, 1024, 4, 1)])
+def test_nearest_codeword_groups_and_tails(ops, rows, cols, group_rows, bits, dtype):
+    """Whole groups, remainders of eight weights, a last group that is not full, indices, packed stream and the
+    straight-through value, at the codeword counts of every table size; one outlier far off the codebook."""
+    from oracle import c_oracle
+
+    rng = np.random.default_rng(rows * 31 + cols)
+    w = (rng.standard_normal((rows, cols)) * 0.05).astype(np.float32)
+    w.reshape(-1)[rows * cols // 2] = 3.0e30 if dtype == "f32" else 6.0e4
+    wt = torch.from_numpy(w).cuda().to(torch.float32 if dtype == "f32" else torch.float16)
+    w = wt.float().cpu().numpy()
+    groups = 1 if group_rows is None else (rows + group_rows - 1) // group_rows
+    cb = np.sort((rng.standard_normal((groups, 1 << bits)) * 0.05).astype(np.float32), axis=1)
+    want = c_oracle.hard_quantize(w, cb, group_rows or rows)
+    idx, packed = ops.hard_quantize(wt, _cuda(cb), group_rows=group_rows or rows, bits=bits)
+    assert np.array_equal(idx.cpu().numpy(), want)
+    assert np.array_equal(packed.cpu().numpy(), ops.pack_bits(idx, bits).cpu().numpy())
+    fq = ops.fake_quantize_ste(wt, _cuda(cb), group_rows=group_rows or rows)
+    c = torch.from_numpy(np.take_along_axis(cb[np.arange(rows) // (group_rows or rows)], want.astype(np.int64), 1)).cuda()
+    assert torch.equal(fq, wt + (c.to(wt.dtype) - wt))
