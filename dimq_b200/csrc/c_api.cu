@@ -28,6 +28,7 @@ int launch_conv2d_wq_tc(const void* x, int x_dtype, const dimq_wq_weight* w, con
                         const void* residual, void* y, int y_dtype, const dimq_conv_geom* g, int epilogue,
                         cudaStream_t st);
 bool dense_pays(int64_t rows);
+bool linear_dense_pays(const void* x, int x_dtype, const dimq_wq_weight* w, int64_t M, int64_t N, int64_t K);
 bool dense_supported(const void* x, int x_dtype, const dimq_wq_weight* w, const void* y, int y_dtype,
                      const void* residual, int64_t M, int64_t N, int64_t K);
 int64_t dense_workspace_bytes(int x_dtype, const dimq_wq_weight* w, int64_t N, int64_t K);
@@ -233,7 +234,7 @@ extern "C" int dimq_linear_wq_workspace_bytes(const void* x, int x_dtype, const 
   }
   // many activation rows: the expanded 16-bit weight (the output is taken to be as wide as it may get
   // - 16-bit - and aligned; dimq_linear_wq_ws checks the real one and falls back if it does not fit)
-  if (dense_pays(M) && (N * 2) % 16 == 0 && dense_supported(x, x_dtype, w, x, x_dtype, nullptr, M, N, K)) {
+  if (linear_dense_pays(x, x_dtype, w, M, N, K) && (N * 2) % 16 == 0 && dense_supported(x, x_dtype, w, x, x_dtype, nullptr, M, N, K)) {
     *bytes = linear_dense_workspace_bytes(x, x_dtype, w, M, N, K);
     return DIMQ_OK;
   }
@@ -253,7 +254,7 @@ extern "C" int dimq_linear_wq_ws(const void* x, int x_dtype, const dimq_wq_weigh
       dimq_linear_wq_workspace_bytes(x, x_dtype, w, M, N, K, &need) == DIMQ_OK && need > 0) {
     // fp32 activations run without scratch too, many 16-bit rows with the expanded weight's alone
     if (workspace_bytes < need && x_dtype != DIMQ_F32 &&
-        !(dense_pays(M) && workspace_bytes >= dense_workspace_bytes(x_dtype, w, N, K)))
+        !(linear_dense_pays(x, x_dtype, w, M, N, K) && workspace_bytes >= dense_workspace_bytes(x_dtype, w, N, K)))
       return DIMQ_ERR_SCRATCH_TOO_SMALL;
     if (mma_regs_supported(x, x_dtype, w, M, N, K) && mma_regs_pays(w, N, K))
       return launch_linear_wq_mma_regs(x, x_dtype, w, bias, bias_dtype, residual, y, y_dtype, M, N, K, epilogue, workspace,
@@ -262,7 +263,7 @@ extern "C" int dimq_linear_wq_ws(const void* x, int x_dtype, const dimq_wq_weigh
       if (workspace_bytes >= need && linear_exact_supported(false, x, x_dtype, w, y, y_dtype, residual, M, N, K))
         return launch_linear_exact(false, x, x_dtype, 1.0f, 0, w, bias, bias_dtype, residual, y, y_dtype, M, N, K, epilogue,
                                    workspace, workspace_bytes, static_cast<cudaStream_t>(stream));
-    } else if (dense_pays(M)) {
+    } else if (linear_dense_pays(x, x_dtype, w, M, N, K)) {
       if (dense_supported(x, x_dtype, w, y, y_dtype, residual, M, N, K))
         return launch_linear_wq_dense(x, x_dtype, w, bias, bias_dtype, residual, y, y_dtype, M, N, K, epilogue,
                                       workspace, workspace_bytes, static_cast<cudaStream_t>(stream));

@@ -32,6 +32,8 @@
 #include "tc_common.cuh"
 
 namespace dimq {
+int tc_split_k(int64_t M, int64_t N, int64_t K);
+
 namespace {
 
 using namespace tc;
@@ -1036,8 +1038,8 @@ void stem_diag_prof(unsigned long long* prof) { g_stem_prof = prof; }   // 16 wo
 
 // ---- GEMM ----------------------------------------------------------------------------------------
 
-// Smallest M for which expanding the weight first pays (below it the in-pipeline kernel or its split-K
-// form runs: the expansion and the second launch cost a few microseconds).
+// From this many rows (pixels) on the weight is expanded first whatever its shape; a convolution below it runs the
+// in-pipeline kernel, a GEMM what linear_dense_pays says.
 constexpr int64_t kDenseMinRows = 1024;
 
 bool dense_pays(int64_t rows) { return rows >= kDenseMinRows; }
@@ -1112,6 +1114,35 @@ int64_t linear_dense_workspace_bytes(const void* x, int x_dtype, const dimq_wq_w
   if (!rows16_applies(x, x_dtype, w)) return least;
   const int64_t need = ExactScratch(M * K, M, 0, 0, 1).total + pad256(N * K * 2);
   return need > least ? need : least;
+}
+
+// Below kDenseMinRows: whether expanding first beats looking up inside the pipeline (lut_gemm_tc.cu, with or without its
+// split of K).  Microseconds from measured calls (B200, graph of calls, M = 33 ... 788 on eight shapes from 512 -> 1000 to
+// 8192 -> 8192; the model is within ~20 % of them):
+//   in-pipeline: 5 (8 when K is split: zeroing and finishing), 0.5 per 64-k block of a CTA - 0.9 when bf16 activations meet
+//   a codebook that is not bf16 and every codeword is a hi + lo pair - and a little for a wide tile;
+//   expanded: 5, 0.62 per million weights and term, the dense kernel's cycles per block, the last tile's epilogue.
+// Examples, in-pipeline / expanded: fp16 codebook 197 x 768 -> 768 17.3 / 9.7, 394 x 1024 -> 4096 37 / 14, 394 x 8192 -> 8192
+// 372 / 96, but 64 x 4096 -> 1024 12.4 / 22.5; bf16 codebook 394 x 8192 -> 8192 186 / 94.  The margins (8, 20 and 30 %)
+// keep the model's error from costing a call anything.
+bool linear_dense_pays(const void* x, int x_dtype, const dimq_wq_weight* w, int64_t M, int64_t N, int64_t K) {
+  if (M >= kDenseMinRows) return true;
+  if (K < kBK || K % kBK != 0 || w->bits > 4) return false;
+  const double kb = static_cast<double>(K / kBK);
+  const bool two_terms = passes_for(x_dtype, w) == 2;
+  const int split = tc_split_k(M, N, K);
+  const int64_t tx = M >= 192 ? 192 : (M + 31) / 32 * 32;
+  const int64_t pipe_tiles = (M + tx - 1) / tx * ((N + 127) / 128) * split;
+  const double pipe = (split > 1 ? 8.0 : 5.0) + static_cast<double>((pipe_tiles + kNumSMs - 1) / kNumSMs) * (kb / split) * (two_terms ? 0.9 : 0.5) +
+                      static_cast<double>(tx) / 64.0 * 0.6;
+  const bool stacked = two_terms && !rows16_applies(x, x_dtype, w);
+  const int64_t m_tiles = (M + kBM - 1) / kBM;
+  const int bn = choose_bn(m_tiles, N, 256, stacked);
+  const double per_block = (bn == 64 ? (stacked ? 450.0 : 430.0) : bn == 128 ? (stacked ? 590.0 : 450.0) : (stacked ? 1180.0 : 590.0)) / 1850.0;
+  const int64_t tiles = m_tiles * ((N + bn - 1) / bn);
+  const double dense = 5.0 + (stacked ? 1.24e-6 : 0.62e-6) * static_cast<double>(N) * static_cast<double>(K) +
+                       static_cast<double>((tiles + kNumSMs - 1) / kNumSMs) * kb * per_block + 0.012 * bn;
+  return dense < (stacked ? 0.8 : two_terms ? 0.92 : 0.7) * pipe;
 }
 
 // CTA pairs pay when the single-CTA tiling is the 128 x 256 one and the pair tiling's waves (74 clusters) at its

@@ -151,7 +151,8 @@ def test_linear_f32_non_finite(ops):
 # ---- bf16 activations against an fp16 codebook: rows scaled into fp16 (GEMM), two terms in one MMA (convolution) --------
 # Bound: the products are exact or carry 2^-17, the accumulators truncate: 3.7e-6 at K = 3072, 5.5e-6 at 4608.
 
-@pytest.mark.parametrize("m,k,n", [(1024, 64, 8), (1025, 768, 328), (2000, 3072, 256), (9473, 256, 512)])
+@pytest.mark.parametrize("m,k,n", [(33, 768, 768), (197, 768, 1000), (400, 1024, 2048), (1024, 64, 8), (1025, 768, 328),
+                                   (2000, 3072, 256), (9473, 256, 512)])
 @pytest.mark.parametrize("bits,group_rows", [(4, None), (3, 128), (2, 1)])
 def test_linear_bf16_rows_with_fp16_codebook(ops, m, k, n, bits, group_rows):
     if group_rows is not None and n // group_rows > 3:
@@ -163,9 +164,10 @@ def test_linear_bf16_rows_with_fp16_codebook(ops, m, k, n, bits, group_rows):
     want = x.double() @ w.t()
     r = x.double().norm(dim=1) * w.norm() / k ** 0.5
     assert ops.last_device_status() == 0 and float(((y.double() - want).norm(dim=1) / r).max()) < 1.2e-5
-    y = ops.dimq_linear_wq(x[:1024], packed, books, bias, n, k, bits=bits, group_rows=group_rows, epilogue="relu",
-                           residual=res[:1024])
-    z = (want[:1024] + bias.double()).relu() + res[:1024].double()
+    mm = min(m, 1024)
+    y = ops.dimq_linear_wq(x[:mm], packed, books, bias, n, k, bits=bits, group_rows=group_rows, epilogue="relu",
+                           residual=res[:mm])
+    z = (want[:mm] + bias.double()).relu() + res[:mm].double()
     assert float((y.double() - z).norm() / z.norm()) < 1.2e-5
 
 
