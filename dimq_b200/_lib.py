@@ -27,7 +27,7 @@ EXPORTED_SYMBOLS = (
     "dimq_version", "dimq_status_string", "dimq_pack_u4", "dimq_unpack_u4", "dimq_pack_bits",
     "dimq_unpack_bits", "dimq_quantize_activation_u4", "dimq_build_product_table", "dimq_linear_lut",
     "dimq_conv_out_size", "dimq_conv2d_lut", "dimq_hard_quantize", "dimq_linear_wq", "dimq_conv2d_wq",
-    "dimq_last_device_status", "dimq_add_layer_norm", "dimq_conv_prepack", "dimq_conv2d_wq_static", "dimq_im2col", "dimq_max_pool_nhwc", "dimq_images_to_nhwc",
+    "dimq_last_device_status", "dimq_add_layer_norm", "dimq_attention_qkv", "dimq_conv_prepack", "dimq_conv2d_wq_static", "dimq_im2col", "dimq_max_pool_nhwc", "dimq_images_to_nhwc",
     "dimq_a4_workspace_bytes", "dimq_linear_lut_tc", "dimq_conv2d_lut_tc",
     "dimq_linear_a4_workspace_bytes", "dimq_linear_a4", "dimq_conv2d_a4_workspace_bytes", "dimq_conv2d_a4",
     "dimq_linear_wq_workspace_bytes", "dimq_linear_wq_ws", "dimq_expand_workspace_bytes", "dimq_linear_wq_expand",
@@ -82,7 +82,7 @@ def host():
 def is_available() -> bool:
     try:
         host()
-    except (RuntimeError, OSError, ImportError):
+    except (RuntimeError, OSError, ImportError, AttributeError):   # absent, unloadable, or older than this file
         return False
     return True
 

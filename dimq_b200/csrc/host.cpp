@@ -17,6 +17,7 @@
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 
+#include <cmath>
 #include <optional>
 #include <stdexcept>
 #include <string>
@@ -686,6 +687,19 @@ Tensor images_to_nhwc(const Tensor& x, at::ScalarType dtype, int* launches) {
   return y;
 }
 
+Tensor attention_qkv(const Tensor& qkv, int64_t heads, int* launches) {
+  require_cuda(qkv, "attention_qkv");
+  if (qkv.dim() != 3 || heads <= 0 || qkv.size(2) % (3 * heads) != 0) fail("attention_qkv expects [batch, tokens, 3 * heads * head_dim]");
+  const c10::cuda::CUDAGuard guard(qkv.device());
+  const Tensor xc = qkv.contiguous();
+  const int64_t d = xc.size(2) / (3 * heads);
+  Tensor y = at::empty({xc.size(0), xc.size(1), heads * d}, xc.options().memory_format(at::MemoryFormat::Contiguous));
+  check(dimq_attention_qkv(xc.data_ptr(), y.data_ptr(), xc.size(0), xc.size(1), heads, d,
+                           1.0f / std::sqrt(static_cast<float>(d)), dtype_code(xc, "qkv"), stream_of(qkv)), "attention_qkv");
+  *launches = 1;
+  return y;
+}
+
 // ---- the Python module ----------------------------------------------------------------------------
 
 #define ARGS(want, name) want_args(n, want, name)
@@ -868,6 +882,19 @@ PyObject* py_max_pool_nhwc(PyObject*, PyObject* const* a, Py_ssize_t n) {
   END_HANDLE_TH_ERRORS
 }
 
+PyObject* py_attention_qkv(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  ARGS(2, "attention_qkv");
+  const Tensor x = as_tensor(a[0]);
+  const int64_t heads = as_int(a[1]);
+  int launches = 0;
+  Tensor y;
+  { NO_GIL; y = attention_qkv(x, heads, &launches); }
+  count_launches(launches);
+  return THPVariable_Wrap(y);
+  END_HANDLE_TH_ERRORS
+}
+
 PyObject* py_images_to_nhwc(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   ARGS(2, "images_to_nhwc");
@@ -946,7 +973,7 @@ PyObject* py_set_launch_count(PyObject*, PyObject* list) {
 #define FAST(name) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_##name)), METH_FASTCALL, nullptr}
 PyMethodDef kMethods[] = {FAST(linear_wq), FAST(linear_a4), FAST(conv2d_wq), FAST(conv2d_a4),
                           FAST(hard_quantize), FAST(fake_quantize_ste), FAST(unpack_bits), FAST(pack_bits), FAST(add_layer_norm),
-                          FAST(max_pool_nhwc), FAST(images_to_nhwc),
+                          FAST(max_pool_nhwc), FAST(images_to_nhwc), FAST(attention_qkv),
                           {"set_launch_count", py_set_launch_count, METH_O, nullptr},
                           {nullptr, nullptr, 0, nullptr}};
 PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_host", nullptr, -1, kMethods, nullptr, nullptr, nullptr, nullptr};

@@ -574,6 +574,12 @@ def images_to_nhwc(images: torch.Tensor, dtype: torch.dtype = torch.bfloat16) ->
     return _lib.host().images_to_nhwc(images, dtype)
 
 
+def attention_qkv(qkv: torch.Tensor, heads: int) -> torch.Tensor:
+    """Softmax attention over a packed projection ``[B, T, 3 * heads * 64]`` (bf16 / fp16, at most 512 tokens) ->
+    ``[B, T, heads * 64]``: ``scaled_dot_product_attention`` without the split, permute and transpose around it."""
+    return _lib.host().attention_qkv(qkv, heads)
+
+
 def add_layer_norm(x: torch.Tensor, delta: torch.Tensor | None, weight: torch.Tensor, bias: torch.Tensor,
                    eps: float = 1e-6):
     """``(x + delta, LayerNorm(x + delta))`` over the last dimension (``delta=None``: ``(x, LayerNorm(x))``).

@@ -181,6 +181,12 @@ class DIMQViT(nn.Module):
 
     def _attention(self, qkv: torch.Tensor, b: int, t: int) -> torch.Tensor:
         hid, heads = self.cfg["hidden"], self.cfg["heads"]
+        # few blocks of 64 query rows, at most two per SM: one launch on the projection as it lies.  197 tokens, 12 heads,
+        # GPU us own / scaled_dot_product_attention: 5.3 / 6.5 for one image, 7.7 / 6.9 for four, 107 / 52 for 128 - and
+        # the eight tensor operations around the latter are ~20 us of host time per layer, which is what a small batch waits for
+        if (hid == 64 * heads and t <= 512 and b * heads * ((t + 63) // 64) <= 296
+                and self.act_dtype in (torch.bfloat16, torch.float16)):
+            return ops.attention_qkv(qkv.view(b, t, 3 * hid), heads)
         qkv = qkv.view(b, t, 3, heads, hid // heads).permute(2, 0, 3, 1, 4)
         a = F.scaled_dot_product_attention(qkv[0], qkv[1], qkv[2])
         return a.transpose(1, 2).reshape(b, t, hid)

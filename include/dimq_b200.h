@@ -333,6 +333,13 @@ DIMQ_API int dimq_conv2d_a4(const void* x, int x_dtype, const dimq_wq_weight* w,
 
 /* ---- dense helper of the whole-model harness --------------------------- */
 
+/* out[b][t][h][:] = softmax(scale * q k^T) v per batch b and head h, for qkv [batch][tokens][3][heads][64] (DIMQ_BF16 or
+ * DIMQ_F16, 16-byte aligned) and out [batch][tokens][heads][64]; at most 512 tokens, head_dim 64.  No counterpart in the
+ * reference: its models use torch's attention; this reads the qkv Linear's output and writes the projection's input as
+ * they are stored. */
+DIMQ_API int dimq_attention_qkv(const void* qkv, void* out, int64_t batch, int64_t tokens, int64_t heads, int64_t head_dim,
+                                float scale, int dtype, void* stream);
+
 /* h_out = LayerNorm(x [+ delta]) * gamma + beta over rows of `cols` 16-bit elements (DIMQ_BF16 or
  * DIMQ_F16), statistics in fp32; with delta != NULL the sum x + delta (rounded to the element type)
  * is also written to x_out (the residual stream).  cols % 8 == 0, cols <= 1024, 16-byte aligned rows.
