@@ -236,6 +236,8 @@ extern "C" int dimq_linear_wq_workspace_bytes(const void* x, int x_dtype, const 
   // - 16-bit - and aligned; dimq_linear_wq_ws checks the real one and falls back if it does not fit)
   if (linear_dense_pays(x, x_dtype, w, M, N, K) && (N * 2) % 16 == 0 && dense_supported(x, x_dtype, w, x, x_dtype, nullptr, M, N, K)) {
     *bytes = linear_dense_workspace_bytes(x, x_dtype, w, M, N, K);
+    // below 1024 rows the in-pipeline kernel may still split K here, for an output the dense kernel cannot write
+    if (!dense_pays(M) && tc_split_k(M, N, K) > 1 && *bytes < M * N * 4) *bytes = M * N * 4;
     return DIMQ_OK;
   }
   // else only where the automatic choice would take the tcgen05 kernel and splitting K pays
@@ -267,6 +269,9 @@ extern "C" int dimq_linear_wq_ws(const void* x, int x_dtype, const dimq_wq_weigh
       if (dense_supported(x, x_dtype, w, y, y_dtype, residual, M, N, K))
         return launch_linear_wq_dense(x, x_dtype, w, bias, bias_dtype, residual, y, y_dtype, M, N, K, epilogue,
                                       workspace, workspace_bytes, static_cast<cudaStream_t>(stream));
+      if (!dense_pays(M) && workspace_bytes >= M * N * 4 && tc_split_k(M, N, K) > 1 && tc_supported(x, x_dtype, w, M, N, K))
+        return launch_linear_wq_tc(x, x_dtype, w, bias, bias_dtype, residual, y, y_dtype, M, N, K, epilogue, 0,
+                                   static_cast<cudaStream_t>(stream), workspace, workspace_bytes);
     } else {
       return launch_linear_wq_tc(x, x_dtype, w, bias, bias_dtype, residual, y, y_dtype, M, N, K, epilogue, 0,
                                  static_cast<cudaStream_t>(stream), workspace, workspace_bytes);

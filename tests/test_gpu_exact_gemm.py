@@ -194,3 +194,13 @@ def test_conv2d_two_terms(ops, cout, cin, ks, stride, size):
                            packed_khwc=ops.conv_prepack(packed, wshape, 4))
     want = F.conv2d(x.double().contiguous(), w.view(wshape), bias.double(), stride, ks // 2)
     assert ops.last_device_status() == 0 and _rel(y, want) < 1.2e-5
+
+
+@pytest.mark.parametrize("m,k,n", [(200, 1024, 512), (300, 4096, 1024), (64, 768, 768)])
+def test_linear_output_type_the_dense_kernel_does_not_write(ops, m, k, n):
+    # bf16 activations with an fp16 result: the in-pipeline kernel, split or not, whatever the model prefers
+    packed, books, w = _weight(ops, n, k, 4, torch.float16, seed=m)
+    x, bias = torch.randn(m, k, device="cuda").bfloat16(), torch.randn(n, device="cuda")
+    y = ops.dimq_linear_wq(x, packed, books, bias, n, k, bits=4, out_dtype=torch.float16)
+    assert y.dtype == torch.float16 and ops.last_device_status() == 0
+    assert _rel(y, x.double() @ w.t() + bias.double()) < 2.0 ** -12 + 1.2e-5
