@@ -20,7 +20,7 @@ from typing import Any, Mapping
 import torch
 import torch.nn as nn
 
-from . import _lib, ops
+from . import ops
 
 
 def _eager(x: torch.Tensor) -> bool:
@@ -108,9 +108,10 @@ class DIMQLinear(_PackedBase):
         if self.act_scale is None:
             buf = self._buffers
             tiled = self._prepacked(x.numel() // self.in_features, x)
-            return _lib.host().linear_wq(x, buf["packed_weight"], buf["codebook"], buf["bias"], self.out_features,
-                                         self.in_features, self.bits, self.group_rows, self.out_dtype,
-                                         ops._EPILOGUES[self.epilogue], residual, tiled)
+            return ops.dimq_linear_wq(x, buf["packed_weight"], buf["codebook"], buf["bias"], self.out_features,
+                                      self.in_features, bits=self.bits, group_rows=self.group_rows,
+                                      out_dtype=self.out_dtype, epilogue=self.epilogue, residual=residual,
+                                      packed_tiled=tiled)
         rows = x.numel() // self.in_features
         if rows >= ops.A4_TC_MIN_ROWS and self.in_features % 64 == 0:
             # The fp32-grade form, except for an fp32 codebook on many rows: there it multiplies two fp16 terms in
@@ -179,10 +180,10 @@ class DIMQConv2d(_PackedBase):
         self._check_input(x)
         if self.act_scale is None:
             buf = self._buffers
-            return _lib.host().conv2d_wq(x, buf["packed_weight"], buf["codebook"], buf["bias"], self.weight_shape,
-                                         self.stride, self.padding, self.dilation, self.groups, self.bits,
-                                         self.group_rows, self.out_dtype, ops._EPILOGUES[self.epilogue], residual,
-                                         self._prepacked())
+            return ops.dimq_conv2d_wq(x, buf["packed_weight"], buf["codebook"], buf["bias"], self.weight_shape,
+                                      self.stride, self.padding, self.dilation, self.groups, bits=self.bits,
+                                      group_rows=self.group_rows, out_dtype=self.out_dtype, epilogue=self.epilogue,
+                                      residual=residual, packed_khwc=self._prepacked())
         khwc = self._prepacked()
         channels_last = x.dim() == 4 and x.is_contiguous(memory_format=torch.channels_last) and not x.is_contiguous()
         if khwc is not None and channels_last and self.stride[0] == self.stride[1] and self.stride[0] in (1, 2):
