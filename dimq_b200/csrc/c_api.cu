@@ -246,35 +246,78 @@ extern "C" int dimq_linear_wq_workspace_bytes(const void* x, int x_dtype, const 
   return DIMQ_OK;
 }
 
+// What dimq_linear_wq_ws does with a workspace of this size, decided in one place so that no call is refused with the
+// bytes the query asked for.  The query does not see the output: where it reports the expanded form's bytes and the
+// output does not suit that form, or reports the k split's bytes and the expanded form would suit the output (fp32 rows
+// of N % 8 == 4), the form whose scratch fits is taken, and the kernel without scratch where none does.
+namespace {
+enum class WsRoute { kPlain, kRegs, kExact, kDense, kSplit };
+
+int linear_ws_route(const void* x, int x_dtype, const dimq_wq_weight* w, const void* residual, const void* y, int y_dtype,
+                    int64_t M, int64_t N, int64_t K, int64_t workspace_bytes, WsRoute* route) {
+  *route = WsRoute::kPlain;
+  int64_t need = 0;
+  const int rc = dimq_linear_wq_workspace_bytes(x, x_dtype, w, M, N, K, &need);
+  if (rc != DIMQ_OK) return rc;
+  if (need == 0) return DIMQ_OK;
+  if (mma_regs_supported(x, x_dtype, w, M, N, K) && mma_regs_pays(w, N, K)) {
+    if (workspace_bytes < need) return DIMQ_ERR_SCRATCH_TOO_SMALL;
+    *route = WsRoute::kRegs;
+  } else if (x_dtype == DIMQ_F32) {     // runs without scratch too
+    if (workspace_bytes >= need && linear_exact_supported(false, x, x_dtype, w, y, y_dtype, residual, M, N, K))
+      *route = WsRoute::kExact;
+  } else if (linear_dense_pays(x, x_dtype, w, M, N, K) && workspace_bytes >= dense_workspace_bytes(x_dtype, w, N, K) &&
+             dense_supported(x, x_dtype, w, y, y_dtype, residual, M, N, K)) {
+    *route = WsRoute::kDense;           // many rows need the expanded weight's bytes alone
+  } else if ((!dense_pays(M) || (N * 2) % 16 != 0) && workspace_bytes >= M * N * 4 && tc_split_k(M, N, K) > 1 &&
+             tc_supported(x, x_dtype, w, M, N, K)) {
+    *route = WsRoute::kSplit;
+  } else if (workspace_bytes < need) {
+    return DIMQ_ERR_SCRATCH_TOO_SMALL;
+  }
+  return DIMQ_OK;
+}
+}  // namespace
+
+extern "C" int dimq_linear_wq_ws_plan(const void* x, int x_dtype, const dimq_wq_weight* w, const void* residual,
+                                      const void* y, int y_dtype, int64_t M, int64_t N, int64_t K,
+                                      int64_t workspace_bytes, int* kernels) {
+  if (w == nullptr || kernels == nullptr) return DIMQ_ERR_NULL_POINTER;
+  *kernels = 0;
+  if (M < 0 || N <= 0 || K <= 0) return DIMQ_ERR_BAD_SIZE;
+  if (!valid_dtype(x_dtype) || !valid_dtype(y_dtype)) return DIMQ_ERR_BAD_DTYPE;
+  int rc = check_wq_weight(w, N);
+  if (rc != DIMQ_OK || M == 0) return rc;
+  WsRoute route;
+  rc = linear_ws_route(x, x_dtype, w, residual, y, y_dtype, M, N, K, workspace_bytes, &route);
+  if (rc == DIMQ_OK) *kernels = route == WsRoute::kPlain ? 1 : 2;
+  return rc;
+}
+
 extern "C" int dimq_linear_wq_ws(const void* x, int x_dtype, const dimq_wq_weight* w, const void* bias, int bias_dtype,
                                  const void* residual, void* y, int y_dtype, int64_t M, int64_t N, int64_t K,
                                  int epilogue, void* workspace, int64_t workspace_bytes, void* stream) {
-  int64_t need = 0;
   if (w != nullptr && workspace != nullptr && M > 0 && N > 0 && K > 0 && valid_dtype(x_dtype) && valid_dtype(y_dtype) &&
       (bias == nullptr || valid_dtype(bias_dtype)) && epilogue >= DIMQ_EPI_NONE && epilogue <= DIMQ_EPI_ADD_RELU &&
-      x != nullptr && y != nullptr &&
-      dimq_linear_wq_workspace_bytes(x, x_dtype, w, M, N, K, &need) == DIMQ_OK && need > 0) {
-    // fp32 activations run without scratch too, many 16-bit rows with the expanded weight's alone
-    if (workspace_bytes < need && x_dtype != DIMQ_F32 &&
-        !(linear_dense_pays(x, x_dtype, w, M, N, K) && workspace_bytes >= dense_workspace_bytes(x_dtype, w, N, K)))
-      return DIMQ_ERR_SCRATCH_TOO_SMALL;
-    if (mma_regs_supported(x, x_dtype, w, M, N, K) && mma_regs_pays(w, N, K))
-      return launch_linear_wq_mma_regs(x, x_dtype, w, bias, bias_dtype, residual, y, y_dtype, M, N, K, epilogue, workspace,
-                                       workspace_bytes, static_cast<cudaStream_t>(stream));
-    if (x_dtype == DIMQ_F32) {
-      if (workspace_bytes >= need && linear_exact_supported(false, x, x_dtype, w, y, y_dtype, residual, M, N, K))
+      x != nullptr && y != nullptr) {
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    WsRoute route;
+    const int rc = linear_ws_route(x, x_dtype, w, residual, y, y_dtype, M, N, K, workspace_bytes, &route);
+    if (rc != DIMQ_OK) return rc;
+    switch (route) {
+      case WsRoute::kRegs:
+        return launch_linear_wq_mma_regs(x, x_dtype, w, bias, bias_dtype, residual, y, y_dtype, M, N, K, epilogue, workspace,
+                                         workspace_bytes, st);
+      case WsRoute::kExact:
         return launch_linear_exact(false, x, x_dtype, 1.0f, 0, w, bias, bias_dtype, residual, y, y_dtype, M, N, K, epilogue,
-                                   workspace, workspace_bytes, static_cast<cudaStream_t>(stream));
-    } else if (linear_dense_pays(x, x_dtype, w, M, N, K)) {
-      if (dense_supported(x, x_dtype, w, y, y_dtype, residual, M, N, K))
-        return launch_linear_wq_dense(x, x_dtype, w, bias, bias_dtype, residual, y, y_dtype, M, N, K, epilogue,
-                                      workspace, workspace_bytes, static_cast<cudaStream_t>(stream));
-      if (!dense_pays(M) && workspace_bytes >= M * N * 4 && tc_split_k(M, N, K) > 1 && tc_supported(x, x_dtype, w, M, N, K))
-        return launch_linear_wq_tc(x, x_dtype, w, bias, bias_dtype, residual, y, y_dtype, M, N, K, epilogue, 0,
-                                   static_cast<cudaStream_t>(stream), workspace, workspace_bytes);
-    } else {
-      return launch_linear_wq_tc(x, x_dtype, w, bias, bias_dtype, residual, y, y_dtype, M, N, K, epilogue, 0,
-                                 static_cast<cudaStream_t>(stream), workspace, workspace_bytes);
+                                   workspace, workspace_bytes, st);
+      case WsRoute::kDense:
+        return launch_linear_wq_dense(x, x_dtype, w, bias, bias_dtype, residual, y, y_dtype, M, N, K, epilogue, workspace,
+                                      workspace_bytes, st);
+      case WsRoute::kSplit:
+        return launch_linear_wq_tc(x, x_dtype, w, bias, bias_dtype, residual, y, y_dtype, M, N, K, epilogue, 0, st, workspace,
+                                   workspace_bytes);
+      case WsRoute::kPlain: break;
     }
   }
   return dimq_linear_wq(x, x_dtype, w, bias, bias_dtype, residual, y, y_dtype, M, N, K, epilogue, DIMQ_ALGO_AUTO, stream);

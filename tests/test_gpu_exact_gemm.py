@@ -204,3 +204,15 @@ def test_linear_output_type_the_dense_kernel_does_not_write(ops, m, k, n):
     y = ops.dimq_linear_wq(x, packed, books, bias, n, k, bits=4, out_dtype=torch.float16)
     assert y.dtype == torch.float16 and ops.last_device_status() == 0
     assert _rel(y, x.double() @ w.t() + bias.double()) < 2.0 ** -12 + 1.2e-5
+
+
+@pytest.mark.parametrize("n", [100, 500, 1004])
+@pytest.mark.parametrize("m,k", [(33, 1024), (64, 4096), (197, 1024), (512, 2048), (1000, 4096), (1025, 2048), (2000, 1024)])
+def test_linear_fp32_result_in_rows_the_16_bit_form_cannot_write(ops, m, k, n):
+    # N % 8 == 4: the split or unsplit in-pipeline kernel, with the scratch its query reports
+    packed, books, w = _weight(ops, n, k, 4, torch.float16, seed=m)
+    x, bias = torch.randn(m, k, device="cuda").bfloat16(), torch.randn(n, device="cuda")
+    y = ops.dimq_linear_wq(x, packed, books, bias, n, k, bits=4)
+    assert y.dtype == torch.float32 and ops.last_device_status() == 0
+    # hi + lo codewords carry 2^-17; the accumulators truncate, 1.2e-6 per 1024 products
+    assert _rel(y, x.double() @ w.t() + bias.double()) < 1.2e-5

@@ -111,6 +111,25 @@ def test_small_m_kernel_plan_through_the_workspace_queries(lib):
     assert query(auto, 4, 4096, 1024) == (0, 0)                         # K below 2048: the index-streaming kernel
 
 
+@pytest.mark.parametrize("x_dtype,y_dtype,book", [(2, 0, 1), (2, 2, 1), (1, 0, 1), (2, 0, 2), (2, 1, 1), (0, 0, 1), (0, 2, 0)])
+def test_linear_workspace_of_the_queried_size_is_enough(lib, x_dtype, y_dtype, book):
+    """dimq_linear_wq_ws takes every call with the bytes its query reports, whatever form the shape prefers and whatever the
+    output is (N % 8 == 4 with an fp32 output: the expanded form could write it, the query reports the k split's bytes)."""
+    from dimq_b200 import _lib
+
+    fake = 1 << 20                                   # an aligned address that is never dereferenced
+    need, kernels = C.c_int64(-1), C.c_int(-1)
+    for n in (100, 500, 1000, 1004, 4096):
+        w = _lib.WqWeight(fake, 4, fake, book, 16, 1, n, None)
+        for k in (768, 1024, 2048, 4096):
+            for m in (1, 8, 33, 40, 64, 197, 512, 1000, 1023, 1024, 1025, 3000):
+                shape = (C.c_int64(m), C.c_int64(n), C.c_int64(k))
+                assert lib.dimq_linear_wq_workspace_bytes(C.c_void_p(fake), x_dtype, C.byref(w), *shape, C.byref(need)) == 0
+                rc = lib.dimq_linear_wq_ws_plan(C.c_void_p(fake), x_dtype, C.byref(w), None, C.c_void_p(fake), y_dtype, *shape,
+                                                need, C.byref(kernels))
+                assert rc == 0 and kernels.value in ((1, 2) if need.value else (1,)), (m, n, k, rc)
+
+
 def test_conv_geometry(lib):
     from dimq_b200._lib import ConvGeom
 
