@@ -216,3 +216,16 @@ def test_linear_fp32_result_in_rows_the_16_bit_form_cannot_write(ops, m, k, n):
     assert y.dtype == torch.float32 and ops.last_device_status() == 0
     # hi + lo codewords carry 2^-17; the accumulators truncate, 1.2e-6 per 1024 products
     assert _rel(y, x.double() @ w.t() + bias.double()) < 1.2e-5
+
+
+@pytest.mark.parametrize("m,k,n", [(384, 4096, 1024), (384, 8192, 512), (197, 1024, 1024), (197, 2048, 1000), (576, 4096, 512)])
+@pytest.mark.parametrize("act,book", [(torch.float16, torch.float16), (torch.bfloat16, torch.bfloat16),
+                                      (torch.bfloat16, torch.float16)])
+def test_linear_fp32_result_below_1024_rows_sums_in_slices(ops, m, k, n, act, book):
+    # The tensor cores' accumulators lose 1.25e-9 of a sum per product (6.4e-7 at 512, 3.7e-6 at 3072).  These shapes are cut
+    # into at least four slices of K; where bf16 activations meet fp16 codewords each product is a hi + lo pair.
+    packed, books, w = _weight(ops, n, k, 4, book, seed=m)
+    x = torch.randn(m, k, device="cuda").to(act)
+    y = ops.dimq_linear_wq(x, packed, books, None, n, k, bits=4)
+    assert y.dtype == torch.float32 and ops.last_device_status() == 0
+    assert _rel(y, x.double() @ w.t()) < 1.1 * 1.25e-9 * k / 4 * (1 if act == book else 2)
