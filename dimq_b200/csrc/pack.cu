@@ -188,48 +188,40 @@ product_table_kernel(const void* __restrict__ codebook, int cb_dtype, int64_t to
 // [c[0], c[last]].  Then every |w - c| <= 2^21 g, two codewords on one side of w lie at distances that differ by g, at
 // least 2^-21 of either, so neither the subtraction nor the square (2^-24 each, no underflow or overflow) can make them
 // equal or swap them: the minimum is at one of the two codewords around w, and the lower one on a tie.  They are found
-// by bisection in a shared-memory table and compared exactly as the scan would.  Everything else - a codebook that is
-// not so spaced, a weight farther out, a NaN - is scanned.
+// by bisection in a shared-memory table and compared exactly as the scan would.
+// A codebook that is sorted and finite but not so spaced (duplicates, near-duplicates), or a weight farther out, is
+// bisected too, and the lowest index of a run of equal distances is found by walking down it, as in hard_quantize_kernel
+// (the argument stands there).  An unsorted or non-finite codebook is scanned, each codeword read once for eight weights;
+// so are up to 8 codewords that are not well spaced, where the scan is as short as the walk.
 //
 // Bound: HBM (4 bytes in, 1 + bits / 8 or 4 out per weight), with ~30 instructions per weight beside it.  The kernel
 // below it replaces here spent 64-bit divisions per element, a serial sortedness check per 2 048 weights and
 // byte-wise stores: 4096 x 1024 fp32, 16 codewords, indices + packed and their unpacking took 28.7 us per call there,
 // 16.4 here (both kernels and three allocations).
-__device__ __noinline__ uint32_t nearest_scan(float wv, const float* __restrict__ cb, int entries) {
-  float d = __fsub_rn(wv, cb[0]);
-  float best = __fmul_rn(d, d);
-  uint32_t bi = 0u;
-  for (int k = 1; k < entries; ++k) {
-    d = __fsub_rn(wv, cb[k]);
-    const float dd = __fmul_rn(d, d);
-    if (dd < best || (dd != dd && best == best)) { best = dd; bi = k; }   // a NaN beats any number, the first NaN stays
-  }
-  return bi;
-}
-
 template <typename T, int E>   // E: the number of codewords rounded up to a power of two
 __global__ void __launch_bounds__(kThreads)
 nearest_sorted_kernel(const T* __restrict__ w, int64_t n, int64_t group_elems, const float* __restrict__ codebooks,
                       int entries, uint8_t* __restrict__ idx_out, uint8_t* __restrict__ packed, int bits,
                       T* __restrict__ fake_out) {
   __shared__ float tab[E + 2];          // -inf, the codewords, +inf up to E
-  __shared__ int gap_bits, bad;
+  __shared__ int gap_bits, unsorted;
   const int tid = threadIdx.x;
   const float kInf = __int_as_float(0x7F800000);
   const float* cb = codebooks + static_cast<int64_t>(blockIdx.y) * entries;
-  if (tid == 0) { gap_bits = 0x7F800000; bad = 0; tab[0] = -kInf; tab[E + 1] = kInf; }
+  if (tid == 0) { gap_bits = 0x7F800000; unsorted = 0; tab[0] = -kInf; tab[E + 1] = kInf; }
   for (int k = tid; k < E; k += kThreads) tab[k + 1] = k < entries ? cb[k] : kInf;
   __syncthreads();
   for (int k = tid; k + 1 < entries; k += kThreads) {
     const float gap = __fsub_rn(tab[k + 2], tab[k + 1]);
-    if (!(gap > 0.0f) || !isfinite(tab[k + 1]) || !isfinite(tab[k + 2])) bad = 1;
-    else atomicMin(&gap_bits, __float_as_int(gap));     // positive floats order like their bits
+    if (!(gap >= 0.0f) || !isfinite(tab[k + 1]) || !isfinite(tab[k + 2])) unsorted = 1;
+    else atomicMin(&gap_bits, __float_as_int(gap));     // floats from zero up order like their bits
   }
   __syncthreads();
   const float gap = __int_as_float(gap_bits);
   const float first = tab[1], last = tab[entries];
   const float reach = gap * 1048576.0f;
-  const bool spaced = bad == 0 && entries > 1 && gap >= 8.8817842e-16f && gap <= 2.7487791e11f && last - first <= reach;
+  const bool sorted = unsorted == 0 && entries > 8;
+  const bool spaced = unsorted == 0 && entries > 1 && gap >= 8.8817842e-16f && gap <= 2.7487791e11f && last - first <= reach;
   // limits a little inside the proven range (the sums round)
   const float lim_lo = spaced ? first - 0.5f * reach : kInf, lim_hi = spaced ? last + 0.5f * reach : -kInf;
 
@@ -259,7 +251,7 @@ nearest_sorted_kernel(const T* __restrict__ w, int64_t n, int64_t group_elems, c
     bool in = true;
 #pragma unroll
     for (int i = 0; i < 8; ++i) in = in && f[i] >= lim_lo && f[i] <= lim_hi;
-    if (in) {
+    if (in || sorted) {
       int pos[8];        // number of codewords below the weight, at most E - 1
 #pragma unroll
       for (int i = 0; i < 8; ++i) pos[i] = 0;
@@ -268,17 +260,52 @@ nearest_sorted_kernel(const T* __restrict__ w, int64_t n, int64_t group_elems, c
 #pragma unroll
         for (int i = 0; i < 8; ++i) pos[i] += tab[pos[i] + step] < f[i] ? step : 0;
       }
+      if (in) {
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        float d = __fsub_rn(f[i], tab[pos[i]]);
-        const float dlo = __fmul_rn(d, d);
-        d = __fsub_rn(f[i], tab[pos[i] + 1]);
-        const float dhi = __fmul_rn(d, d);
-        r[i] = static_cast<uint32_t>(dhi < dlo ? pos[i] : pos[i] - 1);
+        for (int i = 0; i < 8; ++i) {
+          float d = __fsub_rn(f[i], tab[pos[i]]);
+          const float dlo = __fmul_rn(d, d);
+          d = __fsub_rn(f[i], tab[pos[i] + 1]);
+          const float dhi = __fmul_rn(d, d);
+          r[i] = static_cast<uint32_t>(dhi < dlo ? pos[i] : pos[i] - 1);
+        }
+      } else {
+        const float* c = tab + 1;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const int lo = pos[i] > 0 ? pos[i] - 1 : 0, hi = pos[i] < entries ? pos[i] : entries - 1;
+          float d = __fsub_rn(f[i], c[lo]);
+          const float dlo = __fmul_rn(d, d);
+          d = __fsub_rn(f[i], c[hi]);
+          const float dhi = __fmul_rn(d, d);
+          int b = dhi < dlo ? hi : lo;
+          const float best = dhi < dlo ? dhi : dlo;
+          if (!isfinite(f[i])) b = 0;      // the same distance, infinite or NaN, to every codeword
+          while (b > 0) {
+            d = __fsub_rn(f[i], c[b - 1]);
+            if (__fmul_rn(d, d) != best) break;
+            --b;
+          }
+          r[i] = static_cast<uint32_t>(b);
+        }
       }
     } else {
+      float best[8];
 #pragma unroll
-      for (int i = 0; i < 8; ++i) r[i] = nearest_scan(f[i], tab + 1, entries);
+      for (int i = 0; i < 8; ++i) {
+        const float d = __fsub_rn(f[i], first);
+        best[i] = __fmul_rn(d, d);
+        r[i] = 0u;
+      }
+      for (int k = 1; k < entries; ++k) {
+        const float c = tab[k + 1];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const float d = __fsub_rn(f[i], c);
+          const float dd = __fmul_rn(d, d);
+          if (dd < best[i] || (dd != dd && best[i] == best[i])) { best[i] = dd; r[i] = k; }   // the first NaN stays
+        }
+      }
     }
     if (idx_out != nullptr) {
       if (full) {

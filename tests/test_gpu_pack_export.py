@@ -291,3 +291,74 @@ def test_nearest_codeword_groups_and_tails(ops, rows, cols, group_rows, bits, dt
     fq = ops.fake_quantize_ste(wt, _cuda(cb), group_rows=group_rows or rows)
     c = torch.from_numpy(np.take_along_axis(cb[np.arange(rows) // (group_rows or rows)], want.astype(np.int64), 1)).cuda()
     assert torch.equal(fq, wt + (c.to(wt.dtype) - wt))
+
+
+def _odd_books(kind, entries, groups, rng):
+    """Codebooks that are not strictly increasing with wide gaps."""
+    cb = np.sort((rng.standard_normal((groups, entries)) * 0.05).astype(np.float32), axis=1)
+    half = entries // 2
+    if kind == "duplicate":
+        cb[:, half] = cb[:, half - 1]
+    elif kind == "zeros":                       # quantiles of pruned weights
+        cb[:, entries // 4: half + 1] = 0.0
+        cb = np.sort(cb, axis=1)
+    elif kind == "one value":
+        cb[:] = 0.01
+    elif kind == "close":                       # gaps of one rounding step beside a span of 2^25 of them
+        cb[:, half] = np.nextafter(cb[:, half - 1], np.float32(1))
+        cb[:, 0], cb[:, -1] = -1.0, 1.0
+    elif kind == "swapped":
+        cb[:, [0, 1]] = cb[:, [1, 0]]
+    elif kind == "shuffled":
+        cb = cb[:, rng.permutation(entries)]
+    elif kind == "infinite":
+        cb[:, 0], cb[:, -1] = -np.inf, np.inf
+    elif kind == "nan":
+        cb[:, half] = np.nan
+    elif kind == "huge":                        # squares overflow
+        cb = np.sort(cb * np.float32(1e21), axis=1)
+        cb[:, -1] = 3e38
+    return np.ascontiguousarray(cb)
+
+
+@pytest.mark.parametrize("kind", ["duplicate", "zeros", "one value", "close", "swapped", "shuffled", "infinite", "nan", "huge"])
+@pytest.mark.parametrize("rows,cols,group_rows,bits", [(64, 147, None, 4), (257, 512, 128, 3), (300, 4608, 100, 8), (64, 1024, 8, 4),
+                                                       (40, 104, 40, 2)])
+def test_nearest_codeword_of_books_that_are_not_well_spaced(ops, rows, cols, group_rows, bits, kind):
+    from oracle import c_oracle
+
+    rng = np.random.default_rng(rows + cols + len(kind))
+    groups = 1 if group_rows is None else (rows + group_rows - 1) // group_rows
+    cb = _odd_books(kind, 1 << bits, groups, rng)
+    w = (rng.standard_normal((rows, cols)) * 0.05).astype(np.float32)
+    flat = w.reshape(-1)
+    flat[: 1 << bits] = cb[0]                   # on the codewords themselves, and half way between two
+    flat[100:100 + (1 << bits) - 1] = (cb[0, 1:] * np.float32(0.5) + cb[0, :-1] * np.float32(0.5))
+    flat[400:408] = [0.0, -0.0, 1e30, -1e30, 3e38, np.inf, -np.inf, np.nan]
+    want = c_oracle.hard_quantize(w, cb, group_rows or rows)
+    idx, packed = ops.hard_quantize(_cuda(w), _cuda(cb), group_rows=group_rows or rows, bits=bits)
+    assert np.array_equal(idx.cpu().numpy(), want)
+    assert np.array_equal(packed.cpu().numpy(), ops.pack_bits(idx, bits).cpu().numpy())
+
+
+def test_a_duplicate_codeword_costs_no_scan(ops):
+    """256 sorted codewords, two of them equal: bisection and a short walk, not 256 distances per weight (that took 16 times
+    the time of the well-spaced book)."""
+    w = torch.randn(4096, 1024, device="cuda")
+    cb = torch.linspace(-3, 3, 256, device="cuda")
+    dup = cb.clone()
+    dup[100] = dup[99]
+
+    def us(book):
+        start, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        best = float("inf")
+        for _ in range(6):
+            start.record()
+            for _ in range(5):
+                ops.hard_quantize(w, book, bits=8)
+            end.record()
+            end.synchronize()
+            best = min(best, start.elapsed_time(end))
+        return best
+
+    assert us(dup) < 5 * us(cb)
