@@ -31,7 +31,7 @@ def is_available() -> bool:
 
 
 def require_extension() -> None:
-    _lib.lib()
+    _lib.host()
 
 
 def _require_cuda(t: torch.Tensor, what: str) -> None:
@@ -188,12 +188,21 @@ _SCHEMAS = (
 _TORCH_LIBRARY = None
 
 
-def _missing(*args):
-    _lib.host()     # raises: what is missing and how to build it
+def _on_first_call(name: str):
+    """What ``torch.ops.dimq.<name>`` runs until the native host path is loaded: it loads it (or raises: what is missing and
+    how to build it), which registers the CUDA kernel in front of this one, and calls again."""
+    def load_and_call(*args):
+        if not any(isinstance(a, torch.Tensor) and a.is_cuda for a in args):
+            raise NotImplementedError(f"dimq::{name} runs on CUDA tensors only")
+        _lib.host()
+        return getattr(torch.ops.dimq, name)(*args)
+
+    return load_and_call
 
 
 def _register() -> None:
-    """The six schemas; four of their kernels are registered by the native host path when it is loaded."""
+    """The six schemas.  Importing this package maps no compiled file, so that a build in the same process is the one that
+    is used: four of the kernels are registered (for CUDA) by the native host path when it is first loaded."""
     global _TORCH_LIBRARY
     if _TORCH_LIBRARY is not None:
         return
@@ -202,9 +211,8 @@ def _register() -> None:
         library.define(schema)
     library.impl("quantize_activation_u4", _quantize_activation_u4_impl, "CUDA")
     library.impl("build_product_table", _build_product_table_impl, "CUDA")
-    if not _lib.is_available():
-        for name in ("pack_u4", "unpack_u4", "linear_lut", "conv2d_lut"):
-            library.impl(name, _missing, "CUDA")
+    for name in ("pack_u4", "unpack_u4", "linear_lut", "conv2d_lut"):
+        library.impl(name, _on_first_call(name), "CompositeExplicitAutograd")
     _TORCH_LIBRARY = library
 
 

@@ -161,6 +161,49 @@ def test_ops_module_registers_reference_schemas():
         DIMQLinear(torch.zeros(8, dtype=torch.uint8), torch.zeros(8), 1.0, 8, 4, 4, bits=3)
 
 
+_LOADING = r"""
+import sys, torch
+sys.path.insert(0, sys.argv[1])
+import dimq_b200, dimq_backend
+from dimq_b200 import _lib, ops
+
+def mapped():
+    return [n for n in ("/libdimq_b200.so", "/dimq_b200/_host.so") if n in open("/proc/self/maps").read()]
+
+assert not mapped(), mapped()                        # a build in this process is still the one that gets loaded
+assert not torch._C._dispatch_has_kernel_for_dispatch_key("dimq::pack_u4", "CUDA")
+if sys.argv[2] == "missing":
+    _lib.LIB_PATH = _lib.LIB_PATH.with_name("absent.so")
+    assert not dimq_b200.is_available()
+    if torch.cuda.is_available():
+        try:
+            torch.ops.dimq.pack_u4(torch.zeros(4, dtype=torch.uint8, device="cuda"))
+        except RuntimeError as e:
+            assert "dimq_b200.build" in str(e)
+        else:
+            raise SystemExit("no error")
+elif sys.argv[2] == "call":
+    y = torch.ops.dimq.pack_u4(torch.tensor([1, 2, 3], dtype=torch.uint8, device="cuda"))    # the first call of all
+    assert y.tolist() == [0x21, 0x03] and mapped()
+else:
+    try:
+        torch.ops.dimq.pack_u4(torch.zeros(4, dtype=torch.uint8))
+    except NotImplementedError:
+        pass
+    assert not mapped()
+    assert dimq_b200.is_available() and mapped()
+    assert torch._C._dispatch_has_kernel_for_dispatch_key("dimq::pack_u4", "CUDA")
+print("ok")
+"""
+
+
+@pytest.mark.parametrize("mode", ["load", "missing", pytest.param("call", marks=pytest.mark.gpu)])
+def test_compiled_files_are_loaded_on_first_use(lib, mode):
+    out = subprocess.run([sys.executable, "-c", _LOADING, str(ROOT), mode], capture_output=True, text=True, timeout=300)
+    assert out.returncode == 0 and out.stdout.strip().endswith("ok"), out.stdout + out.stderr
+    assert "verrid" not in out.stderr, out.stderr
+
+
 def test_activation_qparams_helpers():
     from dimq_b200 import export
 
