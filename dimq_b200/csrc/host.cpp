@@ -256,14 +256,17 @@ Tensor linear_wq(const Tensor& x, const Tensor& packed, const Tensor& books, con
   void* st = stream_of(x);
   // Regimes that need scratch: a few activation rows against a large weight (the k slices of the small-M kernel meet
   // there), many activation rows (the indices are expanded once to a 16-bit weight), fp32 activations (split into
-  // fp16 terms) and a few hundred rows against a long K (split-K partial tiles).
+  // fp16 terms) and a few hundred rows against a long K (split-K partial tiles).  The query does not see the output:
+  // fp32 activations are split for an fp32 result only.
   int64_t need = 0;
-  dimq_linear_wq_workspace_bytes(xc.data_ptr(), xd, &w.w, m, n, k, &need);
+  if (xd != DIMQ_F32 || yd == DIMQ_F32) dimq_linear_wq_workspace_bytes(xc.data_ptr(), xd, &w.w, m, n, k, &need);
   if (need > 0) {
     Tensor ws = scratch(need, x);
+    int kernels = 0;
+    dimq_linear_wq_ws_plan(xc.data_ptr(), xd, &w.w, ptr(res), y.data_ptr(), yd, m, n, k, need, &kernels);
     check(dimq_linear_wq_ws(xc.data_ptr(), xd, &w.w, ptr(b.t), b.dtype, ptr(res), y.data_ptr(), yd, m, n, k, epilogue,
                             ws.data_ptr(), need, st), "linear_wq_ws");
-    *launches = 2;    // expansion + GEMM, or GEMM + the kernel that finishes the sums
+    *launches = kernels;    // expansion + GEMM, GEMM + the kernel that finishes the sums, or a GEMM alone
     return y;
   }
   check(dimq_linear_wq(xc.data_ptr(), xd, &w.w, ptr(b.t), b.dtype, ptr(res), y.data_ptr(), yd, m, n, k, epilogue,
@@ -425,8 +428,9 @@ Tensor conv2d_wq(const Tensor& x, const Tensor& packed, const Tensor& books, con
   void* st = stream_of(x);
   // Many output pixels: the indices are expanded once to a 16-bit weight in scratch for a dense tensor-core kernel -
   // the implicit GEMM over the re-ordered indices, or the stem kernel for a 3-channel stride-2 convolution.
+  // They write the activations' type or fp32.
   int64_t need = 0;
-  dimq_conv2d_wq_workspace_bytes(xc.data_ptr(), xd, &w.w, &g, &need);
+  if (yd == xd || yd == DIMQ_F32) dimq_conv2d_wq_workspace_bytes(xc.data_ptr(), xd, &w.w, &g, &need);
   if (need > 0) {
     Tensor ws = scratch(need, x);
     check(dimq_conv2d_wq_ws(xc.data_ptr(), xd, &w.w, ptr(b.t), b.dtype, ptr(residual), y.data_ptr(), yd, &g, epilogue,

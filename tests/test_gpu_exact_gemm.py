@@ -229,3 +229,37 @@ def test_linear_fp32_result_below_1024_rows_sums_in_slices(ops, m, k, n, act, bo
     y = ops.dimq_linear_wq(x, packed, books, None, n, k, bits=4)
     assert y.dtype == torch.float32 and ops.last_device_status() == 0
     assert _rel(y, x.double() @ w.t()) < 1.1 * 1.25e-9 * k / 4 * (1 if act == book else 2)
+
+
+@pytest.mark.parametrize("act,out,kernels", [(torch.float32, torch.float32, 2), (torch.float32, torch.bfloat16, 1),
+                                             (torch.bfloat16, torch.float16, 1), (torch.bfloat16, torch.float32, 2)])
+def test_linear_scratch_and_launch_count_follow_the_output(ops, act, out, kernels):
+    from dimq_b200 import _lib
+
+    m, k, n = 2000, 1024, 512
+    packed, books, w = _weight(ops, n, k, 4, torch.float16, seed=3)
+    x = torch.randn(m, k, device="cuda").to(act)
+    ops.dimq_linear_wq(x, packed, books, None, n, k, bits=4, out_dtype=out)
+    torch.cuda.synchronize()
+    torch.cuda.reset_peak_memory_stats()
+    before, count = torch.cuda.memory_allocated(), _lib.LAUNCH_COUNT[0]
+    y = ops.dimq_linear_wq(x, packed, books, None, n, k, bits=4, out_dtype=out)
+    assert _lib.LAUNCH_COUNT[0] - count == kernels
+    extra = torch.cuda.max_memory_allocated() - before - y.numel() * y.element_size()
+    if act == torch.float32:
+        assert (extra > 4 * m * k) == (out == torch.float32)     # the split activations, where they are used
+    assert _rel(y, x.double() @ w.t()) < {torch.float32: 1.2e-5, torch.bfloat16: 2.0 ** -8, torch.float16: 2.0 ** -11}[out]
+
+
+@pytest.mark.parametrize("out,kernels", [(torch.bfloat16, 2), (torch.float32, 2), (torch.float16, 1)])
+def test_conv_launch_count_follows_the_output(ops, out, kernels):
+    from dimq_b200 import _lib
+
+    packed, books, w = _weight(ops, 64, 64, 4, torch.bfloat16, seed=4)
+    x = torch.randn(4, 64, 20, 20, device="cuda").bfloat16().contiguous(memory_format=torch.channels_last)
+    khwc = ops.conv_prepack(packed, (64, 64, 1, 1), 4)
+    count = _lib.LAUNCH_COUNT[0]
+    y = ops.dimq_conv2d_wq(x, packed, books.reshape(-1), None, (64, 64, 1, 1), bits=4, out_dtype=out, packed_khwc=khwc)
+    assert _lib.LAUNCH_COUNT[0] - count == kernels
+    want = F.conv2d(x.double().contiguous(), w.view(64, 64, 1, 1))
+    assert _rel(y, want) < {torch.float32: 1.2e-5, torch.bfloat16: 2.0 ** -8, torch.float16: 2.0 ** -11}[out]
