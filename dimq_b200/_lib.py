@@ -76,6 +76,8 @@ def host():
     module = importlib.util.module_from_spec(spec)
     spec.loader.exec_module(module)
     module.set_launch_count(LAUNCH_COUNT)
+    from . import ops
+    module.set_ops(vars(ops))
     return module
 
 

@@ -152,6 +152,15 @@ void count_launches(int n) {          // GIL held
   if (nv == nullptr || PyList_SetItem(g_launch_count, 0, nv) != 0) throw python_error();
 }
 
+PyObject* g_ops = nullptr;            // the namespace of dimq_b200.ops, which states the rules both sides follow
+
+int64_t a4_tc_min_rows() {            // GIL not held
+  pybind11::gil_scoped_acquire gil;
+  PyObject* v = g_ops != nullptr ? PyDict_GetItemString(g_ops, "A4_TC_MIN_ROWS") : nullptr;
+  if (v == nullptr) fail("dimq_b200.ops.A4_TC_MIN_ROWS is missing");
+  return as_int(v);
+}
+
 void check(int status, const char* what) {
   if (status != DIMQ_OK)
     fail(std::string("dimq_b200.") + what + " failed: " + dimq_status_string(status) + " (status " + std::to_string(status) + ")");
@@ -311,7 +320,7 @@ OptTensor linear_a4(const Tensor& x, const Tensor& packed, const Tensor& book, d
 
 // The reference's linear_lut: fp32 output, one 16-entry codebook.
 Tensor linear_lut(const Tensor& x, const Tensor& packed, const Tensor& book, double scale, int64_t zp, const OptTensor& bias,
-                  int64_t n, int64_t k, int64_t tc_min_rows, int* launches) {
+                  int64_t n, int64_t k, int* launches) {
   require_cuda(x, "linear_lut");
   require_cuda(packed, "linear_lut");
   require_cuda(book, "linear_lut");
@@ -333,7 +342,7 @@ Tensor linear_lut(const Tensor& x, const Tensor& packed, const Tensor& book, dou
   if (linear_a4_into(xc, w, scale, zp, b, std::nullopt, y, m, n, k, DIMQ_EPI_NONE, launches)) return y;
   const int xd = dtype_code(xc, "x");
   void* st = stream_of(x);
-  if (m >= tc_min_rows && k % 64 == 0 && reinterpret_cast<uintptr_t>(w.pw.data_ptr()) % 16 == 0) {
+  if (k % 64 == 0 && reinterpret_cast<uintptr_t>(w.pw.data_ptr()) % 16 == 0 && m >= a4_tc_min_rows()) {
     int64_t need = 0;
     check(dimq_a4_workspace_bytes(xc.numel(), 0, &need), "a4_workspace_bytes");
     Tensor ws = scratch(need, x);
@@ -494,7 +503,7 @@ OptTensor conv2d_a4(const Tensor& x, const Tensor& packed, const Tensor& book, d
 
 // The reference's conv2d_lut: fp32 output, one 16-entry codebook.
 Tensor conv2d_lut(const Tensor& x, const Tensor& packed, const Tensor& book, double scale, int64_t zp, const OptTensor& bias,
-                  const ConvArgs& a, int64_t tc_min_rows, int* launches) {
+                  const ConvArgs& a, int* launches) {
   require_cuda(x, "conv2d_lut");
   if (x.dim() != 4) fail("conv2d_lut expects NCHW input");
   require_cuda(packed, "conv2d_lut");
@@ -518,7 +527,7 @@ Tensor conv2d_lut(const Tensor& x, const Tensor& packed, const Tensor& book, dou
   void* st = stream_of(x);
   float* yp = static_cast<float*>(y.data_ptr());
   if (g.x_stride[1] == 1 && g.y_stride[1] == 1 && g.groups == 1 && g.in_channels % 64 == 0 &&
-      static_cast<int64_t>(g.batch) * g.out_h * g.out_w >= tc_min_rows) {
+      static_cast<int64_t>(g.batch) * g.out_h * g.out_w >= a4_tc_min_rows()) {
     int64_t need = 0;
     check(dimq_a4_workspace_bytes(xc.numel(), numel, &need), "a4_workspace_bytes");
     Tensor ws = scratch(need, x);
@@ -934,12 +943,10 @@ Tensor op_unpack_u4(const Tensor& packed, int64_t numel) {
   return y;
 }
 
-constexpr int64_t kA4TcMinRows = 512;   // ops.A4_TC_MIN_ROWS
-
 Tensor op_linear_lut(const Tensor& x, const Tensor& packed_w, const Tensor& codebook, double act_scale, int64_t act_zp,
                      const OptTensor& bias, int64_t out_features, int64_t in_features) {
   int launches = 0;
-  Tensor y = linear_lut(x, packed_w, codebook, act_scale, act_zp, bias, out_features, in_features, kA4TcMinRows, &launches);
+  Tensor y = linear_lut(x, packed_w, codebook, act_scale, act_zp, bias, out_features, in_features, &launches);
   count_launches_no_gil(launches);
   return y;
 }
@@ -952,7 +959,7 @@ Tensor op_conv2d_lut(const Tensor& x, const Tensor& packed_w, const Tensor& code
   const ConvArgs a = {{i32(out_channels), i32(in_channels_per_group), i32(kernel_h), i32(kernel_w)}, i32(stride_h), i32(stride_w),
                       i32(pad_h), i32(pad_w), i32(dilation_h), i32(dilation_w), groups};
   int launches = 0;
-  Tensor y = conv2d_lut(x, packed_w, codebook, act_scale, act_zp, bias, a, kA4TcMinRows, &launches);
+  Tensor y = conv2d_lut(x, packed_w, codebook, act_scale, act_zp, bias, a, &launches);
   count_launches_no_gil(launches);
   return y;
 }
@@ -974,11 +981,22 @@ PyObject* py_set_launch_count(PyObject*, PyObject* list) {
   Py_RETURN_NONE;
 }
 
+PyObject* py_set_ops(PyObject*, PyObject* dict) {
+  if (!PyDict_Check(dict)) {
+    PyErr_SetString(PyExc_TypeError, "expected the namespace of dimq_b200.ops");
+    return nullptr;
+  }
+  Py_INCREF(dict);
+  Py_XSETREF(g_ops, dict);
+  Py_RETURN_NONE;
+}
+
 #define FAST(name) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_##name)), METH_FASTCALL, nullptr}
 PyMethodDef kMethods[] = {FAST(linear_wq), FAST(linear_a4), FAST(conv2d_wq), FAST(conv2d_a4),
                           FAST(hard_quantize), FAST(fake_quantize_ste), FAST(unpack_bits), FAST(pack_bits), FAST(add_layer_norm),
                           FAST(max_pool_nhwc), FAST(images_to_nhwc), FAST(attention_qkv),
                           {"set_launch_count", py_set_launch_count, METH_O, nullptr},
+                          {"set_ops", py_set_ops, METH_O, nullptr},
                           {nullptr, nullptr, 0, nullptr}};
 PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_host", nullptr, -1, kMethods, nullptr, nullptr, nullptr, nullptr};
 

@@ -263,3 +263,19 @@ def test_conv_launch_count_follows_the_output(ops, out, kernels):
     assert _lib.LAUNCH_COUNT[0] - count == kernels
     want = F.conv2d(x.double().contiguous(), w.view(64, 64, 1, 1))
     assert _rel(y, want) < {torch.float32: 1.2e-5, torch.bfloat16: 2.0 ** -8, torch.float16: 2.0 ** -11}[out]
+
+
+def test_a4_row_limit_is_the_one_ops_states(ops, monkeypatch):
+    # rows of 3 fp32 elements: not the fp32-grade form; the limit chooses between the bf16 pair (two launches) and the table
+    from dimq_b200 import _lib
+
+    m, k, n = 600, 128, 3
+    packed, books, w = _weight(ops, n, k, 4, torch.float32, seed=8)
+    x = torch.randn(m, k, device="cuda")
+    want = _codes(x, 0.23, 7) @ w.t()
+    for limit, kernels in ((ops.A4_TC_MIN_ROWS, 2), (m, 2), (m + 1, 1)):
+        monkeypatch.setattr(ops, "A4_TC_MIN_ROWS", limit)
+        count = _lib.LAUNCH_COUNT[0]
+        y = ops.dimq_linear_lut(x, packed, books.reshape(-1), 0.23, 7, None, n, k)
+        assert _lib.LAUNCH_COUNT[0] - count == kernels, limit
+        assert _rel(y, want) < 1.2e-5
