@@ -35,6 +35,11 @@ void require_cuda(const Tensor& t, const char* what) {
   if (!t.is_cuda()) fail(std::string(what) + " expects a CUDA tensor");
 }
 
+// The kernels get raw pointers: every operand has to be where x is.
+void same_device(const Tensor& t, const Tensor& x, const char* what) {
+  if (t.device() != x.device()) fail(std::string(what) + " must be on the device of the input, " + x.device().str() + ", got " + t.device().str());
+}
+
 int dtype_code(const Tensor& t, const char* what) {
   switch (t.scalar_type()) {
     case at::kFloat: return DIMQ_F32;
@@ -180,10 +185,12 @@ struct Weight {
   dimq_wq_weight w;
 };
 
-Weight wq_weight(const Tensor& packed, const Tensor& books, int64_t bits, int64_t out_rows, int64_t numel,
+Weight wq_weight(const Tensor& x, const Tensor& packed, const Tensor& books, int64_t bits, int64_t out_rows, int64_t numel,
                  std::optional<int64_t> group_rows, const OptTensor& second) {
   require_cuda(packed, "weight-only op");
   require_cuda(books, "weight-only op");
+  same_device(packed, x, "packed_weight");
+  same_device(books, x, "codebook");
   if (packed.scalar_type() != at::kByte) fail("packed_weight must be uint8");
   if (!at::isFloatingType(books.scalar_type())) fail("codebook must be floating point");
   if (bits != 2 && bits != 3 && bits != 4 && bits != 8) fail("unsupported weight bit width " + std::to_string(bits));
@@ -205,6 +212,7 @@ Weight wq_weight(const Tensor& packed, const Tensor& books, int64_t bits, int64_
     r.second = second->contiguous();
     if (r.second->scalar_type() != at::kByte || !r.second->is_cuda() || r.second->numel() < need)
       fail("packed_khwc must be a CUDA uint8 tensor as large as packed_weight");
+    same_device(*r.second, x, "packed_khwc");
   }
   r.w.packed = static_cast<const uint8_t*>(r.pw.data_ptr());
   r.w.bits = static_cast<int32_t>(bits);
@@ -222,10 +230,11 @@ struct Bias {
   int dtype = 0;
 };
 
-Bias bias_arg(const OptTensor& bias, int64_t n, const char* what) {
+Bias bias_arg(const OptTensor& bias, const Tensor& x, int64_t n, const char* what) {
   Bias b;
   if (!bias.has_value()) return b;
   if (!bias->is_cuda()) fail("bias must be CUDA when provided");
+  same_device(*bias, x, "bias");
   if (bias->numel() != n) fail(std::string("bias numel must equal ") + what);
   b.t = bias->contiguous();
   b.dtype = dtype_code(*b.t, "bias");
@@ -242,6 +251,7 @@ OptTensor linear_residual(const OptTensor& residual, const Tensor& y) {
   if (!residual.has_value()) return std::nullopt;
   if (residual->scalar_type() != y.scalar_type() || residual->numel() != y.numel())
     fail("residual must match the output shape and dtype");
+  same_device(*residual, y, "residual");
   return residual->contiguous();
 }
 
@@ -255,8 +265,8 @@ Tensor linear_wq(const Tensor& x, const Tensor& packed, const Tensor& books, con
   if (n <= 0 || k <= 0) fail("linear dimensions must be positive");
   if (x.dim() == 0 || x.size(-1) != k) fail("input last dimension must equal in_features");
   const Tensor xc = x.contiguous();
-  Weight w = wq_weight(packed, books, bits, n, n * k, group_rows, tiled);
-  const Bias b = bias_arg(bias, n, "out_features");
+  Weight w = wq_weight(x, packed, books, bits, n, n * k, group_rows, tiled);
+  const Bias b = bias_arg(bias, x, n, "out_features");
   const c10::cuda::CUDAGuard guard(x.device());
   Tensor y = at::empty(out_shape(x, n), x.options().dtype(out_dtype).memory_format(at::MemoryFormat::Contiguous));
   const OptTensor res = linear_residual(residual, y);
@@ -308,9 +318,9 @@ OptTensor linear_a4(const Tensor& x, const Tensor& packed, const Tensor& book, d
   check_qparams(scale, zp);
   if (n <= 0 || k <= 0) fail("linear dimensions must be positive");
   if (x.dim() == 0 || x.size(-1) != k) fail("input last dimension must equal in_features");
-  Weight w = wq_weight(packed, book, 4, n, n * k, std::nullopt, std::nullopt);
+  Weight w = wq_weight(x, packed, book, 4, n, n * k, std::nullopt, std::nullopt);
   const Tensor xc = x.contiguous();
-  const Bias b = bias_arg(bias, n, "out_features");
+  const Bias b = bias_arg(bias, x, n, "out_features");
   const c10::cuda::CUDAGuard guard(x.device());
   Tensor y = at::empty(out_shape(x, n), x.options().dtype(out_dtype).memory_format(at::MemoryFormat::Contiguous));
   const OptTensor res = linear_residual(residual, y);
@@ -334,8 +344,8 @@ Tensor linear_lut(const Tensor& x, const Tensor& packed, const Tensor& book, dou
   if (packed.numel() < (n * k + 1) / 2) fail("packed_weight is too small for out_features * in_features");
   if (x.dim() == 0 || x.size(-1) != k) fail("input last dimension must equal in_features");
   const Tensor xc = x.contiguous();
-  Weight w = wq_weight(packed, book.contiguous().view(-1), 4, n, n * k, std::nullopt, std::nullopt);
-  const Bias b = bias_arg(bias, n, "out_features");
+  Weight w = wq_weight(x, packed, book.contiguous().view(-1), 4, n, n * k, std::nullopt, std::nullopt);
+  const Bias b = bias_arg(bias, x, n, "out_features");
   const c10::cuda::CUDAGuard guard(x.device());
   Tensor y = at::empty(out_shape(x, n), x.options().dtype(at::kFloat).memory_format(at::MemoryFormat::Contiguous));
   const int64_t m = xc.numel() / k;
@@ -413,6 +423,7 @@ void conv_residual(const OptTensor& residual, const Tensor& y) {
   if (residual.has_value() && (residual->scalar_type() != y.scalar_type() || residual->sizes() != y.sizes() ||
                                residual->strides() != y.strides()))
     fail("residual must match the output shape, dtype and memory format");
+  if (residual.has_value()) same_device(*residual, y, "residual");
 }
 
 int64_t weight_numel(const dimq_conv_geom& g) {
@@ -426,8 +437,8 @@ Tensor conv2d_wq(const Tensor& x, const Tensor& packed, const Tensor& books, con
   if (x.dim() != 4) fail("conv2d_wq expects NCHW input");
   if (!at::isFloatingType(x.scalar_type())) fail("conv2d_wq expects floating input");
   dimq_conv_geom g = conv_geom(x, a);
-  Weight w = wq_weight(packed, books, bits, g.out_channels, weight_numel(g), group_rows, khwc);
-  const Bias b = bias_arg(bias, g.out_channels, "out_channels");
+  Weight w = wq_weight(x, packed, books, bits, g.out_channels, weight_numel(g), group_rows, khwc);
+  const Bias b = bias_arg(bias, x, g.out_channels, "out_channels");
   const c10::cuda::CUDAGuard guard(x.device());
   Tensor y;
   const Tensor xc = conv_io(x, g, out_dtype, y);
@@ -490,8 +501,8 @@ OptTensor conv2d_a4(const Tensor& x, const Tensor& packed, const Tensor& book, d
   if (!at::isFloatingType(x.scalar_type())) fail("conv2d_a4 expects floating input");
   check_qparams(scale, zp);
   dimq_conv_geom g = conv_geom(x, a);
-  Weight w = wq_weight(packed, book, 4, g.out_channels, weight_numel(g), std::nullopt, khwc);
-  const Bias b = bias_arg(bias, g.out_channels, "out_channels");
+  Weight w = wq_weight(x, packed, book, 4, g.out_channels, weight_numel(g), std::nullopt, khwc);
+  const Bias b = bias_arg(bias, x, g.out_channels, "out_channels");
   const c10::cuda::CUDAGuard guard(x.device());
   Tensor y;
   const Tensor xc = conv_io(x, g, out_dtype, y);
@@ -516,12 +527,12 @@ Tensor conv2d_lut(const Tensor& x, const Tensor& packed, const Tensor& book, dou
   dimq_conv_geom g = conv_geom(x, a);
   const int64_t numel = weight_numel(g);
   if (packed.numel() < (numel + 1) / 2) fail("packed_weight is too small for requested conv weight shape");
-  const Bias b = bias_arg(bias, g.out_channels, "out_channels");
+  const Bias b = bias_arg(bias, x, g.out_channels, "out_channels");
   const c10::cuda::CUDAGuard guard(x.device());
   Tensor y;
   const Tensor xc = conv_io(x, g, at::kFloat, y);
   if (y.numel() == 0) return y;
-  Weight w = wq_weight(packed, book.contiguous().view(-1), 4, g.out_channels, numel, std::nullopt, std::nullopt);
+  Weight w = wq_weight(x, packed, book.contiguous().view(-1), 4, g.out_channels, numel, std::nullopt, std::nullopt);
   if (conv2d_a4_into(xc, w, scale, zp, b, std::nullopt, y, g, DIMQ_EPI_NONE, launches)) return y;
   const int xd = dtype_code(xc, "x");
   void* st = stream_of(x);
@@ -657,8 +668,11 @@ std::pair<Tensor, Tensor> add_layer_norm(const Tensor& x, const OptTensor& delta
   OptTensor dc;
   if (delta.has_value()) {
     dc = delta->contiguous();
+    same_device(*dc, x, "delta");
     if (dc->sizes() != xc.sizes() || dc->scalar_type() != xc.scalar_type()) fail("delta must match x in shape and dtype");
   }
+  same_device(weight, x, "weight");
+  same_device(bias, x, "bias");
   const Tensor w = weight.to(xc.scalar_type()).contiguous(), b = bias.to(xc.scalar_type()).contiguous();
   if (w.numel() != cols || b.numel() != cols) fail("weight / bias must have one element per column");
   Tensor x_out = dc.has_value() ? at::empty_like(xc) : xc;

@@ -279,3 +279,34 @@ def test_a4_row_limit_is_the_one_ops_states(ops, monkeypatch):
         y = ops.dimq_linear_lut(x, packed, books.reshape(-1), 0.23, 7, None, n, k)
         assert _lib.LAUNCH_COUNT[0] - count == kernels, limit
         assert _rel(y, want) < 1.2e-5
+
+
+def test_operands_on_another_device_are_refused(ops):
+    # the host path hands raw pointers to the kernels: each operand is checked before any launch
+    m, k, n = 64, 128, 64
+    packed, books, _ = _weight(ops, n, k, 4, torch.float16, seed=2)
+    x, bias, res = torch.randn(m, k, device="cuda"), torch.randn(n, device="cuda"), torch.randn(m, n, device="cuda")
+    img = torch.randn(2, 64, 8, 8, device="cuda")
+    cp, cb, _ = _weight(ops, 64, 64, 4, torch.float16, seed=3)
+    cb = cb.reshape(-1)
+    conv = (None, (64, 64, 1, 1))
+    h = torch.randn(4, 128, device="cuda").bfloat16()
+    g = torch.ones(128, device="cuda")
+    calls = [
+        lambda: ops.dimq_linear_wq(x, packed, books, bias, n, k, residual=res.cpu()),
+        lambda: ops.dimq_linear_wq(x, packed, books, bias.cpu(), n, k),
+        lambda: ops.dimq_linear_wq(x, packed.cpu(), books, bias, n, k),
+        lambda: ops.dimq_linear_wq(x, packed, books.cpu(), bias, n, k),
+        lambda: ops.dimq_linear_wq(x, packed, books, bias, n, k, packed_tiled=packed.cpu()),
+        lambda: ops.dimq_linear_a4(x, packed, books.reshape(-1), 0.1, 3, None, n, k, residual=res.cpu()),
+        lambda: ops.dimq_conv2d_wq(img, cp, cb, *conv, residual=torch.zeros(2, 64, 8, 8)),
+        lambda: ops.dimq_conv2d_wq(img, cp, cb, *conv, packed_khwc=cp.cpu()),
+        lambda: ops.add_layer_norm(h, h.cpu(), g, g),
+        lambda: ops.add_layer_norm(h, None, g.cpu(), g),
+        lambda: ops.add_layer_norm(h, None, g, g.cpu()),
+    ]
+    for i, call in enumerate(calls):
+        with pytest.raises(RuntimeError, match="device|CUDA"):
+            call()
+            torch.cuda.synchronize()
+            raise AssertionError(f"call {i} was accepted")
