@@ -199,7 +199,9 @@ extern "C" int dimq_attention_qkv(const void* qkv, void* out, int64_t batch, int
   const int tp = static_cast<int>((tokens + kChunk - 1) / kChunk * kChunk);
   const size_t smem = static_cast<size_t>(kQ + 2 * tp) * 128;
   auto kern = dtype == DIMQ_BF16 ? attention_qkv_kernel<true> : attention_qkv_kernel<false>;
-  const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+  // the kernel's largest, not this call's: the attribute belongs to the process, and another thread's smaller call between
+  // this line and the launch would take the limit away again
+  const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (kQ + 2 * kMaxT) * 128);
   if (e != cudaSuccess) return static_cast<int>(e);
   const dim3 grid(static_cast<unsigned>((tokens + kQ - 1) / kQ), static_cast<unsigned>(heads), static_cast<unsigned>(batch));
   kern<<<grid, kThreads, smem, static_cast<cudaStream_t>(stream)>>>(static_cast<const uint16_t*>(qkv), static_cast<uint16_t*>(out),

@@ -51,6 +51,8 @@ constexpr int kThreads = (1 + kProducers + kEpiWarps) * 32;
 constexpr uint32_t kABytes = kBM * kBK * 2;   // 16 KB
 constexpr int kHeaderBytes = 1024;
 constexpr int kBiasBytes = kEpiWarps * 128;
+// What a block may use.  Each kernel's limit is set to this, never to a call's own size: the attribute belongs to the process,
+// and a smaller call of another thread between the setting and the launch would take the limit away again.
 constexpr size_t kSmemMax = 227 * 1024;
 
 struct DenseParams {
@@ -987,25 +989,25 @@ int launch_dense(DenseMaps& maps, DenseParams& p, const void* scratch, int64_t K
   if (pair) {
     const int clusters = static_cast<int>(tiles < kNumSMs / 2 ? tiles : kNumSMs / 2);
     if (es == 2) {
-      e = cudaFuncSetAttribute(lut_dense_tc_kernel<2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+      e = cudaFuncSetAttribute(lut_dense_tc_kernel<2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSmemMax));
       if (e != cudaSuccess) return static_cast<int>(e);
       e = launch_dependent(lut_dense_tc_kernel<2, true>, 2 * clusters, kThreads, smem, st, maps, p, 2);
     } else {
-      e = cudaFuncSetAttribute(lut_dense_tc_kernel<4, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+      e = cudaFuncSetAttribute(lut_dense_tc_kernel<4, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSmemMax));
       if (e != cudaSuccess) return static_cast<int>(e);
       e = launch_dependent(lut_dense_tc_kernel<4, true>, 2 * clusters, kThreads, smem, st, maps, p, 2);
     }
   } else if (seg) {
     auto kern = es == 2 ? lut_dense_tc_kernel<2, false, true> : lut_dense_tc_kernel<4, false, true>;
-    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSmemMax));
     if (e != cudaSuccess) return static_cast<int>(e);
     e = launch_dependent(kern, grid, kSegThreads, smem, st, maps, p);
   } else if (es == 2) {
-    e = cudaFuncSetAttribute(lut_dense_tc_kernel<2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    e = cudaFuncSetAttribute(lut_dense_tc_kernel<2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSmemMax));
     if (e != cudaSuccess) return static_cast<int>(e);
     e = launch_dependent(lut_dense_tc_kernel<2, false>, grid, kThreads, smem, st, maps, p);
   } else {
-    e = cudaFuncSetAttribute(lut_dense_tc_kernel<4, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    e = cudaFuncSetAttribute(lut_dense_tc_kernel<4, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSmemMax));
     if (e != cudaSuccess) return static_cast<int>(e);
     e = launch_dependent(lut_dense_tc_kernel<4, false>, grid, kThreads, smem, st, maps, p);
   }
@@ -1770,11 +1772,11 @@ int launch_stem_conv(const void* x, int x_dtype, const dimq_wq_weight* w, const 
   const int grid = p.m_tiles < kNumSMs ? p.m_tiles : kNumSMs;
   cudaError_t e;
   if (es == 2) {
-    e = cudaFuncSetAttribute(lut_stem_conv_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    e = cudaFuncSetAttribute(lut_stem_conv_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSmemMax));
     if (e != cudaSuccess) return static_cast<int>(e);
     e = launch_dependent(lut_stem_conv_kernel<2>, grid, kStemThreads, smem, st, maps, p);
   } else {
-    e = cudaFuncSetAttribute(lut_stem_conv_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    e = cudaFuncSetAttribute(lut_stem_conv_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSmemMax));
     if (e != cudaSuccess) return static_cast<int>(e);
     e = launch_dependent(lut_stem_conv_kernel<4>, grid, kStemThreads, smem, st, maps, p);
   }

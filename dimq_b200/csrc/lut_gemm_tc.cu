@@ -943,10 +943,13 @@ EncodeTiledFn get_encode_tiled() {
   return fn;
 }
 
+constexpr size_t kSmemMax = 227 * 1024;
+
 template <int BITS, bool PAIR, bool SPLIT>
 int launch_tc(const TmapSet& tmap, const TcParams& p, size_t smem, int grid, cudaStream_t st) {
   auto kern = linear_wq_tc_kernel<BITS, PAIR, SPLIT>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+  // the largest, not this call's: the attribute belongs to the process, and other threads launch other sizes
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSmemMax));
   if (e != cudaSuccess) return static_cast<int>(e);
   kern<<<grid, kThreads, smem, st>>>(tmap, p);
   return launch_status();
@@ -1082,7 +1085,6 @@ int finish_launch(const TmapSet& tmaps, TcParams& p, const dimq_wq_weight* w, co
   const size_t fixed = 1024 + kHeaderBytes + epi_bytes + static_cast<size_t>(kIdxPrefetch) * kNumDequantWarps * 32 * (w->bits == 8 ? 64 : 32) +
                        (p.rep ? static_cast<size_t>(kNumDequantGroups) * kRepWords * 4 : 0) +
                        table_bytes(w->bits, w->groups, pair, split);
-  const size_t kSmemMax = 227 * 1024;
   int x_stages = static_cast<int>((kSmemMax - fixed) / p.x_stage_bytes);
   if (x_stages > kXStages) x_stages = kXStages;
   if (x_stages < 3) return DIMQ_ERR_UNSUPPORTED;

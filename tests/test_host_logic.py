@@ -264,3 +264,15 @@ def test_default_build_has_no_diagnostics(lib):
         assert name not in blob, name
     sources = "".join(p.read_text() for p in (ROOT / "dimq_b200" / "csrc").iterdir())
     assert sources.count("getenv(") == 1 and 'getenv("DIMQ_B200_TC_EPI")' in sources
+
+
+def test_shared_memory_limits_are_constants():
+    """cudaFuncSetAttribute acts on the process: a limit set to one call's size can be lowered by another thread's call
+    before the launch.  Every kernel's limit is set to a constant of that kernel."""
+    sites = 0
+    for path in sorted((ROOT / "dimq_b200" / "csrc").glob("*.cu")):
+        for value in re.findall(r"cudaFuncAttributeMaxDynamicSharedMemorySize,\s*(.+?)\)+;", path.read_text()):
+            sites += 1
+            assert set(re.findall(r"[A-Za-z_]\w*", value)) - {"static_cast", "int", "size_t"} <= set(re.findall(r"\bk[A-Z]\w*", value)), \
+                (path.name, value)
+    assert sites >= 8
