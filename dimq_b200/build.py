@@ -72,7 +72,7 @@ def _build_host(objdir: Path) -> None:
          "-isystem", str(cuda / "include"), "-isystem", sysconfig.get_paths()["include"],
          "-c", str(CSRC / "host.cpp"), "-o", str(obj)],
         ["g++", "-shared", "-o", str(HOST), str(obj), "-L", str(PKG), "-l:libdimq_b200.so", "-L", str(root / "lib"),
-         "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python", "-Wl,-rpath,$ORIGIN"],
+         "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python", "-L", str(cuda / "lib64"), "-lcudart", "-Wl,-rpath,$ORIGIN"],
     ):
         res = subprocess.run(cmd, capture_output=True, text=True)
         if res.returncode != 0:

@@ -1005,12 +1005,35 @@ PyObject* py_set_ops(PyObject*, PyObject* dict) {
   Py_RETURN_NONE;
 }
 
+// Whether an event has completed.  Also while a graph is being captured, when a plain query would end the capture: the
+// event was recorded outside it, and in relaxed mode the question touches nothing that is captured.
+PyObject* py_event_done(PyObject*, PyObject* handle) {
+  HANDLE_TH_ERRORS
+  void* event = PyLong_AsVoidPtr(handle);
+  if (event == nullptr && PyErr_Occurred()) throw python_error();
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  cudaError_t e = cudaThreadExchangeStreamCaptureMode(&mode);
+  if (e == cudaSuccess) {
+    e = cudaEventQuery(static_cast<cudaEvent_t>(event));
+    const cudaError_t back = cudaThreadExchangeStreamCaptureMode(&mode);
+    if (e == cudaSuccess) e = back;
+  }
+  if (e == cudaErrorNotReady) {
+    (void)cudaGetLastError();
+    Py_RETURN_FALSE;
+  }
+  if (e != cudaSuccess) fail(std::string("event query failed: ") + cudaGetErrorString(e));
+  Py_RETURN_TRUE;
+  END_HANDLE_TH_ERRORS
+}
+
 #define FAST(name) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_##name)), METH_FASTCALL, nullptr}
 PyMethodDef kMethods[] = {FAST(linear_wq), FAST(linear_a4), FAST(conv2d_wq), FAST(conv2d_a4),
                           FAST(hard_quantize), FAST(fake_quantize_ste), FAST(unpack_bits), FAST(pack_bits), FAST(add_layer_norm),
                           FAST(max_pool_nhwc), FAST(images_to_nhwc), FAST(attention_qkv),
                           {"set_launch_count", py_set_launch_count, METH_O, nullptr},
                           {"set_ops", py_set_ops, METH_O, nullptr},
+                          {"event_done", py_event_done, METH_O, nullptr},
                           {nullptr, nullptr, 0, nullptr}};
 PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_host", nullptr, -1, kMethods, nullptr, nullptr, nullptr, nullptr};
 

@@ -20,7 +20,7 @@ from typing import Any, Mapping
 import torch
 import torch.nn as nn
 
-from . import ops
+from . import _lib, ops
 
 
 def _eager(x: torch.Tensor) -> bool:
@@ -28,6 +28,58 @@ def _eager(x: torch.Tensor) -> bool:
     registered operator."""
     return (type(x) is torch.Tensor and torch._C._len_torch_dispatch_stack() == 0 and not torch._C._is_tracing()
             and torch._C._functorch.peek_interpreter_stack() is None)
+
+
+class _Derived:
+    """A tensor derived from a module's buffer on the GPU, with what a later call needs to know before it may read it: that
+    the buffer still is what it was, and that the writing of the tensor - on the stream of the call that first needed it -
+    comes before.  Holds the buffer's storage, so that a new one cannot turn up at its address."""
+
+    __slots__ = ("source", "version", "extra", "value", "event", "written", "builder", "streams")
+
+    def __init__(self, source: torch.Tensor, extra, value: torch.Tensor) -> None:
+        self.source, self.version, self.extra, self.value = source.detach(), source._version, extra, value
+        with torch.cuda.device(value.device):
+            stream = torch.cuda.current_stream()
+            self.event = torch.cuda.Event()
+            self.event.record(stream)
+        self.written = False                     # known to be complete, for every stream
+        self.builder = stream.cuda_stream
+        self.streams = {stream.cuda_stream}      # those the allocator knows to read the value
+
+    def __reduce__(self):                        # copied and saved modules derive their own
+        return type(None), ()
+
+    def is_of(self, source: torch.Tensor, extra) -> bool:
+        return (self.source.data_ptr() == source.data_ptr() and self.version == source._version
+                and self.source.device == source.device and self.extra == extra)
+
+    def readable(self) -> bool:
+        """Make the current stream wait for the value where it has to.  False in a graph capture that began before the
+        value was written: a replay would not wait."""
+        device = self.source.get_device()
+        raw = torch._C._cuda_getCurrentRawStream(device)
+        if self.written and raw in self.streams:
+            return True
+        with torch.cuda.device(device):
+            if not self.written:
+                if _lib.host().event_done(self.event.cuda_event):
+                    self.written = True
+                elif torch.cuda.is_current_stream_capturing():
+                    return False
+                elif raw != self.builder:
+                    torch.cuda.current_stream().wait_event(self.event)
+            if raw not in self.streams:
+                self.value.record_stream(torch.cuda.current_stream())
+                self.streams.add(raw)
+        return True
+
+
+def _capturing(device: int) -> bool:
+    if device == torch.cuda.current_device():
+        return torch.cuda.is_current_stream_capturing()
+    with torch.cuda.device(device):
+        return torch.cuda.is_current_stream_capturing()
 
 
 def _pair(value) -> tuple[int, int]:
@@ -55,16 +107,33 @@ class _PackedBase(nn.Module):
             raise ValueError("the W4A4 mode needs 4-bit indices and one 16-entry codebook; "
                              "pass act_scale=None for weight-only layers")
 
+    def _derive(self, slot: str, source: torch.Tensor, build, extra=None) -> torch.Tensor:
+        """``build()`` from the buffer ``source``, kept in ``slot`` until the buffer is replaced, moved or written in place.
+        Not kept: what a graph capture builds (only a replay writes it), and what an inference tensor gives (its writes are
+        not counted)."""
+        kept = self.__dict__.get(slot)
+        counted = not source.is_inference()
+        if type(kept) is _Derived and counted and kept.is_of(source, extra) and kept.readable():
+            return kept.value
+        value = build()
+        if counted and not _capturing(source.get_device()):
+            self.__dict__[slot] = _Derived(source, extra, value)
+        return value
+
+    def _apply(self, fn, recurse=True):
+        super()._apply(fn, recurse)
+        for slot, name in (("_tiled", "packed_weight"), ("_khwc", "packed_weight"), ("_scaled_cb", "codebook")):
+            kept, source = self.__dict__.get(slot), getattr(self, name)
+            if type(kept) is _Derived and (source.is_inference() or not kept.is_of(source, kept.extra)):
+                self.__dict__[slot] = None           # a moved module leaves nothing behind
+        return self
+
     def _scaled_codebook(self) -> torch.Tensor:
         """``act_scale * codebook`` in fp32 (the weight operand of the tensor-core W4A4 form), built once
         and rebuilt when the codebook buffer or the scale changes."""
         cb = self.codebook
-        key = (cb.data_ptr(), cb._version, cb.device, self.act_scale)
-        if getattr(self, "_scaled_cb_key", None) != key:
-            self._scaled_cb = cb.detach().float().reshape(-1) * torch.tensor(self.act_scale, dtype=torch.float32,
-                                                                               device=cb.device)
-            self._scaled_cb_key = key
-        return self._scaled_cb
+        return self._derive("_scaled_cb", cb, lambda: cb.detach().float().reshape(-1) * torch.tensor(
+            self.act_scale, dtype=torch.float32, device=cb.device), self.act_scale)
 
     def _check_input(self, x: torch.Tensor) -> None:
         if not self.use_cuda_kernel:
@@ -88,7 +157,6 @@ class DIMQLinear(_PackedBase):
         # rows meets a weight that kernel takes (a second copy of the indices), rebuilt whenever the
         # packed_weight buffer is replaced, moved or written in place
         self._tiled = None
-        self._tiled_key = None
 
     def _prepacked(self, rows: int, x: torch.Tensor) -> torch.Tensor | None:
         if (rows > 16 or self.bits not in (2, 3, 4) or self.out_features % 16 != 0 or self.in_features % 128 != 0
@@ -97,11 +165,7 @@ class DIMQLinear(_PackedBase):
                 or self.out_features * self.in_features * self.bits < (1 << 24)):
             return None
         pw = self.packed_weight
-        key = (pw.data_ptr(), pw._version, pw.device)
-        if self._tiled is None or self._tiled_key != key:
-            self._tiled = ops.linear_prepack(pw, self.out_features, self.in_features, self.bits)
-            self._tiled_key = key
-        return self._tiled
+        return self._derive("_tiled", pw, lambda: ops.linear_prepack(pw, self.out_features, self.in_features, self.bits))
 
     def forward(self, x: torch.Tensor, residual: torch.Tensor | None = None) -> torch.Tensor:
         self._check_input(x)
@@ -164,17 +228,12 @@ class DIMQConv2d(_PackedBase):
         # indices re-ordered for the tensor-core conv: built on first use on the GPU and rebuilt
         # whenever the packed_weight buffer is replaced, moved or written in place
         self._khwc = None
-        self._khwc_key = None
 
     def _prepacked(self) -> torch.Tensor | None:
         if self.groups != 1 or self.weight_shape[1] % 64 != 0:
             return None
         pw = self._buffers["packed_weight"]
-        key = (pw.data_ptr(), pw._version, pw.device)
-        if self._khwc is None or self._khwc_key != key:
-            self._khwc = ops.conv_prepack(pw, self.weight_shape, self.bits)
-            self._khwc_key = key
-        return self._khwc
+        return self._derive("_khwc", pw, lambda: ops.conv_prepack(pw, self.weight_shape, self.bits))
 
     def forward(self, x: torch.Tensor, residual: torch.Tensor | None = None) -> torch.Tensor:
         self._check_input(x)
@@ -184,12 +243,13 @@ class DIMQConv2d(_PackedBase):
                                       self.stride, self.padding, self.dilation, self.groups, bits=self.bits,
                                       group_rows=self.group_rows, out_dtype=self.out_dtype, epilogue=self.epilogue,
                                       residual=residual, packed_khwc=self._prepacked())
-        khwc = self._prepacked()
+        tc = self.groups == 1 and self.weight_shape[1] % 64 == 0
         channels_last = x.dim() == 4 and x.is_contiguous(memory_format=torch.channels_last) and not x.is_contiguous()
-        if khwc is not None and channels_last and self.stride[0] == self.stride[1] and self.stride[0] in (1, 2):
+        if tc and channels_last and self.stride[0] == self.stride[1] and self.stride[0] in (1, 2):
             oh = (x.shape[2] + 2 * self.padding[0] - self.dilation[0] * (self.weight_shape[2] - 1) - 1) // self.stride[0] + 1
             ow = (x.shape[3] + 2 * self.padding[1] - self.dilation[1] * (self.weight_shape[3] - 1) - 1) // self.stride[1] + 1
             if x.shape[0] * oh * ow >= ops.A4_TC_MIN_ROWS:
+                khwc = self._prepacked()
                 # fp16 / bf16 codebooks are one exact term: the fp32-grade form (64 x 64 channels on 56^2, batch 64:
                 # 66 us, the bf16 pair 82; 512 on 7^2: 35 / 52); an fp32 codebook takes two there (94 / 82, 60 / 52)
                 if self.codebook.dtype != torch.float32:
@@ -209,8 +269,10 @@ class DIMQConv2d(_PackedBase):
         if residual is not None or self.epilogue is not None:
             raise RuntimeError("a fused epilogue or residual needs the weight-only mode, or channels_last input "
                                f"with at least {ops.A4_TC_MIN_ROWS} output pixels")
-        if khwc is not None and x.dim() == 4 and _eager(x):
-            # NCHW activations, or few pixels: the re-ordered indices are kept here, not re-derived per call
+        if tc and x.dim() == 4 and _eager(x):
+            # NCHW activations, or few pixels: the re-ordered indices are kept here, not re-derived per call.  A captured
+            # graph re-derives them in every replay: it follows packed_weight itself, as dimq_conv2d_lut does.
+            khwc = None if _capturing(x.get_device()) else self._prepacked()
             y = ops.dimq_conv2d_a4(x, self.packed_weight, self.codebook, self.act_scale, self.act_zero_point, self.bias,
                                    self.weight_shape, self.stride, self.padding, self.dilation, self.groups,
                                    packed_khwc=khwc)
