@@ -107,6 +107,12 @@ class _PackedBase(nn.Module):
             raise ValueError("the W4A4 mode needs 4-bit indices and one 16-entry codebook; "
                              "pass act_scale=None for weight-only layers")
 
+    def _tensor(self, name: str) -> torch.Tensor | None:
+        """``getattr(self, name)``, without the attribute protocol of ``nn.Module`` while it is the buffer it was registered as
+        (a codebook or bias may have become a parameter or a parametrised property since)."""
+        buffers = self._buffers
+        return buffers[name] if name in buffers else getattr(self, name)
+
     def _derive(self, slot: str, source: torch.Tensor, build, extra=None) -> torch.Tensor:
         """``build()`` from the buffer ``source``, kept in ``slot`` until the buffer is replaced, moved or written in place.
         Not kept: what a graph capture builds (only a replay writes it), and what an inference tensor gives (its writes are
@@ -138,7 +144,7 @@ class _PackedBase(nn.Module):
     def _check_input(self, x: torch.Tensor) -> None:
         if not self.use_cuda_kernel:
             raise RuntimeError("dimq_b200 has no Python fallback path (use_cuda_kernel=False is not supported)")
-        if not (x.is_cuda and self._buffers["packed_weight"].is_cuda):
+        if not (x.is_cuda and self._tensor("packed_weight").is_cuda):
             raise RuntimeError("dimq_b200 layers run on CUDA tensors only; move the module and its input to a B200")
 
 
@@ -170,10 +176,9 @@ class DIMQLinear(_PackedBase):
     def forward(self, x: torch.Tensor, residual: torch.Tensor | None = None) -> torch.Tensor:
         self._check_input(x)
         if self.act_scale is None:
-            buf = self._buffers
             tiled = self._prepacked(x.numel() // self.in_features, x)
-            return ops.dimq_linear_wq(x, buf["packed_weight"], buf["codebook"], buf["bias"], self.out_features,
-                                      self.in_features, bits=self.bits, group_rows=self.group_rows,
+            return ops.dimq_linear_wq(x, self._tensor("packed_weight"), self._tensor("codebook"), self._tensor("bias"),
+                                      self.out_features, self.in_features, bits=self.bits, group_rows=self.group_rows,
                                       out_dtype=self.out_dtype, epilogue=self.epilogue, residual=residual,
                                       packed_tiled=tiled)
         rows = x.numel() // self.in_features
@@ -232,15 +237,14 @@ class DIMQConv2d(_PackedBase):
     def _prepacked(self) -> torch.Tensor | None:
         if self.groups != 1 or self.weight_shape[1] % 64 != 0:
             return None
-        pw = self._buffers["packed_weight"]
+        pw = self._tensor("packed_weight")
         return self._derive("_khwc", pw, lambda: ops.conv_prepack(pw, self.weight_shape, self.bits))
 
     def forward(self, x: torch.Tensor, residual: torch.Tensor | None = None) -> torch.Tensor:
         self._check_input(x)
         if self.act_scale is None:
-            buf = self._buffers
-            return ops.dimq_conv2d_wq(x, buf["packed_weight"], buf["codebook"], buf["bias"], self.weight_shape,
-                                      self.stride, self.padding, self.dilation, self.groups, bits=self.bits,
+            return ops.dimq_conv2d_wq(x, self._tensor("packed_weight"), self._tensor("codebook"), self._tensor("bias"),
+                                      self.weight_shape, self.stride, self.padding, self.dilation, self.groups, bits=self.bits,
                                       group_rows=self.group_rows, out_dtype=self.out_dtype, epilogue=self.epilogue,
                                       residual=residual, packed_khwc=self._prepacked())
         tc = self.groups == 1 and self.weight_shape[1] % 64 == 0

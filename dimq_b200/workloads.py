@@ -135,7 +135,8 @@ class DIMQViT(nn.Module):
             self.q[name.replace(".", "__")] = DIMQLinear.from_export_layer(layer, out_dtype=out_dtype, epilogue=epi)
 
     def _t(self, key: str) -> torch.Tensor:
-        return self._buffers[key.replace(".", "__")]
+        name = key.replace(".", "__")
+        return self._buffers[name] if name in self._buffers else getattr(self, name)
 
     def _lin(self, name: str) -> DIMQLinear:
         return self.q._modules[name.replace(".", "__")]

@@ -111,6 +111,22 @@ def test_modules_are_copied_and_saved_without_it(gpu):
         assert twin._khwc is None and torch.equal(twin.packed_weight, layer.packed_weight)
 
 
+def test_buffers_may_have_become_parameters(monkeypatch):
+    seen = []
+    monkeypatch.setattr(ops, "dimq_linear_wq", lambda x, pw, cb, bias, *a, **k: seen.append((pw, cb, bias)))
+    monkeypatch.setattr(ops, "dimq_conv2d_wq", lambda x, pw, cb, bias, *a, **k: seen.append((pw, cb, bias)))
+    monkeypatch.setattr(DIMQLinear, "_check_input", lambda self, x: self._tensor("packed_weight"))
+    monkeypatch.setattr(DIMQConv2d, "_check_input", lambda self, x: self._tensor("packed_weight"))
+    monkeypatch.setattr(DIMQConv2d, "_prepacked", lambda self: None)
+    for layer in (DIMQLinear(torch.zeros(32, dtype=torch.uint8), torch.zeros(16), None, None, 8, 8, torch.zeros(8)),
+                  DIMQConv2d(torch.zeros(32, dtype=torch.uint8), torch.zeros(16), None, None, (8, 8, 1, 1), torch.zeros(8))):
+        layer.codebook = torch.nn.Parameter(torch.ones(16))              # trained on top of the export
+        layer.bias = torch.nn.Parameter(torch.ones(8))
+        layer.packed_weight = torch.nn.Parameter(layer.packed_weight, requires_grad=False)
+        layer(torch.zeros(1, 8, 1, 8))
+        assert seen[-1][0] is layer.packed_weight and seen[-1][1] is layer.codebook and seen[-1][2] is layer.bias
+
+
 # ---- on the GPU ----------------------------------------------------------------------------------
 
 def _a4_conv(seed=0):
