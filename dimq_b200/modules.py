@@ -23,11 +23,14 @@ import torch.nn as nn
 from . import _lib, ops
 
 
-def _eager(x: torch.Tensor) -> bool:
-    """Plain eager execution: no tracer, dispatch mode, tensor subclass or function transform that has to see the
-    registered operator."""
-    return (type(x) is torch.Tensor and torch._C._len_torch_dispatch_stack() == 0 and not torch._C._is_tracing()
-            and torch._C._functorch.peek_interpreter_stack() is None)
+def _eager(x: torch.Tensor, *params: torch.Tensor | None) -> bool:
+    """Plain eager execution: no tracer, dispatch or function mode, tensor subclass, function transform or gradient that
+    has to see the registered operator."""
+    if not (type(x) is torch.Tensor and torch._C._len_torch_dispatch_stack() == 0
+            and torch._C._len_torch_function_stack() == 0 and not torch._C._is_tracing()
+            and torch._C._functorch.peek_interpreter_stack() is None):
+        return False
+    return not torch.is_grad_enabled() or not (x.requires_grad or any(p is not None and p.requires_grad for p in params))
 
 
 class _Derived:
@@ -273,7 +276,7 @@ class DIMQConv2d(_PackedBase):
         if residual is not None or self.epilogue is not None:
             raise RuntimeError("a fused epilogue or residual needs the weight-only mode, or channels_last input "
                                f"with at least {ops.A4_TC_MIN_ROWS} output pixels")
-        if tc and x.dim() == 4 and _eager(x):
+        if tc and x.dim() == 4 and _eager(x, self.codebook, self.bias):
             # NCHW activations, or few pixels: the re-ordered indices are kept here, not re-derived per call.  A captured
             # graph re-derives them in every replay: it follows packed_weight itself, as dimq_conv2d_lut does.
             khwc = None if _capturing(x.get_device()) else self._prepacked()

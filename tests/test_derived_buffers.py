@@ -10,7 +10,7 @@ import types
 import pytest
 import torch
 
-from dimq_b200 import _lib, ops
+from dimq_b200 import _lib, modules, ops
 from dimq_b200.modules import DIMQConv2d, DIMQLinear
 
 
@@ -125,6 +125,29 @@ def test_buffers_may_have_become_parameters(monkeypatch):
         layer.packed_weight = torch.nn.Parameter(layer.packed_weight, requires_grad=False)
         layer(torch.zeros(1, 8, 1, 8))
         assert seen[-1][0] is layer.packed_weight and seen[-1][1] is layer.codebook and seen[-1][2] is layer.bias
+
+
+def test_the_registered_operator_is_bypassed_in_plain_eager_calls_only():
+    from torch.overrides import TorchFunctionMode
+    from torch.utils._python_dispatch import TorchDispatchMode
+
+    class Function(TorchFunctionMode):
+        def __torch_function__(self, func, types, args=(), kwargs=None):
+            return func(*args, **(kwargs or {}))
+
+    class Dispatch(TorchDispatchMode):
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            return func(*args, **(kwargs or {}))
+
+    x, p = torch.zeros(2), torch.nn.Parameter(torch.zeros(2))
+    assert modules._eager(x) and modules._eager(x, None, x)
+    assert not modules._eager(x, p) and not modules._eager(x.clone().requires_grad_())
+    with torch.no_grad():
+        assert modules._eager(x, p)
+    for mode in (Function(), Dispatch()):
+        with mode:
+            seen = modules._eager(x)
+        assert not seen
 
 
 # ---- on the GPU ----------------------------------------------------------------------------------
