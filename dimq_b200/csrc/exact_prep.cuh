@@ -23,12 +23,13 @@ namespace {
 constexpr int kPrepThreads = 256;
 constexpr int kExpandTable = 129 * 16;   // words: a block of 256 units covers at most 128 rows (K >= 64), 129 groups
 
-// exponent e with max_abs * 2^e in [2^14, 2^15), kept where 2^-e is a normal number and the product of a row's
-// and a column's 2^-e cannot underflow (max_abs below 2^-49 = 1.8e-15 is scaled by 2^63 only)
+// exponent e with max_abs * 2^e in [2^14, 2^15), kept where 2^-e is a normal number: max_abs below 2^-112 is scaled by 2^126,
+// which takes the smallest subnormal to 2^-23, still a multiple of fp16's smallest.  The product of a row's and a column's
+// 2^-e may leave fp32; the epilogue multiplies by one after the other.
 __device__ __forceinline__ int fp16_scale_exponent(float max_abs) {
   if (!(max_abs > 0.0f)) return 0;
   const int e = 14 - ilogbf(max_abs);
-  return e > 63 ? 63 : e;
+  return e > 126 ? 126 : e;
 }
 
 __device__ __forceinline__ bool finite_f32(float v) { return fabsf(v) <= 3.402823466e38f; }
@@ -266,7 +267,7 @@ exact_prep_kernel(const PrepParams p) {
     for (int i = 0; i < 4; ++i) mx = fmaxf(mx, __uint_as_float(smem[half_id * 4 + i]));
     const int ex = fp16_scale_exponent(mx);
     if (t == 0) p.row_scale[row] = scalbnf(1.0f, -ex);
-    const float up = scalbnf(1.0f, ex);      // -113 <= ex <= 63: a normal number
+    const float up = scalbnf(1.0f, ex);      // -113 <= ex <= 126: a normal number
     for (int64_t k = t * 8; k < p.C; k += 1024) {
       float f[8];
       load8(xr, DIMQ_BF16, k, f);
@@ -299,7 +300,7 @@ exact_prep_kernel(const PrepParams p) {
     for (int i = 0; i < 4; ++i) mx = fmaxf(mx, __uint_as_float(smem[half_id * 4 + i]));
     const int ex = fp16_scale_exponent(mx);
     if (t == 0) p.row_scale[row] = scalbnf(1.0f, -ex);
-    const float up = scalbnf(1.0f, ex);      // -113 <= ex <= 63: a normal number
+    const float up = scalbnf(1.0f, ex);      // -113 <= ex <= 126: a normal number
     __half* hi = p.xo + row * 2 * p.C;
     for (int64_t k = t * 4; k < p.C; k += 512) {
       const float4 v = __ldg(reinterpret_cast<const float4*>(xr + k));

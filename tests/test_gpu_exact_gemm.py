@@ -310,3 +310,31 @@ def test_operands_on_another_device_are_refused(ops):
             call()
             torch.cuda.synchronize()
             raise AssertionError(f"call {i} was accepted")
+
+
+@pytest.mark.parametrize("act,book,bound", [(torch.float32, torch.float32, 4 * REL), (torch.float32, torch.float16, 4 * REL),
+                                            (torch.float32, torch.bfloat16, 4 * REL), (torch.bfloat16, torch.float16, 1.2e-5)])
+def test_linear_rows_of_every_size(ops, act, book, bound):
+    # rows from the subnormals to 1e33 (both forms scale a row by a power of two into fp16's range), each against its own norm
+    m, k, n = 1100, 768, 64
+    packed, books, w = _weight(ops, n, k, 4, book, seed=17)
+    books, w = books * 64, w * 64                                # about 1
+    size = 10.0 ** torch.linspace(-36.5, 33, m, device="cuda", dtype=torch.float64).view(-1, 1)
+    x = (torch.randn(m, k, device="cuda", dtype=torch.float64) * size).to(act)
+    y = ops.dimq_linear_wq(x, packed, books, None, n, k, bits=4)
+    assert y.dtype == torch.float32 and ops.last_device_status() == 0
+    err = (y.double() - x.double() @ w.t()).norm(dim=1) / (x.double().norm(dim=1) * w.norm() / k ** 0.5)
+    assert float(err.max()) < bound
+
+
+@pytest.mark.parametrize("xs,ws", [(1e-42, 1e12), (1e-30, 1e30), (1e30, 1e-30), (1e12, 1e-42), (1e-20, 1e-16), (1e20, 1e14), (1e-36, 1e36)])
+def test_linear_f32_scales_that_meet(ops, xs, ws):
+    # rows and codewords of opposite extremes: the scales are undone one after the other
+    m, k, n = 130, 768, 64
+    packed, books, w = _weight(ops, n, k, 4, torch.float32, seed=18)
+    books = (books.double() * 50 * ws).float()
+    idx = torch.stack([packed.view(n, -1) & 15, packed.view(n, -1) >> 4], 2).view(n, k).long()
+    w = books.double().reshape(-1)[idx]
+    x = (torch.randn(m, k, device="cuda", dtype=torch.float64) * xs).float()
+    y = ops.dimq_linear_wq(x, packed, books, None, n, k, bits=4)
+    assert _rel(y, x.double() @ w.t()) < 4 * REL
