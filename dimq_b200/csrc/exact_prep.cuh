@@ -4,11 +4,14 @@
 //
 // Why fp16 terms.  The tensor cores multiply 16-bit operands exactly and add in fp32.
 //   * W4A4: the activation codes minus their zero point are integers in [-15, 15], exact in fp16.
-//   * fp32 activations: x * 2^e = hi + lo with fp16 hi and lo; e is chosen per row so that the row's largest finite
-//     magnitude lies in [2^14, 2^15).  hi carries 11 bits, lo the next 11 and the sign of lo one more: 2^-24 of the
-//     element, as fp32 itself, down to 2^-16 of the row's largest element and 2^-40 of that element below it.
-//   * codewords: fp16 ones are their own term.  Others are scaled per group in the same way; bf16 ones (8 bits) are
-//     then one term, fp32 ones hi + lo.
+//   * fp32 activations: x * 2^e = hi + lo * 2^-12 with fp16 hi and lo; e is chosen per row so that the row's largest
+//     finite magnitude lies in [2^14, 2^15).  hi carries 11 bits, lo the next 11 and the sign of lo one more: about 2^-23
+//     of the element.  lo is stored 2^12 times as large, so that it has its bits left where hi comes to fp16's end: an
+//     element keeps 2^-23 down to 2^-28 of the row's largest and is known to 2^-51 of that below.  (With lo as it is,
+//     the range ended at 2^-18: rows of order 1 with one element of 1e8 that meets a zero codeword came out at 6.8e-5.)
+//     The sums of the products with a lo are taken out of the accumulators apart and multiplied by 2^-12.
+//   * codewords: fp16 ones are their own term.  Others are scaled per group in the same way; bf16 ones (8 bits, exact down
+//     to 2^-30 of the group's largest) are then one term, fp32 ones hi + lo.
 // Three products (x_hi w_hi, x_hi w_lo, x_lo w_hi) carry an fp32 product to about 2^-23; a bf16 split would need six.
 // Non-finite values: an infinite or NaN activation has hi = 0 and keeps its value in lo, which meets w_hi only;
 // a codeword of a two-term weight keeps it in w_lo, which meets x_hi only - so no infinity is multiplied by an
@@ -21,6 +24,7 @@ namespace dimq {
 namespace {
 
 constexpr int kPrepThreads = 256;
+constexpr float kLoScale = 4096.0f;      // lo terms are stored this many times as large (the SEG epilogue divides)
 constexpr int kExpandTable = 129 * 16;   // words: a block of 256 units covers at most 128 rows (K >= 64), 129 groups
 
 // exponent e with max_abs * 2^e in [2^14, 2^15), kept where 2^-e is a normal number: max_abs below 2^-112 is scaled by 2^126,
@@ -36,7 +40,7 @@ __device__ __forceinline__ bool finite_f32(float v) { return fabsf(v) <= 3.40282
 
 // lut_expand_kernel's work for one block of 256 units (unit = 32 consecutive indices of one row).
 //   fmt 0: fp16 codewords, 1: bf16 (terms == 2: and the bf16 remainder c - bf16(c)), 2: fp16 of c * 2^e with e per
-//   group (terms == 2: and the fp16 remainder); col_scale[row] = 2^-e.
+//   group (terms == 2: and the fp16 remainder times kLoScale); col_scale[row] = 2^-e.
 template <int BITS>
 __device__ __forceinline__ void expand_block(uint32_t* tbl, int64_t block, const uint8_t* __restrict__ packed,
                                              const void* __restrict__ codebooks, int cb_dtype, int entries,
@@ -74,7 +78,7 @@ __device__ __forceinline__ void expand_block(uint32_t* tbl, int64_t block, const
         const float cs = scalbnf(c, ex);
         __half h = __float2half_rn(cs), l = __float2half_rn(0.0f);
         if (terms == 2) {
-          if (finite_f32(c)) l = __float2half_rn(cs - __half2float(h));
+          if (finite_f32(c)) l = __float2half_rn((cs - __half2float(h)) * kLoScale);
           else { l = h; h = __float2half_rn(0.0f); }
         }
         v = __half_as_ushort(h) | (static_cast<uint32_t>(__half_as_ushort(l)) << 16);
@@ -311,7 +315,7 @@ exact_prep_kernel(const PrepParams p) {
         const float s = a[i] * up;
         if (finite_f32(a[i])) {
           h[i] = __float2half_rn(s);
-          l[i] = __float2half_rn(s - __half2float(h[i]));
+          l[i] = __float2half_rn((s - __half2float(h[i])) * kLoScale);
         } else {
           h[i] = __float2half_rn(0.0f);
           l[i] = __float2half_rn(a[i]);

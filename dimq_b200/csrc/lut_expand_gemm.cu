@@ -86,6 +86,9 @@ struct DenseParams {
   const float* row_scale;
   const float* col_scale;
   float out_scale;
+  // SEG form: the k block (over all passes) where products with lo terms, which are kLoScale times too large, meet those
+  // without - no segment spans it - and whether the lo side comes first
+  int seg_cut, lo_first;
   void* y_nchw;             // convolution with an NCHW output: plain stores instead of the TMA store
 #ifdef DIMQ_B200_DIAG
   int diag;
@@ -371,6 +374,11 @@ constexpr int kSegBlocks = 4;
 constexpr int kSegAccStages = 4, kSegAccCols = 128;   // four buffers of 128 columns: the MMA warp runs ahead of a tile's final stores
 // three producers (a narrow tile's copies need no more) leave the epilogue warps 168 registers for the sums
 constexpr int kSegThreads = (1 + 3 + kEpiWarps) * 32;
+// end of the segment that starts at k block seg0
+__device__ __forceinline__ int seg_end_of(int seg0, int total_kb, const DenseParams& p) {
+  const int most = seg0 < p.seg_cut && p.seg_cut < total_kb ? p.seg_cut : total_kb;
+  return seg0 + kSegBlocks < most ? seg0 + kSegBlocks : most;
+}
 template <int ES, bool PAIR, bool SEG = false>
 __global__ void __launch_bounds__(SEG ? kSegThreads : kThreads, 1)
 lut_dense_tc_kernel(const __grid_constant__ DenseMaps maps, const DenseParams p) {
@@ -572,7 +580,7 @@ lut_dense_tc_kernel(const __grid_constant__ DenseMaps maps, const DenseParams p)
     if (p.b_res && ok && !__all_sync(0xFFFFFFFFu, mbar_wait(smem_u32(&hdr->b_res_full), 0u, abort_flag, 0x1A00u))) ok = false;
     STEM_ACC_DECL;
     STEM_CLK(t_all);
-    const int seg_kb = SEG ? kSegBlocks : total_kb;   // a multiple of kps, or the whole tile: no stage holds two segments
+    // segments start at multiples of kps, so that no stage holds two (seg_cut is odd with kps = 1 only)
     int seg0 = 0;                                     // first k block of the current segment
     for (int t = tile0; t < num_tiles && ok;) {
       STEM_CLK(t_w1);
@@ -580,7 +588,7 @@ lut_dense_tc_kernel(const __grid_constant__ DenseMaps maps, const DenseParams p)
       STEM_ACC(1, t_w1);
       tc_fence_after();
       const uint32_t d_tmem = tmem_base + as * kBufCols;
-      const int seg_end = SEG && seg0 + seg_kb < total_kb ? seg0 + seg_kb : total_kb;
+      const int seg_end = SEG ? seg_end_of(seg0, total_kb, p) : total_kb;
       const int seg_first = SEG ? seg0 : 0;
       for (int g = seg_first; g < seg_end; g += p.kps) {
         const int nblk = total_kb - g < p.kps ? total_kb - g : p.kps;   // 64-k blocks in this stage
@@ -677,7 +685,7 @@ lut_dense_tc_kernel(const __grid_constant__ DenseMaps maps, const DenseParams p)
         float sum[2][32];
         const float rs = p.row_scale == nullptr ? p.out_scale
                          : row_off >= 0 ? p.row_scale[static_cast<int64_t>(m_blk) * kBM + quarter * 32 + lane] : 0.0f;
-        for (int seg0 = 0; seg0 < total_kb; seg0 += kSegBlocks) {
+        for (int seg0 = 0; seg0 < total_kb; seg0 = seg_end_of(seg0, total_kb, p)) {
           if (!__all_sync(0xFFFFFFFFu, mbar_wait(smem_u32(&hdr->d_full[as]), aph, abort_flag, 0x1500u | as))) { ok = false; break; }
           tc_fence_after();
           const uint32_t d_tmem = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + as * kBufCols;
@@ -690,12 +698,16 @@ lut_dense_tc_kernel(const __grid_constant__ DenseMaps maps, const DenseParams p)
           if (lane == 0) mbar_arrive(smem_u32(&hdr->d_empty[as]));
           __syncwarp();
           if (++as == kAccBufs) { as = 0; aph ^= 1u; }
+          const float unit = (seg0 < p.seg_cut) == (p.lo_first != 0) ? 1.0f / kLoScale : 1.0f;
           if (seg0 == 0) {
 #pragma unroll
-            for (int j = 0; j < 32; ++j) { sum[0][j] = __uint_as_float(r0[j]); sum[1][j] = __uint_as_float(r1[j]); }
+            for (int j = 0; j < 32; ++j) { sum[0][j] = __uint_as_float(r0[j]) * unit; sum[1][j] = __uint_as_float(r1[j]) * unit; }
           } else {
 #pragma unroll
-            for (int j = 0; j < 32; ++j) { sum[0][j] += __uint_as_float(r0[j]); sum[1][j] += __uint_as_float(r1[j]); }
+            for (int j = 0; j < 32; ++j) {
+              sum[0][j] = fmaf(__uint_as_float(r0[j]), unit, sum[0][j]);
+              sum[1][j] = fmaf(__uint_as_float(r1[j]), unit, sum[1][j]);
+            }
           }
         }
         if (!ok) break;
@@ -953,6 +965,7 @@ int launch_dense(DenseMaps& maps, DenseParams& p, const void* scratch, int64_t K
   // A convolution whose expanded weight is one tile wide and fits beside the activation stages keeps it in
   // shared memory: no per-stage weight copies.
   p.kps = (!pair && p.bn * (p.stack + 1) <= 128) ? 2 : 1;
+  if (seg && p.seg_cut < p.k_blocks * p.passes && p.seg_cut % 2 != 0) p.kps = 1;
 #ifdef DIMQ_B200_DIAG
   if (g_dense_diag & 65536) p.kps = 1;   // timing experiments: one block per stage
 #endif
@@ -1940,12 +1953,16 @@ int exact_prepare(PrepParams& q, DenseParams& p, const dimq_wq_weight* w, const 
   // products of terms, the small ones first
   p.b_terms = terms;
   p.passes = 0;
+  const int k_blocks = static_cast<int>(K / kBK);
   auto pass = [&p](int a, int b) { p.a_term[p.passes] = a; p.b_term[p.passes++] = b; };
   if (a4) {       // in column order: a convolution may keep the weight resident, pass after pass
     for (int b = 0; b < terms; ++b) pass(0, b);
+    p.seg_cut = k_blocks;
   } else {
     pass(1, 0);
     if (terms == 2) pass(0, 1);
+    p.seg_cut = k_blocks * p.passes;
+    p.lo_first = 1;
     pass(0, 0);
   }
   return rc;

@@ -226,7 +226,9 @@ DIMQ_API int dimq_conv2d_wq_static(const void* x, int x_dtype, const dimq_wq_wei
  *    applies bias / epilogue / residual.
  *  - fp32 activations and output, more than 8 rows, 2- to 4-bit indices, K a multiple of 64: activations and
  *    codewords are split into fp16 terms (2*M*K + up to 2*N*K halves) and multiplied on the tensor cores at fp32
- *    grade; with too small a workspace the fp32 SIMT kernel runs instead.
+ *    grade: each product to about 2^-23 while the activation is not below 2^-28 of the largest in its row, and the
+ *    codeword not below 2^-28 (bf16: 2^-30) of the largest in its group; what is smaller is known to 2^-51 (bf16: 2^-38)
+ *    of that largest.  With too small a workspace the fp32 SIMT kernel runs instead.
  * dimq_linear_wq_workspace_bytes reports the bytes of the regime that applies and 0 otherwise (then
  * dimq_linear_wq_ws is dimq_linear_wq with DIMQ_ALGO_AUTO and the workspace is not touched).  The
  * workspace must be 16-byte aligned; its contents after the call are unspecified.  The reference has no

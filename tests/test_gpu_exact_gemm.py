@@ -338,3 +338,41 @@ def test_linear_f32_scales_that_meet(ops, xs, ws):
     x = (torch.randn(m, k, device="cuda", dtype=torch.float64) * xs).float()
     y = ops.dimq_linear_wq(x, packed, books, None, n, k, bits=4)
     assert _rel(y, x.double() @ w.t()) < 4 * REL
+
+
+@pytest.mark.parametrize("m,k,n", [(40, 64, 64), (300, 192, 132), (197, 768, 1000), (130, 1088, 64)])
+@pytest.mark.parametrize("book", [torch.float16, torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("outlier", [1.0, 1e5, 1e8])
+def test_linear_f32_rows_with_an_outlier(ops, m, k, n, book, outlier):
+    # one activation per row far above the others, which meets zero codewords; K of odd and even numbers of 64
+    packed, books, w = _weight(ops, n, k, 4, book, seed=m)
+    idx = torch.stack([packed.view(n, -1) & 15, packed.view(n, -1) >> 4], 2).view(n, k)
+    idx[:, 5] = 3
+    books = books.reshape(-1).clone()
+    books[3] = 0
+    packed, w = ops.pack_bits(idx, 4), books.double()[idx.long()]
+    x = torch.randn(m, k, device="cuda")
+    x[:, 5] = outlier * x[:, 5].sign()
+    y = ops.dimq_linear_wq(x, packed, books, None, n, k, bits=4)
+    assert ops.last_device_status() == 0 and _rel(y, x.double() @ w.t()) < REL
+
+
+@pytest.mark.parametrize("k", [64, 192, 768])
+@pytest.mark.parametrize("a4", [False, True])
+def test_fp32_codebooks_with_an_outlier(ops, k, a4):
+    # one codeword far above the others, which meets zero activations
+    m, n = 150, 64
+    packed, books, w = _weight(ops, n, k, 4, torch.float32, seed=k)
+    idx = torch.stack([packed.view(n, -1) & 15, packed.view(n, -1) >> 4], 2).view(n, k)
+    idx[idx == 3] = 4
+    idx[:, 7] = 3
+    books = books.reshape(-1).clone()
+    books[3] = 1e6                            # 2^25 times the others
+    packed, w = ops.pack_bits(idx, 4), books.double()[idx.long()]
+    x = torch.randn(m, k, device="cuda")
+    x[:, 7] = 0
+    if a4:
+        y, want = ops.dimq_linear_lut(x, packed, books, 0.23, 7, None, n, k), _codes(x, 0.23, 7) @ w.t()
+    else:
+        y, want = ops.dimq_linear_wq(x, packed, books, None, n, k, bits=4), x.double() @ w.t()
+    assert ops.last_device_status() == 0 and _rel(y, want) < REL
