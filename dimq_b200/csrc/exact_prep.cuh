@@ -13,9 +13,13 @@
 //   * codewords: fp16 ones are their own term.  Others are scaled per group in the same way; bf16 ones (8 bits, exact down
 //     to 2^-30 of the group's largest) are then one term, fp32 ones hi + lo.
 // Three products (x_hi w_hi, x_hi w_lo, x_lo w_hi) carry an fp32 product to about 2^-23; a bf16 split would need six.
-// Non-finite values: an infinite or NaN activation has hi = 0 and keeps its value in lo, which meets w_hi only;
-// a codeword of a two-term weight keeps it in w_lo, which meets x_hi only - so no infinity is multiplied by an
-// artificial zero, and x = 0 against an infinite codeword is NaN as in fp32.
+// Non-finite values of the fp32 form: an infinite activation has hi = 0 and keeps its value in lo, which meets w_hi only; a
+// codeword that would underflow to w_hi = 0 takes fp16's smallest instead (w_lo carries the difference), so the product has
+// the sign of both.  A row with a NaN has the scale NaN.  An infinite or NaN codeword is a NaN here: no split of it is right,
+// as x_lo may be zero, or of the other sign, where x is not.  Where an output comes out as a NaN and its row has none, the
+// epilogue computes it again in plain fp32.
+// W4A4 codes are one exact term: a zero code against an infinite codeword is NaN as in fp32, with one term or two (there
+// w_lo keeps the value and w_hi = 0).
 #pragma once
 
 #include "common.cuh"
@@ -41,11 +45,12 @@ __device__ __forceinline__ bool finite_f32(float v) { return fabsf(v) <= 3.40282
 // lut_expand_kernel's work for one block of 256 units (unit = 32 consecutive indices of one row).
 //   fmt 0: fp16 codewords, 1: bf16 (terms == 2: and the bf16 remainder c - bf16(c)), 2: fp16 of c * 2^e with e per
 //   group (terms == 2: and the fp16 remainder times kLoScale); col_scale[row] = 2^-e.
+//   split_x: for activations in two terms, see above (fmt 0 and 2).
 template <int BITS>
 __device__ __forceinline__ void expand_block(uint32_t* tbl, int64_t block, const uint8_t* __restrict__ packed,
                                              const void* __restrict__ codebooks, int cb_dtype, int entries,
                                              int64_t group_rows, int64_t rows, int64_t K, int fmt, int terms,
-                                             uint16_t* __restrict__ out, float* __restrict__ col_scale) {
+                                             uint16_t* __restrict__ out, float* __restrict__ col_scale, bool split_x) {
   const int64_t units_per_row = K / 32;
   const int64_t total = rows * units_per_row;
   const int64_t u = block * 256 + threadIdx.x;
@@ -66,7 +71,7 @@ __device__ __forceinline__ void expand_block(uint32_t* tbl, int64_t block, const
       const float c = i < n_slots && e < entries ? load_as_float(codebooks, cb_dtype, g * entries + e) : 0.0f;
       uint32_t v;
       if (fmt == 0) {
-        v = __half_as_ushort(__float2half_rn(c));
+        v = split_x && !finite_f32(c) ? 0x7FFFu : __half_as_ushort(__float2half_rn(c));
       } else if (fmt == 1) {
         const __nv_bfloat16 h = __float2bfloat16_rn(c);
         v = __bfloat16_as_ushort(h) | (static_cast<uint32_t>(__bfloat16_as_ushort(__float2bfloat16_rn(c - __bfloat162float(h)))) << 16);
@@ -77,9 +82,14 @@ __device__ __forceinline__ void expand_block(uint32_t* tbl, int64_t block, const
         const int ex = fp16_scale_exponent(mx);
         const float cs = scalbnf(c, ex);
         __half h = __float2half_rn(cs), l = __float2half_rn(0.0f);
+        if (split_x && !finite_f32(c)) {
+          h = __ushort_as_half(0x7FFFu);
+        } else if (split_x && c != 0.0f && fabsf(cs) <= 2.98023224e-8f) {   // 2^-25
+          h = __float2half_rn(copysignf(5.96046448e-8f, c));
+        }
         if (terms == 2) {
           if (finite_f32(c)) l = __float2half_rn((cs - __half2float(h)) * kLoScale);
-          else { l = h; h = __float2half_rn(0.0f); }
+          else if (!split_x) { l = h; h = __float2half_rn(0.0f); }
         }
         v = __half_as_ushort(h) | (static_cast<uint32_t>(__half_as_ushort(l)) << 16);
         // the scale of every row of this group that starts in this block's units (first unit of the row)
@@ -172,7 +182,7 @@ struct PrepParams {
   const void* codebooks;
   int cb_dtype, entries;
   int64_t group_rows, rows, K;
-  int fmt, terms;
+  int fmt, terms, split_x;   // see expand_block
   uint16_t* wo;
   float* col_scale;
 };
@@ -210,7 +220,7 @@ exact_prep_kernel(const PrepParams p) {
   const int64_t blk = blockIdx.x;
   if (blk >= p.x_blocks) {
     expand_block<BITS>(smem, blk - p.x_blocks, p.packed, p.codebooks, p.cb_dtype, p.entries, p.group_rows, p.rows, p.K,
-                       p.fmt, p.terms, p.wo, p.col_scale);
+                       p.fmt, p.terms, p.wo, p.col_scale, p.split_x != 0);
     return;
   }
   if (p.mode == kPrepCodes) {
@@ -288,22 +298,30 @@ exact_prep_kernel(const PrepParams p) {
     const bool live = row < p.n;
     const float* xr = static_cast<const float*>(p.x) + (live ? row : 0) * p.C;
     float mx = 0.0f;
+    bool nan = false;
     if (live)
       for (int64_t k = t * 4; k < p.C; k += 512) {      // C % 64 == 0
         const float4 v = __ldg(reinterpret_cast<const float4*>(xr + k));
         const float a[4] = {fabsf(v.x), fabsf(v.y), fabsf(v.z), fabsf(v.w)};
 #pragma unroll
-        for (int i = 0; i < 4; ++i) mx = fmaxf(mx, finite_f32(a[i]) ? a[i] : 0.0f);
+        for (int i = 0; i < 4; ++i) {
+          mx = fmaxf(mx, finite_f32(a[i]) ? a[i] : 0.0f);
+          nan = nan || a[i] != a[i];
+        }
       }
 #pragma unroll
     for (int d = 16; d > 0; d >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xFFFFFFFFu, mx, d));
-    if ((tid & 31) == 0) smem[tid >> 5] = __float_as_uint(mx);
+    nan = __any_sync(0xFFFFFFFFu, nan);
+    if ((tid & 31) == 0) { smem[tid >> 5] = __float_as_uint(mx); smem[8 + (tid >> 5)] = nan ? 1u : 0u; }
     __syncthreads();
     if (!live) return;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) mx = fmaxf(mx, __uint_as_float(smem[half_id * 4 + i]));
+    for (int i = 0; i < 4; ++i) {
+      mx = fmaxf(mx, __uint_as_float(smem[half_id * 4 + i]));
+      nan = nan || smem[8 + half_id * 4 + i] != 0u;
+    }
     const int ex = fp16_scale_exponent(mx);
-    if (t == 0) p.row_scale[row] = scalbnf(1.0f, -ex);
+    if (t == 0) p.row_scale[row] = nan ? __int_as_float(0x7FFFFFFF) : scalbnf(1.0f, -ex);
     const float up = scalbnf(1.0f, ex);      // -113 <= ex <= 126: a normal number
     __half* hi = p.xo + row * 2 * p.C;
     for (int64_t k = t * 4; k < p.C; k += 512) {

@@ -89,6 +89,12 @@ struct DenseParams {
   // SEG form: the k block (over all passes) where products with lo terms, which are kLoScale times too large, meet those
   // without - no segment spans it - and whether the lo side comes first
   int seg_cut, lo_first;
+  // fp32 activations, kSegSplit (else null): what an output that came out as a NaN is computed from again
+  const float* x32;
+  const uint8_t* packed;
+  const void* codebooks;
+  int bits, cb_dtype, entries;
+  int64_t K, group_rows;
   void* y_nchw;             // convolution with an NCHW output: plain stores instead of the TMA store
 #ifdef DIMQ_B200_DIAG
   int diag;
@@ -127,6 +133,7 @@ struct DenseHeader {
   uint64_t b_res_full;              // convolution with a resident weight: all its tiles have landed
   uint32_t tmem_base;
   volatile uint32_t abort_flag;
+  volatile int redo[kEpiWarps];     // kSegSplit: 1 + 2 * tile + chunk from where on an epilogue warp has stored nothing
 };
 static_assert(sizeof(DenseHeader) <= kHeaderBytes, "header");
 
@@ -374,14 +381,39 @@ constexpr int kSegBlocks = 4;
 constexpr int kSegAccStages = 4, kSegAccCols = 128;   // four buffers of 128 columns: the MMA warp runs ahead of a tile's final stores
 // three producers (a narrow tile's copies need no more) leave the epilogue warps 168 registers for the sums
 constexpr int kSegThreads = (1 + 3 + kEpiWarps) * 32;
+// 32 outputs of one row (per lane) by fp32 FMAs: a lane looks up the codeword of its column, the warp shares them.
+__device__ __forceinline__ void plain_chunk(float (&v)[32], const DenseParams& p, int64_t row, int64_t n_first, int lane) {
+  const int64_t n = n_first + lane;
+#pragma unroll
+  for (int j = 0; j < 32; ++j) v[j] = 0.0f;
+#pragma unroll 1
+  for (int64_t k = 0; k < p.K; ++k) {
+    const float xv = row < p.M ? p.x32[row * p.K + k] : 0.0f;
+    float c = 0.0f;
+    if (n < p.N) {
+      const int64_t bit = (n * p.K + k) * p.bits;
+      const int sh = static_cast<int>(bit & 7);
+      uint32_t idx = p.packed[bit >> 3] >> sh;
+      if (sh + p.bits > 8) idx |= static_cast<uint32_t>(p.packed[(bit >> 3) + 1]) << (8 - sh);
+      idx &= (1u << p.bits) - 1u;
+      if (idx < static_cast<uint32_t>(p.entries)) c = load_as_float(p.codebooks, p.cb_dtype, n / p.group_rows * p.entries + idx);
+    }
+#pragma unroll
+    for (int j = 0; j < 32; ++j) v[j] = fmaf(xv, __shfl_sync(0xFFFFFFFFu, c, j), v[j]);
+  }
+}
+
 // end of the segment that starts at k block seg0
 __device__ __forceinline__ int seg_end_of(int seg0, int total_kb, const DenseParams& p) {
   const int most = seg0 < p.seg_cut && p.seg_cut < total_kb ? p.seg_cut : total_kb;
   return seg0 + kSegBlocks < most ? seg0 + kSegBlocks : most;
 }
-template <int ES, bool PAIR, bool SEG = false>
-__global__ void __launch_bounds__(SEG ? kSegThreads : kThreads, 1)
+// FORM: what the SEG form multiplies (kDense: not that form)
+enum DenseForm { kDense = 0, kSegCodes = 1, kSegSplit = 2 };   // W4A4 codes; fp32 activations in two terms
+template <int ES, bool PAIR, int FORM = kDense>
+__global__ void __launch_bounds__(FORM != kDense ? kSegThreads : kThreads, 1)
 lut_dense_tc_kernel(const __grid_constant__ DenseMaps maps, const DenseParams p) {
+  constexpr bool SEG = FORM != kDense;
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   // [stages: A 16 KB | B bn*128 B (all 1024-aligned)] [header] [bias slices] [staging tiles]
   // rounded up to 1024 bytes in the shared window; plain pointer arithmetic on the array keeps the
@@ -646,6 +678,10 @@ lut_dense_tc_kernel(const __grid_constant__ DenseMaps maps, const DenseParams p)
     const int n_chunks = p.bn / 32;
     uint32_t as = 0, aph = 0;
     bool ok = true;
+    if (FORM == kSegSplit) {
+      if (lane == 0) hdr->redo[ew] = 0;
+      __syncwarp();
+    }
     if (SEG || p.row_scale != nullptr) asm volatile("griddepcontrol.wait;" ::: "memory");   // the scales come from the kernel before
     STEM_ACC_DECL;
     STEM_CLK(t_all);
@@ -738,7 +774,23 @@ lut_dense_tc_kernel(const __grid_constant__ DenseMaps maps, const DenseParams p)
                 }
               }
             }
-            store_chunk<ES, ES == 4>(v, my_bias, my_out, maps, p, n_first, row_off, c1, c2, c3, lane);
+            if constexpr (FORM == kSegSplit) {
+              bool later = hdr->redo[ew] != 0;
+              float probe = 0.0f;                // a NaN if any of them is infinite or a NaN
+#pragma unroll
+              for (int j = 0; j < 32; ++j) probe = fmaf(v[j], 0.0f, probe);
+              if (__any_sync(0xFFFFFFFFu, probe != probe && rs == rs) && !later) {
+                bool nan = false;
+#pragma unroll
+                for (int j = 0; j < 32; ++j) nan = nan || v[j] != v[j];
+                if (__any_sync(0xFFFFFFFFu, nan && rs == rs)) {
+                  hdr->redo[ew] = 1 + 2 * t + i;
+                  later = true;
+                }
+              }
+              if (later) continue;
+            }
+            store_chunk<ES, ES == 4 && FORM == kSegCodes>(v, my_bias, my_out, maps, p, n_first, row_off, c1, c2, c3, lane);
           }
         }
         continue;
@@ -800,6 +852,29 @@ lut_dense_tc_kernel(const __grid_constant__ DenseMaps maps, const DenseParams p)
     }
     STEM_ACC(0, t_all);
     if (ew == 0) STEM_FLUSH(8, 2);
+    if constexpr (FORM == kSegSplit) {
+      const int first = hdr->redo[ew];
+      if (ok && first != 0) {     // the chunks left out, here where nothing waits for this warp and it holds no sums
+        int i = (first - 1) & 1;
+#pragma unroll 1
+        for (int t = (first - 1) >> 1; t < num_tiles; t += tile_step, i = 0) {
+          const int n_blk = t % p.n_tiles, c1 = t / p.n_tiles * kBM + quarter * 32;
+          const int64_t row = static_cast<int64_t>(c1) + lane;
+#pragma unroll 1
+          for (; i < 2; ++i) {
+            const int c = sub + 2 * i;
+            const int64_t n_first = static_cast<int64_t>(n_blk) * p.bn + c * 32, n = n_first + lane;
+            if (c >= n_chunks || n_first >= p.N) break;
+            float v[32];
+            plain_chunk(v, p, row, n_first, lane);
+            __syncwarp();
+            my_bias[lane] = p.bias != nullptr && n < p.N ? load_as_float(p.bias, p.bias_dtype, n) : 0.0f;
+            __syncwarp();
+            store_chunk<ES, false>(v, my_bias, my_out, maps, p, n_first, row < p.M ? row * p.N : -1, c1, 0, 0, lane);
+          }
+        }
+      }
+    }
     __syncwarp();
     if (elect_one()) tma_store_wait_all();
     __syncwarp();
@@ -830,7 +905,7 @@ lut_expand_kernel(const uint8_t* __restrict__ packed, const void* __restrict__ c
   // and it waits (griddepcontrol.wait) before it reads what this kernel writes
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   __shared__ uint32_t tbl[BITS <= 4 ? kExpandTable : 1];
-  expand_block<BITS>(tbl, blockIdx.x, packed, codebooks, cb_dtype, entries, group_rows, rows, K, fmt, passes, out, nullptr);
+  expand_block<BITS>(tbl, blockIdx.x, packed, codebooks, cb_dtype, entries, group_rows, rows, K, fmt, passes, out, nullptr, false);
 }
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -1011,7 +1086,8 @@ int launch_dense(DenseMaps& maps, DenseParams& p, const void* scratch, int64_t K
       e = launch_dependent(lut_dense_tc_kernel<4, true>, 2 * clusters, kThreads, smem, st, maps, p, 2);
     }
   } else if (seg) {
-    auto kern = es == 2 ? lut_dense_tc_kernel<2, false, true> : lut_dense_tc_kernel<4, false, true>;
+    auto kern = p.x32 != nullptr ? lut_dense_tc_kernel<4, false, kSegSplit>     // its output is fp32
+                : es == 2 ? lut_dense_tc_kernel<2, false, kSegCodes> : lut_dense_tc_kernel<4, false, kSegCodes>;
     e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSmemMax));
     if (e != cudaSuccess) return static_cast<int>(e);
     e = launch_dependent(kern, grid, kSegThreads, smem, st, maps, p);
@@ -1946,10 +2022,19 @@ int exact_prepare(PrepParams& q, DenseParams& p, const dimq_wq_weight* w, const 
   q.xo = reinterpret_cast<__half*>(base + at.x);
   q.row_scale = a4 ? nullptr : reinterpret_cast<float*>(base + at.row);
   q.col_scale = w->cb_dtype == DIMQ_F16 ? nullptr : reinterpret_cast<float*>(base + at.col);
+  q.split_x = a4 ? 0 : 1;
   const int rc = launch_prep(q, w, packed, N, K, w->cb_dtype == DIMQ_F16 ? 0 : 2, terms, base + at.w, x_blocks, st);
   p.row_scale = q.row_scale;
   p.col_scale = q.col_scale;
   p.out_scale = a4 ? scale : 1.0f;
+  p.x32 = a4 ? nullptr : static_cast<const float*>(q.x);
+  p.packed = packed;
+  p.codebooks = w->codebooks;
+  p.bits = w->bits;
+  p.cb_dtype = w->cb_dtype;
+  p.entries = w->entries;
+  p.group_rows = w->group_rows;
+  p.K = K;
   // products of terms, the small ones first
   p.b_terms = terms;
   p.passes = 0;

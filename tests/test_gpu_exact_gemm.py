@@ -376,3 +376,51 @@ def test_fp32_codebooks_with_an_outlier(ops, k, a4):
     else:
         y, want = ops.dimq_linear_wq(x, packed, books, None, n, k, bits=4), x.double() @ w.t()
     assert ops.last_device_status() == 0 and _rel(y, want) < REL
+
+
+@pytest.mark.parametrize("book", [torch.float16, torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("bits,group_rows", [(4, None), (3, 40), (2, 1)])
+def test_linear_f32_non_finite_codewords(ops, book, bits, group_rows):
+    # an infinite or NaN codeword gives what fp32 products and sums give, whatever its type
+    m, k, n = 140, 192, 100
+    packed, books, _ = _weight(ops, n, k, bits, book, group_rows, seed=6)
+    books = books.clamp(-1e3, 1e3)
+    books[0, 1], books[-1, 2] = float("inf"), float("-inf")
+    if books.shape[0] > 2:
+        books[1, 0] = float("nan")
+    idx = ops.unpack_bits(packed, n * k, bits).view(n, k).long()
+    idx[3:7], idx[9, ::2] = 3, 0                 # columns of finite codewords only, and a mixed one
+    packed = ops.pack_bits(idx.to(torch.uint8), bits)
+    rows = torch.arange(n, device="cuda") // (group_rows or n)
+    w = torch.gather(books.float()[rows], 1, idx)
+    x = torch.randn(m, k, device="cuda")
+    x[5], x[6], x[:, 11] = 0.0, x[6].bfloat16().float(), x[:, 11].half().float()      # zeros, and values exact in one term
+    x[7, 3], x[8, 4], x[9, 5] = float("inf"), float("-inf"), float("nan")
+    x[10] *= torch.logspace(0, -30, k, device="cuda")
+    y = ops.dimq_linear_wq(x, packed, books if group_rows else books.reshape(-1), None, n, k, bits=bits, group_rows=group_rows)
+    # infinities and NaN of the sum follow from those of its products, in any order
+    prod = x.unsqueeze(1) * w.unsqueeze(0)
+    nan = prod.isnan().any(2) | ((prod == float("inf")).any(2) & (prod == float("-inf")).any(2))
+    sign = (prod == float("inf")).any(2).float() - (prod == float("-inf")).any(2).float()
+    assert torch.equal(y.isnan(), nan)
+    assert torch.equal(y.isinf(), ~nan & (sign != 0)) and torch.equal(y[y.isinf()].sign(), sign[y.isinf()])
+    ok = y.isfinite()
+    want = torch.nan_to_num(x.double(), 0, 0, 0) @ torch.nan_to_num(w.double(), 0, 0, 0).t()
+    bound = 1e-6 * torch.nan_to_num(x.double(), 0, 0, 0).norm(dim=1, keepdim=True) * torch.nan_to_num(w.double(), 0, 0, 0).norm(dim=1)
+    assert bool(((y.double() - want).abs() <= bound + 1e-30)[ok].all())
+
+
+def test_linear_f32_infinite_activations_against_tiny_codewords(ops):
+    # a codeword far below the largest of its book is not zero: infinity times it is infinity
+    m, k, n = 40, 64, 64
+    books = torch.tensor([1e4, -1e4, 1e-20, -1e-20, 0.0] + [1.0] * 11, device="cuda")
+    idx = torch.randint(5, 16, (n, k), device="cuda")
+    idx[:, 0] = torch.arange(n, device="cuda") % 5
+    x = torch.randn(m, k, device="cuda")
+    x[3, 0], x[4, 0] = float("inf"), float("-inf")
+    for book in (books, books.bfloat16()):
+        y = ops.dimq_linear_wq(x, ops.pack_bits(idx.to(torch.uint8), 4), book, None, n, k, bits=4)
+        want = x @ book.float()[idx].t()
+        assert torch.equal(y.isnan(), want.isnan()) and torch.equal(y.isinf(), want.isinf())
+        assert torch.equal(y[y.isinf()].sign(), want[want.isinf()].sign())
+        assert _rel(y[:3], (x.double() @ book.double()[idx].t())[:3]) < REL
