@@ -1005,25 +1005,81 @@ PyObject* py_set_ops(PyObject*, PyObject* dict) {
   Py_RETURN_NONE;
 }
 
+// ---- events of the tensors that modules keep (dimq_b200/modules.py) --------------------------------
+
+constexpr char kEvent[] = "dimq_b200.event";
+
+void cuda_ok(cudaError_t e, const char* what) {
+  if (e != cudaSuccess) fail(std::string(what) + " failed: " + cudaGetErrorString(e));
+}
+
+cudaEvent_t as_event(PyObject* o) {
+  void* e = PyCapsule_GetPointer(o, kEvent);
+  if (e == nullptr) throw python_error();
+  return static_cast<cudaEvent_t>(e);
+}
+
+c10::DeviceIndex as_device(PyObject* o) { return static_cast<c10::DeviceIndex>(as_int(o)); }
+
+// a new event, recorded on the device's current stream
+PyObject* py_record_event(PyObject*, PyObject* device) {
+  HANDLE_TH_ERRORS
+  const c10::cuda::CUDAGuard guard(as_device(device));
+  cudaEvent_t e = nullptr;
+  cuda_ok(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "cudaEventCreateWithFlags");
+  PyObject* capsule = PyCapsule_New(e, kEvent, [](PyObject* o) {
+    (void)cudaEventDestroy(static_cast<cudaEvent_t>(PyCapsule_GetPointer(o, kEvent)));
+  });
+  if (capsule == nullptr) {
+    (void)cudaEventDestroy(e);
+    throw python_error();
+  }
+  const cudaError_t rc = cudaEventRecord(e, c10::cuda::getCurrentCUDAStream(as_device(device)).stream());
+  if (rc != cudaSuccess) Py_DECREF(capsule);
+  cuda_ok(rc, "cudaEventRecord");
+  return capsule;
+  END_HANDLE_TH_ERRORS
+}
+
 // Whether an event has completed.  Also while a graph is being captured, when a plain query would end the capture: the
 // event was recorded outside it, and in relaxed mode the question touches nothing that is captured.
-PyObject* py_event_done(PyObject*, PyObject* handle) {
+PyObject* py_event_done(PyObject*, PyObject* event) {
   HANDLE_TH_ERRORS
-  void* event = PyLong_AsVoidPtr(handle);
-  if (event == nullptr && PyErr_Occurred()) throw python_error();
+  const cudaEvent_t ev = as_event(event);
   cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
-  cudaError_t e = cudaThreadExchangeStreamCaptureMode(&mode);
-  if (e == cudaSuccess) {
-    e = cudaEventQuery(static_cast<cudaEvent_t>(event));
-    const cudaError_t back = cudaThreadExchangeStreamCaptureMode(&mode);
-    if (e == cudaSuccess) e = back;
-  }
+  cuda_ok(cudaThreadExchangeStreamCaptureMode(&mode), "cudaThreadExchangeStreamCaptureMode");
+  const cudaError_t e = cudaEventQuery(ev);
+  const cudaError_t back = cudaThreadExchangeStreamCaptureMode(&mode);
   if (e == cudaErrorNotReady) {
     (void)cudaGetLastError();
     Py_RETURN_FALSE;
   }
-  if (e != cudaSuccess) fail(std::string("event query failed: ") + cudaGetErrorString(e));
+  cuda_ok(e, "cudaEventQuery");
+  cuda_ok(back, "cudaThreadExchangeStreamCaptureMode");
   Py_RETURN_TRUE;
+  END_HANDLE_TH_ERRORS
+}
+
+PyObject* py_wait_event(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  want_args(n, 2, "wait_event");
+  cuda_ok(cudaStreamWaitEvent(c10::cuda::getCurrentCUDAStream(as_device(a[1])).stream(), as_event(a[0]), 0), "cudaStreamWaitEvent");
+  Py_RETURN_NONE;
+  END_HANDLE_TH_ERRORS
+}
+
+// Whether the device's current stream is being captured into a graph
+PyObject* py_capturing(PyObject*, PyObject* device) {
+  HANDLE_TH_ERRORS
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  const cudaError_t e = cudaStreamIsCapturing(c10::cuda::getCurrentCUDAStream(as_device(device)).stream(), &status);
+  if (e == cudaErrorStreamCaptureImplicit) {      // the legacy stream beside a capture on a blocking one: not itself captured
+    (void)cudaGetLastError();
+    Py_RETURN_FALSE;
+  }
+  cuda_ok(e, "cudaStreamIsCapturing");
+  if (status != cudaStreamCaptureStatusNone) Py_RETURN_TRUE;
+  Py_RETURN_FALSE;
   END_HANDLE_TH_ERRORS
 }
 
@@ -1033,7 +1089,10 @@ PyMethodDef kMethods[] = {FAST(linear_wq), FAST(linear_a4), FAST(conv2d_wq), FAS
                           FAST(max_pool_nhwc), FAST(images_to_nhwc), FAST(attention_qkv),
                           {"set_launch_count", py_set_launch_count, METH_O, nullptr},
                           {"set_ops", py_set_ops, METH_O, nullptr},
+                          {"record_event", py_record_event, METH_O, nullptr},
                           {"event_done", py_event_done, METH_O, nullptr},
+                          FAST(wait_event),
+                          {"capturing", py_capturing, METH_O, nullptr},
                           {nullptr, nullptr, 0, nullptr}};
 PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_host", nullptr, -1, kMethods, nullptr, nullptr, nullptr, nullptr};
 

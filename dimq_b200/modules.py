@@ -38,51 +38,40 @@ class _Derived:
     the buffer still is what it was, and that the writing of the tensor - on the stream of the call that first needed it -
     comes before.  Holds the buffer's storage, so that a new one cannot turn up at its address."""
 
-    __slots__ = ("source", "version", "extra", "value", "event", "written", "builder", "streams")
+    __slots__ = ("source", "address", "version", "extra", "value", "event", "written", "builder", "streams")
 
     def __init__(self, source: torch.Tensor, extra, value: torch.Tensor) -> None:
-        self.source, self.version, self.extra, self.value = source.detach(), source._version, extra, value
-        with torch.cuda.device(value.device):
-            stream = torch.cuda.current_stream()
-            self.event = torch.cuda.Event()
-            self.event.record(stream)
+        self.source, self.address, self.version = source.detach(), source.data_ptr(), source._version
+        self.extra, self.value = extra, value
+        device = value.get_device()
+        self.event = _lib.host().record_event(device)
         self.written = False                     # known to be complete, for every stream
-        self.builder = stream.cuda_stream
-        self.streams = {stream.cuda_stream}      # those the allocator knows to read the value
+        self.builder = torch._C._cuda_getCurrentRawStream(device)
+        self.streams = {self.builder}            # those the allocator knows to read the value
 
     def __reduce__(self):                        # copied and saved modules derive their own
         return type(None), ()
 
     def is_of(self, source: torch.Tensor, extra) -> bool:
-        return (self.source.data_ptr() == source.data_ptr() and self.version == source._version
-                and self.source.device == source.device and self.extra == extra)
+        return self.address == source.data_ptr() and self.version == source._version and self.extra == extra
 
     def readable(self) -> bool:
         """Make the current stream wait for the value where it has to.  False in a graph capture that began before the
         value was written: a replay would not wait."""
-        device = self.source.get_device()
+        device = self.value.get_device()
         raw = torch._C._cuda_getCurrentRawStream(device)
-        if self.written and raw in self.streams:
-            return True
-        with torch.cuda.device(device):
-            if not self.written:
-                if _lib.host().event_done(self.event.cuda_event):
-                    self.written = True
-                elif torch.cuda.is_current_stream_capturing():
-                    return False
-                elif raw != self.builder:
-                    torch.cuda.current_stream().wait_event(self.event)
-            if raw not in self.streams:
-                self.value.record_stream(torch.cuda.current_stream())
-                self.streams.add(raw)
+        if not self.written:
+            host = _lib.host()
+            if host.event_done(self.event):
+                self.written = True
+            elif host.capturing(device):
+                return False
+            elif raw != self.builder:
+                host.wait_event(self.event, device)
+        if raw not in self.streams:
+            self.value.record_stream(torch.cuda.current_stream(device))
+            self.streams.add(raw)
         return True
-
-
-def _capturing(device: int) -> bool:
-    if device == torch.cuda.current_device():
-        return torch.cuda.is_current_stream_capturing()
-    with torch.cuda.device(device):
-        return torch.cuda.is_current_stream_capturing()
 
 
 def _pair(value) -> tuple[int, int]:
@@ -110,11 +99,14 @@ class _PackedBase(nn.Module):
             raise ValueError("the W4A4 mode needs 4-bit indices and one 16-entry codebook; "
                              "pass act_scale=None for weight-only layers")
 
-    def _tensor(self, name: str) -> torch.Tensor | None:
-        """``getattr(self, name)``, without the attribute protocol of ``nn.Module`` while it is the buffer it was registered as
-        (a codebook or bias may have become a parameter or a parametrised property since)."""
+    def _operands(self) -> tuple[torch.Tensor, torch.Tensor, torch.Tensor | None]:
+        """Indices, codebook, bias - without the attribute protocol of ``nn.Module`` while all are the buffers they were
+        registered as (a codebook or bias may have become a parameter or a parametrised property since)."""
         buffers = self._buffers
-        return buffers[name] if name in buffers else getattr(self, name)
+        try:
+            return buffers["packed_weight"], buffers["codebook"], buffers["bias"]
+        except KeyError:
+            return self.packed_weight, self.codebook, self.bias
 
     def _derive(self, slot: str, source: torch.Tensor, build, extra=None) -> torch.Tensor:
         """``build()`` from the buffer ``source``, kept in ``slot`` until the buffer is replaced, moved or written in place.
@@ -125,7 +117,7 @@ class _PackedBase(nn.Module):
         if type(kept) is _Derived and counted and kept.is_of(source, extra) and kept.readable():
             return kept.value
         value = build()
-        if counted and not _capturing(source.get_device()):
+        if counted and not _lib.host().capturing(source.get_device()):
             self.__dict__[slot] = _Derived(source, extra, value)
         return value
 
@@ -144,10 +136,10 @@ class _PackedBase(nn.Module):
         return self._derive("_scaled_cb", cb, lambda: cb.detach().float().reshape(-1) * torch.tensor(
             self.act_scale, dtype=torch.float32, device=cb.device), self.act_scale)
 
-    def _check_input(self, x: torch.Tensor) -> None:
+    def _check_input(self, x: torch.Tensor, packed_weight: torch.Tensor) -> None:
         if not self.use_cuda_kernel:
             raise RuntimeError("dimq_b200 has no Python fallback path (use_cuda_kernel=False is not supported)")
-        if not (x.is_cuda and self._tensor("packed_weight").is_cuda):
+        if not (x.is_cuda and packed_weight.is_cuda):
             raise RuntimeError("dimq_b200 layers run on CUDA tensors only; move the module and its input to a B200")
 
 
@@ -177,35 +169,33 @@ class DIMQLinear(_PackedBase):
         return self._derive("_tiled", pw, lambda: ops.linear_prepack(pw, self.out_features, self.in_features, self.bits))
 
     def forward(self, x: torch.Tensor, residual: torch.Tensor | None = None) -> torch.Tensor:
-        self._check_input(x)
+        packed, book, bias = self._operands()
+        self._check_input(x, packed)
         if self.act_scale is None:
             tiled = self._prepacked(x.numel() // self.in_features, x)
-            return ops.dimq_linear_wq(x, self._tensor("packed_weight"), self._tensor("codebook"), self._tensor("bias"),
-                                      self.out_features, self.in_features, bits=self.bits, group_rows=self.group_rows,
-                                      out_dtype=self.out_dtype, epilogue=self.epilogue, residual=residual,
-                                      packed_tiled=tiled)
+            return ops.dimq_linear_wq(x, packed, book, bias, self.out_features, self.in_features, bits=self.bits,
+                                      group_rows=self.group_rows, out_dtype=self.out_dtype, epilogue=self.epilogue,
+                                      residual=residual, packed_tiled=tiled)
         rows = x.numel() // self.in_features
         if rows >= ops.A4_TC_MIN_ROWS and self.in_features % 64 == 0:
             # The fp32-grade form, except for an fp32 codebook on many rows: there it multiplies two fp16 terms in
             # tiles of 128 x 128, the bf16 pair below in tiles of 256 (768 -> 3072: 20.5 against 21.1 us at 512 rows,
             # 36 / 30 at 1576; with an fp16 codebook, one term, 13.6 / 20.9 and 22 / 30, 120 / 124 for 4096 x 3072 -> 3072).
-            if self.codebook.dtype != torch.float32 or rows < 1024:
-                y = ops.dimq_linear_a4(x, self.packed_weight, self.codebook, self.act_scale, self.act_zero_point,
-                                       self.bias, self.out_features, self.in_features, out_dtype=self.out_dtype,
-                                       epilogue=self.epilogue, residual=residual)
+            if book.dtype != torch.float32 or rows < 1024:
+                y = ops.dimq_linear_a4(x, packed, book, self.act_scale, self.act_zero_point, bias, self.out_features,
+                                       self.in_features, out_dtype=self.out_dtype, epilogue=self.epilogue, residual=residual)
                 if y is not None:
                     return y
             # centred activation codes (exact in bf16) times the scaled codebook through the weight-only
             # tensor-core path; per-layer state is cached, nothing is re-derived per call
             codes = ops.centre_quantize_u4(x, self.act_scale, self.act_zero_point)
-            return ops.dimq_linear_wq(codes, self.packed_weight, self._scaled_codebook(), self.bias,
-                                      self.out_features, self.in_features, bits=4, out_dtype=self.out_dtype,
-                                      epilogue=self.epilogue, residual=residual)
+            return ops.dimq_linear_wq(codes, packed, self._scaled_codebook(), bias, self.out_features, self.in_features,
+                                      bits=4, out_dtype=self.out_dtype, epilogue=self.epilogue, residual=residual)
         if residual is not None or self.epilogue is not None:
             raise RuntimeError("a fused epilogue or residual needs the weight-only mode or at least "
                                f"{ops.A4_TC_MIN_ROWS} activation rows")
-        return ops.dimq_linear_lut(x, self.packed_weight, self.codebook, self.act_scale, self.act_zero_point,
-                                   self.bias, self.out_features, self.in_features)
+        return ops.dimq_linear_lut(x, packed, book, self.act_scale, self.act_zero_point, bias, self.out_features,
+                                   self.in_features)
 
     @classmethod
     def from_export_layer(cls, layer: Mapping[str, Any], *, use_cuda_kernel: bool = True, **extra) -> "DIMQLinear":
@@ -240,15 +230,15 @@ class DIMQConv2d(_PackedBase):
     def _prepacked(self) -> torch.Tensor | None:
         if self.groups != 1 or self.weight_shape[1] % 64 != 0:
             return None
-        pw = self._tensor("packed_weight")
+        pw = self._operands()[0]
         return self._derive("_khwc", pw, lambda: ops.conv_prepack(pw, self.weight_shape, self.bits))
 
     def forward(self, x: torch.Tensor, residual: torch.Tensor | None = None) -> torch.Tensor:
-        self._check_input(x)
+        packed, book, bias = self._operands()
+        self._check_input(x, packed)
         if self.act_scale is None:
-            return ops.dimq_conv2d_wq(x, self._tensor("packed_weight"), self._tensor("codebook"), self._tensor("bias"),
-                                      self.weight_shape, self.stride, self.padding, self.dilation, self.groups, bits=self.bits,
-                                      group_rows=self.group_rows, out_dtype=self.out_dtype, epilogue=self.epilogue,
+            return ops.dimq_conv2d_wq(x, packed, book, bias, self.weight_shape, self.stride, self.padding, self.dilation,
+                                      self.groups, bits=self.bits, group_rows=self.group_rows, out_dtype=self.out_dtype, epilogue=self.epilogue,
                                       residual=residual, packed_khwc=self._prepacked())
         tc = self.groups == 1 and self.weight_shape[1] % 64 == 0
         channels_last = x.dim() == 4 and x.is_contiguous(memory_format=torch.channels_last) and not x.is_contiguous()
@@ -259,35 +249,33 @@ class DIMQConv2d(_PackedBase):
                 khwc = self._prepacked()
                 # fp16 / bf16 codebooks are one exact term: the fp32-grade form (64 x 64 channels on 56^2, batch 64:
                 # 66 us, the bf16 pair 82; 512 on 7^2: 35 / 52); an fp32 codebook takes two there (94 / 82, 60 / 52)
-                if self.codebook.dtype != torch.float32:
-                    y = ops.dimq_conv2d_a4(x, self.packed_weight, self.codebook, self.act_scale, self.act_zero_point,
-                                           self.bias, self.weight_shape, self.stride, self.padding, self.dilation,
-                                           self.groups, out_dtype=self.out_dtype, epilogue=self.epilogue,
-                                           residual=residual, packed_khwc=khwc)
+                if book.dtype != torch.float32:
+                    y = ops.dimq_conv2d_a4(x, packed, book, self.act_scale, self.act_zero_point, bias, self.weight_shape,
+                                           self.stride, self.padding, self.dilation, self.groups, out_dtype=self.out_dtype,
+                                           epilogue=self.epilogue, residual=residual, packed_khwc=khwc)
                     if y is not None:
                         return y
                 # centred activation codes times the scaled codebook through the weight-only implicit-GEMM path,
                 # with the re-ordered indices and the scaled codebook cached on the module
                 codes = ops.centre_quantize_u4(x, self.act_scale, self.act_zero_point)
-                return ops.dimq_conv2d_wq(codes, self.packed_weight, self._scaled_codebook(), self.bias,
+                return ops.dimq_conv2d_wq(codes, packed, self._scaled_codebook(), bias,
                                           self.weight_shape, self.stride, self.padding, self.dilation, self.groups,
                                           bits=4, out_dtype=self.out_dtype, epilogue=self.epilogue, residual=residual,
                                           packed_khwc=khwc)
         if residual is not None or self.epilogue is not None:
             raise RuntimeError("a fused epilogue or residual needs the weight-only mode, or channels_last input "
                                f"with at least {ops.A4_TC_MIN_ROWS} output pixels")
-        if tc and x.dim() == 4 and _eager(x, self.codebook, self.bias):
+        if tc and x.dim() == 4 and _eager(x, book, bias):
             # NCHW activations, or few pixels: the re-ordered indices are kept here, not re-derived per call.  A captured
             # graph re-derives them in every replay: it follows packed_weight itself, as dimq_conv2d_lut does.
-            khwc = None if _capturing(x.get_device()) else self._prepacked()
-            y = ops.dimq_conv2d_a4(x, self.packed_weight, self.codebook, self.act_scale, self.act_zero_point, self.bias,
+            khwc = None if _lib.host().capturing(x.get_device()) else self._prepacked()
+            y = ops.dimq_conv2d_a4(x, packed, book, self.act_scale, self.act_zero_point, bias,
                                    self.weight_shape, self.stride, self.padding, self.dilation, self.groups,
                                    packed_khwc=khwc)
             if y is not None:
                 return y
-        return ops.dimq_conv2d_lut(x, self.packed_weight, self.codebook, self.act_scale, self.act_zero_point,
-                                   self.bias, self.weight_shape, self.stride, self.padding, self.dilation,
-                                   self.groups)
+        return ops.dimq_conv2d_lut(x, packed, book, self.act_scale, self.act_zero_point, bias, self.weight_shape, self.stride,
+                                   self.padding, self.dilation, self.groups)
 
     @classmethod
     def from_export_layer(cls, layer: Mapping[str, Any], *, use_cuda_kernel: bool = True, **extra) -> "DIMQConv2d":

@@ -2,7 +2,6 @@
 
 from __future__ import annotations
 
-import contextlib
 import copy
 import pickle
 import types
@@ -21,27 +20,19 @@ class _Gpu:
         self.current, self.capturing, self.done, self.log, self.built = 1, False, False, [], 0
         gpu = self
 
-        class Event:
-            cuda_event = 7
-
-            def record(self, stream):
-                gpu.log.append(("record", stream.cuda_stream))
-
-        def stream():
-            raw = gpu.current
-            return types.SimpleNamespace(cuda_stream=raw, wait_event=lambda e: gpu.log.append(("wait", raw)))
+        def record(device):
+            gpu.log.append(("record", gpu.current))
+            return "event"
 
         def prepack(pw, *args):
             gpu.built += 1
             return pw.clone()
 
-        monkeypatch.setattr(torch.cuda, "Event", Event)
-        monkeypatch.setattr(torch.cuda, "current_stream", lambda *a: stream())
-        monkeypatch.setattr(torch.cuda, "device", lambda d: contextlib.nullcontext())
-        monkeypatch.setattr(torch.cuda, "current_device", lambda: -1)
-        monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: gpu.capturing)
+        monkeypatch.setattr(torch.cuda, "current_stream", lambda *a: types.SimpleNamespace(cuda_stream=gpu.current))
         monkeypatch.setattr(torch._C, "_cuda_getCurrentRawStream", lambda d: gpu.current, raising=False)
-        monkeypatch.setattr(_lib, "host", lambda: types.SimpleNamespace(event_done=lambda h: gpu.done))
+        monkeypatch.setattr(_lib, "host", lambda: types.SimpleNamespace(
+            record_event=record, event_done=lambda e: gpu.done, capturing=lambda d: gpu.capturing,
+            wait_event=lambda e, d: gpu.log.append(("wait", gpu.current))))
         monkeypatch.setattr(torch.Tensor, "record_stream", lambda t, s: gpu.log.append(("uses", s.cuda_stream)))
         monkeypatch.setattr(ops, "conv_prepack", prepack)
 
@@ -115,8 +106,8 @@ def test_buffers_may_have_become_parameters(monkeypatch):
     seen = []
     monkeypatch.setattr(ops, "dimq_linear_wq", lambda x, pw, cb, bias, *a, **k: seen.append((pw, cb, bias)))
     monkeypatch.setattr(ops, "dimq_conv2d_wq", lambda x, pw, cb, bias, *a, **k: seen.append((pw, cb, bias)))
-    monkeypatch.setattr(DIMQLinear, "_check_input", lambda self, x: self._tensor("packed_weight"))
-    monkeypatch.setattr(DIMQConv2d, "_check_input", lambda self, x: self._tensor("packed_weight"))
+    monkeypatch.setattr(DIMQLinear, "_check_input", lambda self, x, pw: None)
+    monkeypatch.setattr(DIMQConv2d, "_check_input", lambda self, x, pw: None)
     monkeypatch.setattr(DIMQConv2d, "_prepacked", lambda self: None)
     for layer in (DIMQLinear(torch.zeros(32, dtype=torch.uint8), torch.zeros(16), None, None, 8, 8, torch.zeros(8)),
                   DIMQConv2d(torch.zeros(32, dtype=torch.uint8), torch.zeros(16), None, None, (8, 8, 1, 1), torch.zeros(8))):
