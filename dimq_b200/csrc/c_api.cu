@@ -254,12 +254,13 @@ namespace {
 enum class WsRoute { kPlain, kRegs, kExact, kDense, kSplit };
 
 int linear_ws_route(const void* x, int x_dtype, const dimq_wq_weight* w, const void* residual, const void* y, int y_dtype,
-                    int64_t M, int64_t N, int64_t K, int64_t workspace_bytes, WsRoute* route) {
+                    int64_t M, int64_t N, int64_t K, int64_t workspace_bytes, int64_t* asked, WsRoute* route) {
   *route = WsRoute::kPlain;
-  int64_t need = 0;
-  const int rc = dimq_linear_wq_workspace_bytes(x, x_dtype, w, M, N, K, &need);
+  const int rc = dimq_linear_wq_workspace_bytes(x, x_dtype, w, M, N, K, asked);
   if (rc != DIMQ_OK) return rc;
+  const int64_t need = *asked;
   if (need == 0) return DIMQ_OK;
+  if (workspace_bytes < 0) workspace_bytes = need;      // a plan with the scratch the query asks for
   if (mma_regs_supported(x, x_dtype, w, M, N, K) && mma_regs_pays(w, N, K)) {
     if (workspace_bytes < need) return DIMQ_ERR_SCRATCH_TOO_SMALL;
     *route = WsRoute::kRegs;
@@ -287,17 +288,21 @@ int linear_ws_route(const void* x, int x_dtype, const dimq_wq_weight* w, const v
 
 extern "C" int dimq_linear_wq_ws_plan(const void* x, int x_dtype, const dimq_wq_weight* w, const void* residual,
                                       const void* y, int y_dtype, int64_t M, int64_t N, int64_t K,
-                                      int64_t workspace_bytes, int* kernels) {
-  if (w == nullptr || kernels == nullptr) return DIMQ_ERR_NULL_POINTER;
+                                      int64_t workspace_bytes, int64_t* bytes, int* kernels) {
+  if (w == nullptr || bytes == nullptr || kernels == nullptr) return DIMQ_ERR_NULL_POINTER;
+  *bytes = 0;
   *kernels = 0;
   if (M < 0 || N <= 0 || K <= 0) return DIMQ_ERR_BAD_SIZE;
   if (!valid_dtype(x_dtype) || !valid_dtype(y_dtype)) return DIMQ_ERR_BAD_DTYPE;
   int rc = check_wq_weight(w, N);
   if (rc != DIMQ_OK || M == 0) return rc;
   WsRoute route;
-  rc = linear_ws_route(x, x_dtype, w, residual, y, y_dtype, M, N, K, workspace_bytes, &route);
-  if (rc == DIMQ_OK) *kernels = route == WsRoute::kPlain ? 1 : 2;
-  return rc;
+  int64_t need = 0;
+  rc = linear_ws_route(x, x_dtype, w, residual, y, y_dtype, M, N, K, workspace_bytes, &need, &route);
+  if (rc != DIMQ_OK) return rc;
+  *kernels = route == WsRoute::kPlain ? 1 : 2;
+  *bytes = route == WsRoute::kPlain ? 0 : route == WsRoute::kSplit ? M * N * 4 : need;
+  return DIMQ_OK;
 }
 
 extern "C" int dimq_linear_wq_ws(const void* x, int x_dtype, const dimq_wq_weight* w, const void* bias, int bias_dtype,
@@ -308,7 +313,8 @@ extern "C" int dimq_linear_wq_ws(const void* x, int x_dtype, const dimq_wq_weigh
       x != nullptr && y != nullptr) {
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     WsRoute route;
-    const int rc = linear_ws_route(x, x_dtype, w, residual, y, y_dtype, M, N, K, workspace_bytes, &route);
+    int64_t need = 0;
+    const int rc = linear_ws_route(x, x_dtype, w, residual, y, y_dtype, M, N, K, workspace_bytes < 0 ? 0 : workspace_bytes, &need, &route);
     if (rc != DIMQ_OK) return rc;
     switch (route) {
       case WsRoute::kRegs:

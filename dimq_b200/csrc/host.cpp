@@ -275,14 +275,12 @@ Tensor linear_wq(const Tensor& x, const Tensor& packed, const Tensor& books, con
   void* st = stream_of(x);
   // Regimes that need scratch: a few activation rows against a large weight (the k slices of the small-M kernel meet
   // there), many activation rows (the indices are expanded once to a 16-bit weight), fp32 activations (split into
-  // fp16 terms) and a few hundred rows against a long K (split-K partial tiles).  The query does not see the output:
-  // fp32 activations are split for an fp32 result only.
+  // fp16 terms) and a few hundred rows against a long K (split-K partial tiles).
   int64_t need = 0;
-  if (xd != DIMQ_F32 || yd == DIMQ_F32) dimq_linear_wq_workspace_bytes(xc.data_ptr(), xd, &w.w, m, n, k, &need);
+  int kernels = 0;
+  dimq_linear_wq_ws_plan(xc.data_ptr(), xd, &w.w, ptr(res), y.data_ptr(), yd, m, n, k, -1, &need, &kernels);
   if (need > 0) {
     Tensor ws = scratch(need, x);
-    int kernels = 0;
-    dimq_linear_wq_ws_plan(xc.data_ptr(), xd, &w.w, ptr(res), y.data_ptr(), yd, m, n, k, need, &kernels);
     check(dimq_linear_wq_ws(xc.data_ptr(), xd, &w.w, ptr(b.t), b.dtype, ptr(res), y.data_ptr(), yd, m, n, k, epilogue,
                             ws.data_ptr(), need, st), "linear_wq_ws");
     *launches = kernels;    // expansion + GEMM, GEMM + the kernel that finishes the sums, or a GEMM alone

@@ -238,8 +238,8 @@ class DIMQConv2d(_PackedBase):
         self._check_input(x, packed)
         if self.act_scale is None:
             return ops.dimq_conv2d_wq(x, packed, book, bias, self.weight_shape, self.stride, self.padding, self.dilation,
-                                      self.groups, bits=self.bits, group_rows=self.group_rows, out_dtype=self.out_dtype, epilogue=self.epilogue,
-                                      residual=residual, packed_khwc=self._prepacked())
+                                      self.groups, bits=self.bits, group_rows=self.group_rows, out_dtype=self.out_dtype,
+                                      epilogue=self.epilogue, residual=residual, packed_khwc=self._prepacked())
         tc = self.groups == 1 and self.weight_shape[1] % 64 == 0
         channels_last = x.dim() == 4 and x.is_contiguous(memory_format=torch.channels_last) and not x.is_contiguous()
         if tc and channels_last and self.stride[0] == self.stride[1] and self.stride[0] in (1, 2):

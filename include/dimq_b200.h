@@ -239,11 +239,13 @@ DIMQ_API int dimq_linear_wq_workspace_bytes(const void* x, int x_dtype, const di
 DIMQ_API int dimq_linear_wq_ws(const void* x, int x_dtype, const dimq_wq_weight* w, const void* bias, int bias_dtype,
                                const void* residual, void* y, int y_dtype, int64_t M, int64_t N, int64_t K,
                                int epilogue, void* workspace, int64_t workspace_bytes, void* stream);
-/* What dimq_linear_wq_ws does with these arguments and a workspace of this size, without doing it: its status (OK, or
- * DIMQ_ERR_SCRATCH_TOO_SMALL) and the number of kernels it launches.  Host logic only; no pointer is dereferenced. */
+/* What dimq_linear_wq_ws does with these arguments and a workspace of this size (negative: of the size the query reports),
+ * without doing it: its status (OK, or DIMQ_ERR_SCRATCH_TOO_SMALL), the bytes of scratch it uses - 0 where the output does
+ * not suit the form the query had in mind - and the number of kernels it launches.  Host logic only; no pointer is
+ * dereferenced. */
 DIMQ_API int dimq_linear_wq_ws_plan(const void* x, int x_dtype, const dimq_wq_weight* w, const void* residual,
                                     const void* y, int y_dtype, int64_t M, int64_t N, int64_t K,
-                                    int64_t workspace_bytes, int* kernels);
+                                    int64_t workspace_bytes, int64_t* bytes, int* kernels);
 
 /* The same for dimq_conv2d_wq: with w->packed_khwc, channels_last 16-bit x and y, groups 1, input
  * channels a multiple of 64, stride 1 or 2 and at least 1024 output pixels, the re-ordered indices are

@@ -118,7 +118,7 @@ def test_linear_workspace_of_the_queried_size_is_enough(lib, x_dtype, y_dtype, b
     from dimq_b200 import _lib
 
     fake = 1 << 20                                   # an aligned address that is never dereferenced
-    need, kernels = C.c_int64(-1), C.c_int(-1)
+    need, uses, kernels = C.c_int64(-1), C.c_int64(-1), C.c_int(-1)
     for n in (100, 500, 1000, 1004, 4096):
         w = _lib.WqWeight(fake, 4, fake, book, 16, 1, n, None)
         for k in (768, 1024, 2048, 4096):
@@ -126,8 +126,13 @@ def test_linear_workspace_of_the_queried_size_is_enough(lib, x_dtype, y_dtype, b
                 shape = (C.c_int64(m), C.c_int64(n), C.c_int64(k))
                 assert lib.dimq_linear_wq_workspace_bytes(C.c_void_p(fake), x_dtype, C.byref(w), *shape, C.byref(need)) == 0
                 rc = lib.dimq_linear_wq_ws_plan(C.c_void_p(fake), x_dtype, C.byref(w), None, C.c_void_p(fake), y_dtype, *shape,
-                                                need, C.byref(kernels))
-                assert rc == 0 and kernels.value in ((1, 2) if need.value else (1,)), (m, n, k, rc)
+                                                need, C.byref(uses), C.byref(kernels))
+                assert rc == 0 and kernels.value == (2 if uses.value else 1) and 0 <= uses.value <= need.value, (m, n, k, rc)
+                # and the bytes it says it uses are enough for the same plan
+                plan = uses.value, kernels.value
+                assert lib.dimq_linear_wq_ws_plan(C.c_void_p(fake), x_dtype, C.byref(w), None, C.c_void_p(fake), y_dtype, *shape,
+                                                  C.c_int64(plan[0] or -1), C.byref(uses), C.byref(kernels)) == 0
+                assert (uses.value, kernels.value) == plan, (m, n, k)
 
 
 def test_conv_geometry(lib):
