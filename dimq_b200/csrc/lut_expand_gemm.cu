@@ -934,15 +934,20 @@ CUtensorMapDataType map_dtype(int dtype) {
 // a commit: ~590 at N = 256, ~450 at N = 128, ~430 at N = 64: below N = 256 the per-instruction floor
 // of about 106 cycles shows).
 // Two-term weights: 256 wide they take two passes; narrower tiles multiply both terms at once (stacked).
+double block_cycles(int bn, bool stacked) {
+  if (bn == 256) return stacked ? 1180.0 : 590.0;
+  if (bn == 128) return stacked ? 590.0 : 450.0;
+  return stacked ? 450.0 : 430.0;
+}
+
 int choose_bn(int64_t m_tiles, int64_t N, int max_bn = 256, bool stacked = false) {
   const int cand[3] = {256, 128, 64};
-  const double cycles[3] = {stacked ? 1180.0 : 590.0, stacked ? 590.0 : 450.0, stacked ? 450.0 : 430.0};
   int best = max_bn;
   double best_cost = -1.0;
   for (int i = 0; i < 3; ++i) {
     if (cand[i] > max_bn) continue;
     const int64_t tiles = m_tiles * ((N + cand[i] - 1) / cand[i]);
-    const double cost = static_cast<double>((tiles + kNumSMs - 1) / kNumSMs) * cycles[i];
+    const double cost = static_cast<double>((tiles + kNumSMs - 1) / kNumSMs) * block_cycles(cand[i], stacked);
     if (best_cost < 0.0 || cost < best_cost) { best_cost = cost; best = cand[i]; }
   }
   return best;
@@ -1229,7 +1234,7 @@ bool linear_dense_pays(const void* x, int x_dtype, const dimq_wq_weight* w, int6
   const bool stacked = two_terms && !rows16_applies(x, x_dtype, w);
   const int64_t m_tiles = (M + kBM - 1) / kBM;
   const int bn = choose_bn(m_tiles, N, 256, stacked);
-  const double per_block = (bn == 64 ? (stacked ? 450.0 : 430.0) : bn == 128 ? (stacked ? 590.0 : 450.0) : (stacked ? 1180.0 : 590.0)) / 1850.0;
+  const double per_block = block_cycles(bn, stacked) / 1850.0;      // us
   const int64_t tiles = m_tiles * ((N + bn - 1) / bn);
   const double dense = 5.0 + (stacked ? 1.24e-6 : 0.62e-6) * static_cast<double>(N) * static_cast<double>(K) +
                        static_cast<double>((tiles + kNumSMs - 1) / kNumSMs) * kb * per_block + 0.012 * bn;

@@ -215,11 +215,14 @@ DIMQ_API int dimq_conv2d_wq_static(const void* x, int x_dtype, const dimq_wq_wei
  *    different CTAs, each writes its partial sums to the workspace (slices * M * N * 4 bytes, at most 8
  *    slices at a time) and a second small kernel adds them in a fixed order and applies bias / epilogue /
  *    residual: no atomics, the same bits every run.
- *  - many activation rows (M >= 1024, 16-bit x, K a multiple of 64, 16-byte aligned y rows): the
- *    indices are expanded ONCE per call into a 16-bit weight matrix in the workspace (N*K*2 bytes; twice
- *    that when bf16 activations meet a codebook that is not stored in bf16 and every codeword is carried
- *    as a hi + lo pair) and a dense TMA + tcgen05 GEMM runs over it.  Looking the indices up inside the
- *    GEMM pipeline instead repeats the N*K lookups once per 192 activation rows.
+ *  - many activation rows (16-bit x and a result of its type or fp32, K a multiple of 64, 16-byte aligned y rows; from
+ *    1024 rows on always, below where a cost model over the shape says so - for a 16-bit result only, if K would
+ *    otherwise be split): the indices are expanded ONCE per call into a 16-bit weight matrix in the workspace (N*K*2
+ *    bytes; twice that when bf16 activations meet a codebook that is not stored in bf16 and every codeword is carried
+ *    as a hi + lo pair) and a dense TMA + tcgen05 GEMM runs over it.  bf16 activations against an fp16 codebook ask for
+ *    M*K halves, M floats and the weight once: the rows are scaled by powers of two into fp16 (exact down to 2^-30 of
+ *    the row's largest element) and multiplied once; with the pair's bytes alone the pair runs.  Looking the indices
+ *    up inside the GEMM pipeline instead repeats the N*K lookups once per 192 activation rows.
  *  - a few hundred activation rows against a long K, whose tiles would occupy only a few SMs: the
  *    in-pipeline tcgen05 kernel cuts K into slices (split-K), adds the partial sums into the workspace
  *    (M*N*4 bytes, float atomics: the last bits can differ from run to run) and a second small kernel
