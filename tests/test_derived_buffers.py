@@ -106,8 +106,7 @@ def test_buffers_may_have_become_parameters(monkeypatch):
     seen = []
     monkeypatch.setattr(ops, "dimq_linear_wq", lambda x, pw, cb, bias, *a, **k: seen.append((pw, cb, bias)))
     monkeypatch.setattr(ops, "dimq_conv2d_wq", lambda x, pw, cb, bias, *a, **k: seen.append((pw, cb, bias)))
-    monkeypatch.setattr(DIMQLinear, "_check_input", lambda self, x, pw: None)
-    monkeypatch.setattr(DIMQConv2d, "_check_input", lambda self, x, pw: None)
+    monkeypatch.setattr(modules._PackedBase, "_refuse", lambda self: None)
     monkeypatch.setattr(DIMQConv2d, "_prepacked", lambda self: None)
     for layer in (DIMQLinear(torch.zeros(32, dtype=torch.uint8), torch.zeros(16), None, None, 8, 8, torch.zeros(8)),
                   DIMQConv2d(torch.zeros(32, dtype=torch.uint8), torch.zeros(16), None, None, (8, 8, 1, 1), torch.zeros(8))):
