@@ -23,14 +23,15 @@ import torch.nn as nn
 from . import _lib, ops
 
 
-def _eager(x: torch.Tensor, *params: torch.Tensor | None) -> bool:
+def _eager(x: torch.Tensor, codebook: torch.Tensor, bias: torch.Tensor | None) -> bool:
     """Plain eager execution: no tracer, dispatch or function mode, tensor subclass, function transform or gradient that
     has to see the registered operator."""
     if not (type(x) is torch.Tensor and torch._C._len_torch_dispatch_stack() == 0
             and torch._C._len_torch_function_stack() == 0 and not torch._C._is_tracing()
             and torch._C._functorch.peek_interpreter_stack() is None):
         return False
-    return not torch.is_grad_enabled() or not (x.requires_grad or any(p is not None and p.requires_grad for p in params))
+    return not torch.is_grad_enabled() or not (x.requires_grad or codebook.requires_grad
+                                               or (bias is not None and bias.requires_grad))
 
 
 class _Derived:
@@ -38,15 +39,15 @@ class _Derived:
     the buffer still is what it was, and that the writing of the tensor - on the stream of the call that first needed it -
     comes before.  Holds the buffer's storage, so that a new one cannot turn up at its address."""
 
-    __slots__ = ("source", "address", "version", "extra", "value", "event", "written", "builder", "streams")
+    __slots__ = ("source", "address", "version", "extra", "value", "device", "event", "written", "builder", "streams")
 
     def __init__(self, source: torch.Tensor, extra, value: torch.Tensor) -> None:
         self.source, self.address, self.version = source.detach(), source.data_ptr(), source._version
         self.extra, self.value = extra, value
-        device = value.get_device()
-        self.event = _lib.host().record_event(device)
+        self.device = value.get_device()
+        self.event = _lib.host().record_event(self.device)
         self.written = False                     # known to be complete, for every stream
-        self.builder = torch._C._cuda_getCurrentRawStream(device)
+        self.builder = torch._C._cuda_getCurrentRawStream(self.device)
         self.streams = {self.builder}            # those the allocator knows to read the value
 
     def __reduce__(self):                        # copied and saved modules derive their own
@@ -58,18 +59,19 @@ class _Derived:
     def readable(self) -> bool:
         """Make the current stream wait for the value where it has to.  False in a graph capture that began before the
         value was written: a replay would not wait."""
-        device = self.value.get_device()
-        raw = torch._C._cuda_getCurrentRawStream(device)
+        raw = torch._C._cuda_getCurrentRawStream(self.device)
+        if self.written and raw in self.streams:
+            return True
         if not self.written:
             host = _lib.host()
             if host.event_done(self.event):
                 self.written = True
-            elif host.capturing(device):
+            elif host.capturing(self.device):
                 return False
             elif raw != self.builder:
-                host.wait_event(self.event, device)
+                host.wait_event(self.event, self.device)
         if raw not in self.streams:
-            self.value.record_stream(torch.cuda.current_stream(device))
+            self.value.record_stream(torch.cuda.current_stream(self.device))
             self.streams.add(raw)
         return True
 
@@ -99,16 +101,18 @@ class _PackedBase(nn.Module):
             raise ValueError("the W4A4 mode needs 4-bit indices and one 16-entry codebook; "
                              "pass act_scale=None for weight-only layers")
 
-    def _derive(self, slot: str, source: torch.Tensor, build, extra=None) -> torch.Tensor:
-        """``build()`` from the buffer ``source``, kept in ``slot`` until the buffer is replaced, moved or written in place.
-        Not kept: what a graph capture builds (only a replay writes it), and what an inference tensor gives (its writes are
-        not counted)."""
+    def _kept(self, slot: str, source: torch.Tensor, extra=None) -> torch.Tensor | None:
+        """What is kept in ``slot``, if ``source`` still is the buffer it was derived from and the current stream may read it."""
         kept = self.__dict__.get(slot)
-        counted = not source.is_inference()
-        if type(kept) is _Derived and counted and kept.is_of(source, extra) and kept.readable():
+        if type(kept) is _Derived and not source.is_inference() and kept.is_of(source, extra) and kept.readable():
             return kept.value
-        value = build()
-        if counted and not _lib.host().capturing(source.get_device()):
+        return None
+
+    def _keep(self, slot: str, source: torch.Tensor, value: torch.Tensor, extra=None) -> torch.Tensor:
+        """Keep ``value``, just derived from the buffer ``source``, until that is replaced, moved or written in place.  Not
+        kept: what a graph capture builds (only a replay writes it), and what an inference tensor gives (its writes are not
+        counted)."""
+        if not source.is_inference() and not _lib.host().capturing(value.get_device()):
             self.__dict__[slot] = _Derived(source, extra, value)
         return value
 
@@ -124,8 +128,11 @@ class _PackedBase(nn.Module):
         """``act_scale * codebook`` in fp32 (the weight operand of the tensor-core W4A4 form), built once
         and rebuilt when the codebook buffer or the scale changes."""
         cb = self.codebook
-        return self._derive("_scaled_cb", cb, lambda: cb.detach().float().reshape(-1) * torch.tensor(
-            self.act_scale, dtype=torch.float32, device=cb.device), self.act_scale)
+        scaled = self._kept("_scaled_cb", cb, self.act_scale)
+        if scaled is None:
+            scale = torch.tensor(self.act_scale, dtype=torch.float32, device=cb.device)
+            scaled = self._keep("_scaled_cb", cb, cb.detach().float().reshape(-1) * scale, self.act_scale)
+        return scaled
 
     def _refuse(self) -> None:
         if not self.use_cuda_kernel:
@@ -156,7 +163,10 @@ class DIMQLinear(_PackedBase):
                 or self.out_features * self.in_features * self.bits < (1 << 24)):
             return None
         pw = self.packed_weight
-        return self._derive("_tiled", pw, lambda: ops.linear_prepack(pw, self.out_features, self.in_features, self.bits))
+        tiled = self._kept("_tiled", pw)
+        if tiled is None:
+            tiled = self._keep("_tiled", pw, ops.linear_prepack(pw, self.out_features, self.in_features, self.bits))
+        return tiled
 
     def forward(self, x: torch.Tensor, residual: torch.Tensor | None = None) -> torch.Tensor:
         buffers = self._buffers
@@ -228,7 +238,10 @@ class DIMQConv2d(_PackedBase):
         pw = self._buffers.get("packed_weight")
         if pw is None:
             pw = self.packed_weight
-        return self._derive("_khwc", pw, lambda: ops.conv_prepack(pw, self.weight_shape, self.bits))
+        khwc = self._kept("_khwc", pw)
+        if khwc is None:
+            khwc = self._keep("_khwc", pw, ops.conv_prepack(pw, self.weight_shape, self.bits))
+        return khwc
 
     def forward(self, x: torch.Tensor, residual: torch.Tensor | None = None) -> torch.Tensor:
         buffers = self._buffers

@@ -130,13 +130,13 @@ def test_the_registered_operator_is_bypassed_in_plain_eager_calls_only():
             return func(*args, **(kwargs or {}))
 
     x, p = torch.zeros(2), torch.nn.Parameter(torch.zeros(2))
-    assert modules._eager(x) and modules._eager(x, None, x)
-    assert not modules._eager(x, p) and not modules._eager(x.clone().requires_grad_())
+    assert modules._eager(x, x, None) and modules._eager(x, x, x)
+    assert not modules._eager(x, p, None) and not modules._eager(x, x, p) and not modules._eager(x.clone().requires_grad_(), x, None)
     with torch.no_grad():
-        assert modules._eager(x, p)
+        assert modules._eager(x, p, p)
     for mode in (Function(), Dispatch()):
         with mode:
-            seen = modules._eager(x)
+            seen = modules._eager(x, x, None)
         assert not seen
 
 
