@@ -403,9 +403,13 @@ __device__ __forceinline__ void plain_chunk(float (&v)[32], const DenseParams& p
   }
 }
 
+// SEG form: where the run of k blocks that block kb is in ends; neither a segment nor a ring stage spans it
+__device__ __forceinline__ int seg_limit(int kb, int total_kb, const DenseParams& p) {
+  return kb < p.seg_cut && p.seg_cut < total_kb ? p.seg_cut : total_kb;
+}
 // end of the segment that starts at k block seg0
 __device__ __forceinline__ int seg_end_of(int seg0, int total_kb, const DenseParams& p) {
-  const int most = seg0 < p.seg_cut && p.seg_cut < total_kb ? p.seg_cut : total_kb;
+  const int most = seg_limit(seg0, total_kb, p);
   return seg0 + kSegBlocks < most ? seg0 + kSegBlocks : most;
 }
 // FORM: what the SEG form multiplies (kDense: not that form)
@@ -526,7 +530,7 @@ lut_dense_tc_kernel(const __grid_constant__ DenseMaps maps, const DenseParams p)
               STEM_ACC(1, t_w);
               full = smem_u32(&hdr->full[stage]);
               dst = smem_u32(smem + stage * stage_bytes);
-              const int left = total_kb - g;
+              const int left = (SEG ? seg_limit(g, total_kb, p) : total_kb) - g;
               const uint32_t bytes = static_cast<uint32_t>(left < p.kps ? left : p.kps) * sub_bytes;
               if (elect_one()) {
                 if constexpr (PAIR) { if (rank == 0) mbar_arrive_expect_tx(full, 2 * bytes); }   // both CTAs' copies
@@ -575,7 +579,7 @@ lut_dense_tc_kernel(const __grid_constant__ DenseMaps maps, const DenseParams p)
             __syncwarp();
             STEM_ACC(2, t_is);
           }
-          if (++sub == p.kps || g + 1 == total_kb) {   // the stage is complete (a tile's last stage may hold one block)
+          if (++sub == p.kps || g + 1 == total_kb || (SEG && g + 1 == p.seg_cut)) {   // the stage is complete (the last one of a run may hold one block)
             sub = 0;
             ++issued;
             if (++stage == n_st) { stage = 0; phase ^= 1u; }
@@ -612,7 +616,6 @@ lut_dense_tc_kernel(const __grid_constant__ DenseMaps maps, const DenseParams p)
     if (p.b_res && ok && !__all_sync(0xFFFFFFFFu, mbar_wait(smem_u32(&hdr->b_res_full), 0u, abort_flag, 0x1A00u))) ok = false;
     STEM_ACC_DECL;
     STEM_CLK(t_all);
-    // segments start at multiples of kps, so that no stage holds two (seg_cut is odd with kps = 1 only)
     int seg0 = 0;                                     // first k block of the current segment
     for (int t = tile0; t < num_tiles && ok;) {
       STEM_CLK(t_w1);
@@ -623,7 +626,7 @@ lut_dense_tc_kernel(const __grid_constant__ DenseMaps maps, const DenseParams p)
       const int seg_end = SEG ? seg_end_of(seg0, total_kb, p) : total_kb;
       const int seg_first = SEG ? seg0 : 0;
       for (int g = seg_first; g < seg_end; g += p.kps) {
-        const int nblk = total_kb - g < p.kps ? total_kb - g : p.kps;   // 64-k blocks in this stage
+        const int nblk = seg_end - g < p.kps ? seg_end - g : p.kps;   // 64-k blocks in this stage (a segment within a run holds an even number)
         STEM_CLK(t_w2);
         if (!__all_sync(0xFFFFFFFFu, mbar_wait(smem_u32(&hdr->full[stage]), phase, abort_flag, 0x1300u | stage))) { ok = false; break; }
         STEM_ACC(2, t_w2);
@@ -776,9 +779,10 @@ lut_dense_tc_kernel(const __grid_constant__ DenseMaps maps, const DenseParams p)
             }
             if constexpr (FORM == kSegSplit) {
               bool later = hdr->redo[ew] != 0;
-              float probe = 0.0f;                // a NaN if any of them is infinite or a NaN
+              float part[4] = {0.0f, 0.0f, 0.0f, 0.0f};       // four short chains
 #pragma unroll
-              for (int j = 0; j < 32; ++j) probe = fmaf(v[j], 0.0f, probe);
+              for (int j = 0; j < 32; ++j) part[j & 3] = fmaf(v[j], 0.0f, part[j & 3]);
+              const float probe = (part[0] + part[1]) + (part[2] + part[3]);     // a NaN if any v is infinite or a NaN
               if (__any_sync(0xFFFFFFFFu, probe != probe && rs == rs) && !later) {
                 bool nan = false;
 #pragma unroll
@@ -1045,7 +1049,6 @@ int launch_dense(DenseMaps& maps, DenseParams& p, const void* scratch, int64_t K
   // A convolution whose expanded weight is one tile wide and fits beside the activation stages keeps it in
   // shared memory: no per-stage weight copies.
   p.kps = (!pair && p.bn * (p.stack + 1) <= 128) ? 2 : 1;
-  if (seg && p.seg_cut < p.k_blocks * p.passes && p.seg_cut % 2 != 0) p.kps = 1;
 #ifdef DIMQ_B200_DIAG
   if (g_dense_diag & 65536) p.kps = 1;   // timing experiments: one block per stage
 #endif
