@@ -179,7 +179,7 @@ product_table_kernel(const void* __restrict__ codebook, int cb_dtype, int64_t to
 }
 
 // ---------------------------------------------------------------------------
-// hard quantise over a well-spaced sorted codebook: the path of trained and quantile codebooks
+// hard quantise over whole groups: trained and quantile codebooks
 // ---------------------------------------------------------------------------
 // One codebook per blockIdx.y; a block walks its group's weights, 8 consecutive ones per thread and step.
 //
@@ -197,7 +197,9 @@ product_table_kernel(const void* __restrict__ codebook, int cb_dtype, int64_t to
 // Bound: HBM (4 bytes in, 1 + bits / 8 or 4 out per weight), with ~30 instructions per weight beside it.  The kernel
 // below it replaces here spent 64-bit divisions per element, a serial sortedness check per 2 048 weights and
 // byte-wise stores: 4096 x 1024 fp32, 16 codewords, indices + packed and their unpacking took 28.7 us per call there,
-// 16.4 here (both kernels and three allocations).
+// 16.4 here (both kernels and three allocations).  256 codewords, indices + packed: well spaced 25 us (there 70), one duplicate
+// 29 (70), a quarter of them zero 36 (84), unsorted 236 (255); 512 groups of 4 608 weights, unsorted, 162 (149: the last
+// of a group's three blocks is a quarter full here), one duplicate 21 (149).
 template <typename T, int E>   // E: the number of codewords rounded up to a power of two
 __global__ void __launch_bounds__(kThreads)
 nearest_sorted_kernel(const T* __restrict__ w, int64_t n, int64_t group_elems, const float* __restrict__ codebooks,
