@@ -198,22 +198,22 @@ product_table_kernel(const void* __restrict__ codebook, int cb_dtype, int64_t to
 // below it replaces here spent 64-bit divisions per element, a serial sortedness check per 2 048 weights and
 // byte-wise stores: 4096 x 1024 fp32, 16 codewords, indices + packed and their unpacking took 28.7 us per call there,
 // 16.4 here (both kernels and three allocations).  256 codewords, indices + packed: well spaced 25 us (there 70), one duplicate
-// 29 (70), a quarter of them zero 36 (84), unsorted 236 (255); 512 groups of 4 608 weights, unsorted, 162 (149: the last
-// of a group's three blocks is a quarter full here), one duplicate 21 (149).
-template <typename T, int E>   // E: the number of codewords rounded up to a power of two
+// 29 (70), a quarter of them zero 36 (84), unsorted 236 (255); 512 groups of 4 608 weights, unsorted, 147 (149),
+// one duplicate 19 (149).
+template <typename T, int E, bool FULL>   // E: the number of codewords rounded up to a power of two; FULL: blocks of kThreads
 __global__ void __launch_bounds__(kThreads)
 nearest_sorted_kernel(const T* __restrict__ w, int64_t n, int64_t group_elems, const float* __restrict__ codebooks,
                       int entries, uint8_t* __restrict__ idx_out, uint8_t* __restrict__ packed, int bits,
                       T* __restrict__ fake_out) {
   __shared__ float tab[E + 2];          // -inf, the codewords, +inf up to E
   __shared__ int gap_bits, unsorted;
-  const int tid = threadIdx.x;
+  const int tid = threadIdx.x, threads = FULL ? kThreads : static_cast<int>(blockDim.x);
   const float kInf = __int_as_float(0x7F800000);
   const float* cb = codebooks + static_cast<int64_t>(blockIdx.y) * entries;
   if (tid == 0) { gap_bits = 0x7F800000; unsorted = 0; tab[0] = -kInf; tab[E + 1] = kInf; }
-  for (int k = tid; k < E; k += kThreads) tab[k + 1] = k < entries ? cb[k] : kInf;
+  for (int k = tid; k < E; k += threads) tab[k + 1] = k < entries ? cb[k] : kInf;
   __syncthreads();
-  for (int k = tid; k + 1 < entries; k += kThreads) {
+  for (int k = tid; k + 1 < entries; k += threads) {
     const float gap = __fsub_rn(tab[k + 2], tab[k + 1]);
     if (!(gap >= 0.0f) || !isfinite(tab[k + 1]) || !isfinite(tab[k + 2])) unsorted = 1;
     else atomicMin(&gap_bits, __float_as_int(gap));     // floats from zero up order like their bits
@@ -230,8 +230,8 @@ nearest_sorted_kernel(const T* __restrict__ w, int64_t n, int64_t group_elems, c
   const int64_t start = static_cast<int64_t>(blockIdx.y) * group_elems;      // a multiple of 8
   const int64_t end = start + group_elems < n ? start + group_elems : n;
   const int64_t total_bytes = (n * bits + 7) / 8;
-  for (int64_t base = start + (static_cast<int64_t>(blockIdx.x) * kThreads + tid) * 8; base < end;
-       base += static_cast<int64_t>(gridDim.x) * kThreads * 8) {
+  for (int64_t base = start + (static_cast<int64_t>(blockIdx.x) * threads + tid) * 8; base < end;
+       base += static_cast<int64_t>(gridDim.x) * threads * 8) {
     const bool full = base + 8 <= end;
     float f[8];
     if (full) {
@@ -354,13 +354,20 @@ nearest_sorted_kernel(const T* __restrict__ w, int64_t n, int64_t group_elems, c
 template <typename T>
 int launch_nearest_sorted(const void* w, int64_t n, int64_t groups, int64_t group_elems, const float* codebooks, int entries,
                           uint8_t* idx, uint8_t* packed, int bits, void* fake_out, cudaStream_t st) {
-  // enough blocks for every SM to hold eight, each with as few steps as that leaves
-  const int64_t chunks = ((group_elems < n ? group_elems : n) + kThreads * 8 - 1) / (kThreads * 8);
+  // enough blocks for every SM to hold eight, each with as few steps as that leaves.  Where one step does, no more threads
+  // than give a group's blocks the same number of weights each (4 608: three blocks of 192 threads, not 256, 256 and 64 -
+  // 256 unsorted codewords per group 147 us, not 162); with several steps full blocks keep more loads in flight.
+  const int64_t units = ((group_elems < n ? group_elems : n) + 7) / 8;
+  const int64_t chunks = (units + kThreads - 1) / kThreads;
   const int64_t most = (8 * kNumSMs + groups - 1) / groups;
-  const dim3 grid(static_cast<unsigned>(chunks < most ? chunks : most), static_cast<unsigned>(groups));
+  const int64_t blocks = chunks < most ? chunks : most;
+  const unsigned threads = chunks <= most ? static_cast<unsigned>((units + blocks * 32 - 1) / (blocks * 32) * 32) : kThreads;
+  const dim3 grid(static_cast<unsigned>(blocks), static_cast<unsigned>(groups));
   const T* src = static_cast<const T*>(w);
   T* fake = static_cast<T*>(fake_out);
-#define DIMQ_NEAREST(E) nearest_sorted_kernel<T, E><<<grid, kThreads, 0, st>>>(src, n, group_elems, codebooks, entries, idx, packed, bits, fake)
+#define DIMQ_NEAREST(E)                                                                                                            \
+  (threads == kThreads ? nearest_sorted_kernel<T, E, true> : nearest_sorted_kernel<T, E, false>)<<<grid, threads, 0, st>>>(        \
+      src, n, group_elems, codebooks, entries, idx, packed, bits, fake)
   if (entries <= 4) DIMQ_NEAREST(4);
   else if (entries <= 8) DIMQ_NEAREST(8);
   else if (entries <= 16) DIMQ_NEAREST(16);
