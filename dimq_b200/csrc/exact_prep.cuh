@@ -16,8 +16,8 @@
 // Non-finite values of the fp32 form: an infinite activation has hi = 0 and keeps its value in lo, which meets w_hi only; a
 // codeword that would underflow to w_hi = 0 takes fp16's smallest instead (w_lo carries the difference), so the product has
 // the sign of both.  A row with a NaN has the scale NaN.  An infinite or NaN codeword is a NaN here: no split of it is right,
-// as x_lo may be zero, or of the other sign, where x is not.  Where an output comes out as a NaN and its row has none, the
-// epilogue computes it again in plain fp32.
+// as x_lo may be zero, or of the other sign, where x is not.  Where an output of such a codebook comes out as a NaN and its
+// row has none, the epilogue computes it again in plain fp32.
 // W4A4 codes are one exact term: a zero code against an infinite codeword is NaN as in fp32, with one term or two (there
 // w_lo keeps the value and w_hi = 0).
 #pragma once

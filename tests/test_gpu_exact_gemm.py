@@ -410,6 +410,58 @@ def test_linear_f32_non_finite_codewords(ops, book, bits, group_rows):
     assert bool(((y.double() - want).abs() <= bound + 1e-30)[ok].all())
 
 
+@pytest.mark.parametrize("book", [torch.float16, torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("bits", [2, 3, 4])
+def test_linear_f32_infinite_activations_against_finite_codewords(ops, book, bits):
+    # zero, subnormal, smallest and largest codewords of either sign: what the tensor cores give stands, NaN included
+    m, k, n = 200, 192, 132
+    packed, books, _ = _weight(ops, n, k, bits, book, seed=bits)
+    books = books.reshape(-1).clone()
+    f = torch.finfo(book)
+    books[0], books[1] = 0.0, -f.smallest_normal / 64
+    if bits > 2:
+        books[2], books[3] = f.smallest_normal, -f.max / 64      # no product of a finite activation overflows
+    idx = ops.unpack_bits(packed, n * k, bits).view(n, k).long()
+    idx[5:9] = books.numel() - 1                  # columns without a zero codeword
+    packed, w = ops.pack_bits(idx.to(torch.uint8), bits), books.float()[idx]
+    x = torch.randn(m, k, device="cuda")
+    x[3, 5], x[40, 9], x[199, 191] = float("inf"), float("-inf"), float("inf")
+    x[50, 1], x[50, 2], x[60, 0] = float("inf"), float("-inf"), float("nan")
+    y = ops.dimq_linear_wq(x, packed, books, None, n, k, bits=bits)
+    assert ops.last_device_status() == 0
+    rows = [3, 40, 50, 60, 199]
+    prod = x[rows].unsqueeze(1) * w.unsqueeze(0)
+    plus, minus = (prod == float("inf")).any(2), (prod == float("-inf")).any(2)
+    nan = prod.isnan().any(2) | (plus & minus)
+    assert torch.equal(y[rows].isnan(), nan)
+    assert torch.equal(y[rows] == float("inf"), plus & ~nan) and torch.equal(y[rows] == float("-inf"), minus & ~nan)
+
+
+def test_infinite_activations_cost_no_second_computation(ops):
+    # Outputs are computed again only where the codebook has an infinity or a NaN (that took 40 times the time here).
+    m, k, n = 1576, 768, 3072
+    packed, books, _ = _weight(ops, n, k, 4, torch.float32, seed=1)
+    books = books.reshape(-1).clone()
+    books[2] = 0.0
+    x = torch.randn(m, k, device="cuda")
+    bad = x.clone()
+    bad[:, 5] = float("inf")
+
+    def us(act):
+        start, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        best = float("inf")
+        for _ in range(5):
+            start.record()
+            for _ in range(3):
+                ops.dimq_linear_wq(act, packed, books, None, n, k, bits=4)
+            end.record()
+            end.synchronize()
+            best = min(best, start.elapsed_time(end))
+        return best
+
+    assert us(bad) < 3 * us(x)
+
+
 def test_linear_f32_infinite_activations_against_tiny_codewords(ops):
     # a codeword far below the largest of its book is not zero: infinity times it is infinity
     m, k, n = 40, 64, 64
